@@ -48,20 +48,19 @@ static_assert(sizeof(TriRef) == 12, "TriRef must be 12 bytes");
 
 // Reciprocal square root in FP64, full precision.
 // Seed: the FP64 approximate reciprocal square root instruction (rsqrt.approx.ftz.f64, relative
-// error below 1e-6 measured on B200); two Newton-Raphson steps y <- y + y/2 (1 - x y^2) in FP64
-// (the classical iteration for x^{-1/2}; each step squares the relative error, so the result is
-// within 1.2 ulp, measured against 1/sqrt over 4M arguments in [1e-12, 16]).  Inputs are squared
-// distances of quadrature points: positive and normal.  (Measured in the nearfield kernel: 4%
-// faster than an FP32 seed, which needs two conversions, and 7% faster than CUDA's rsqrt().)
+// error below 1e-6 measured on B200).  One step of Householder's method of third order for
+// x^{-1/2}: with e = 1 - x y^2 the root is y (1 - e)^{-1/2} = y (1 + e/2 + 3 e^2/8 + O(e^3)), so a
+// seed error of 1e-6 leaves 5/2 (1e-6)^3, far below one rounding: at most 0.51 ulp from 1/sqrt over
+// 4M arguments in [1e-12, 64] (two Newton-Raphson steps: 0.99 ulp).  The kernels around it are bound
+// by FP64 instructions, five here where two Newton steps take eight: dense constant-basis single
+// layer of 8192 triangles 1.23 -> 1.07 ms, linear-basis V and K nearfield of 32768 triangles
+// 6.83 -> 6.66 ms (bound by its scatter).  Inputs are squared distances of quadrature points:
+// positive and normal.
 __device__ __forceinline__ double rsqrt_nr(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  double h = x * y;
-  double e = fma(-h, y, 1.0);
-  y = fma(0.5 * y, e, y);
-  h = x * y;
-  e = fma(-h, y, 1.0);
-  return fma(0.5 * y, e, y);
+  const double e = fma(-x, y * y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
 }
 
 // Lagrange polynomial mu of the nodes xi[0..m) at x, prod_{l != mu} (x - xi_l) / (xi_mu - xi_l)
