@@ -1,5 +1,6 @@
 // C-ABI implementation: status, device init, surfaces, operators and nearfield entry points.
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stdarg.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -175,6 +176,8 @@ extern "C" h2b_surface *h2b_surface_new(uint32_t vertices, const double *x, uint
                       s->stream) != cudaSuccess ||
       cudaMemcpyAsync(s->d_x, x, sizeof(double) * 3ull * vertices, cudaMemcpyHostToDevice,
                       s->stream) != cudaSuccess ||
+      cudaMallocAsync(&s->d_qrec, sizeof(QuadRec) * (size_t) triangles, s->stream) != cudaSuccess ||
+      h2b_near_quad_records(s->d_tri, triangles, s->d_qrec, s->stream) != H2B_OK ||
       cudaMallocAsync(&s->d_vt_off, sizeof(uint32_t) * (vertices + 1ull), s->stream) != cudaSuccess ||
       cudaMallocAsync(&s->d_vt_tri, sizeof(uint32_t) * 3ull * triangles, s->stream) != cudaSuccess ||
       cudaMemcpyAsync(s->d_vt_off, s->adj.off, sizeof(uint32_t) * (vertices + 1ull),
@@ -196,6 +199,7 @@ extern "C" void h2b_surface_del(h2b_surface *s) {
   // every entry point ends synchronised, so no kernel still reads these arrays; stream-ordered
   // frees do not synchronise the device (other handles keep running)
   if (s->d_tri) cudaFreeAsync(s->d_tri, s->stream);
+  if (s->d_qrec) cudaFreeAsync(s->d_qrec, s->stream);
   if (s->d_x) cudaFreeAsync(s->d_x, s->stream);
   if (s->d_vt_off) cudaFreeAsync(s->d_vt_off, s->stream);
   if (s->d_vt_tri) cudaFreeAsync(s->d_vt_tri, s->stream);
@@ -361,6 +365,7 @@ void h2b_fill_launch(const h2b_bem *b, h2b_near_launch *L) {
   L->col_linear = b->col_basis == H2B_BASIS_LINEAR;
   L->q = b->q;
   L->tri = b->s->d_tri;
+  L->qrec = b->s->d_qrec;
   L->kconst = b->kconst;
   L->k_re = b->k_re;
   L->k_imn = -b->k_im;
@@ -396,6 +401,15 @@ int h2b_devplan_upload(const h2b_nearplan *p, cudaStream_t st, h2b_devplan *dp) 
   if (p->ntiles) {
     H2B_CUDA_TRY(cudaMallocAsync(&dp->tiles, sizeof(h2b_tile) * p->ntiles, st));
     H2B_CUDA_TRY(cudaMemcpyAsync(dp->tiles, p->tiles, sizeof(h2b_tile) * p->ntiles,
+                                 cudaMemcpyHostToDevice, st));
+  }
+  bool mates = false;
+  for (uint32_t i = 0; i < p->ntiles && !mates; i++) mates = p->tiles[i].mate != 0;
+  if (mates) {
+    std::vector<uint32_t> half(p->ntiles);
+    dp->nhalf = h2b_nearplan_halves(p, half.data());
+    H2B_CUDA_TRY(cudaMallocAsync(&dp->half, sizeof(uint32_t) * dp->nhalf, st));
+    H2B_CUDA_TRY(cudaMemcpyAsync(dp->half, half.data(), sizeof(uint32_t) * dp->nhalf,
                                  cudaMemcpyHostToDevice, st));
   }
   if (p->nrefs) {
@@ -466,6 +480,7 @@ int h2b_classify_device(const h2b_surface *s, const void *refs, const h2b_tile *
 
 void h2b_devplan_free(h2b_devplan *dp, cudaStream_t st) {
   if (dp->tiles) cudaFreeAsync(dp->tiles, st);
+  if (dp->half) cudaFreeAsync(dp->half, st);
   if (dp->refs) cudaFreeAsync(dp->refs, st);
   if (dp->sing) cudaFreeAsync(dp->sing, st);
   memset(dp, 0, sizeof(*dp));
@@ -486,6 +501,38 @@ int h2b_check_err_flag(const h2b_bem *b, cudaStream_t st) {
 // ------------------------------------------------------------------------------------------
 // Nearfield blocks
 // ------------------------------------------------------------------------------------------
+
+// Tile size of a block: the one with the least estimated time, rounds of the SMs (1.5 resident tiles
+// each, measured between one and two) times the lanes a tile's triangle pairs take.  A tile side of
+// s vertices touches about 2 s + 4.3 sqrt(s) triangles (the inner ones and those along the border,
+// counted on refined spheres), rows in groups of 32 lanes, so smaller tiles evaluate border pairs more
+// often but spread a small block over the SMs; with constant bases tiles share no pairs.  FIXED is
+// the fixed cost of a tile in pairs (clearing, staging and writing it).  60 x 57 linear block: four
+// tiles of 32 take 46 us, 8 x 8 tiles 16 us.  578 x 578 complex double layer: tiles of 16 take
+// 613 us, of 32 533 us.
+static uint32_t block_tile(const h2b_bem *b, uint32_t rows, uint32_t cols, bool same) {
+  constexpr double FIXED = 400.0;
+  const bool rl = b->row_basis == H2B_BASIS_LINEAR, cl = b->col_basis == H2B_BASIS_LINEAR;
+  uint32_t best = H2B_TILE_MAX;
+  double least = 0.0;
+  for (uint32_t t = H2B_TILE_MAX; t >= 8; t /= 2) {
+    auto tri = [&](uint32_t n, bool lin) {
+      const double s = n < t ? n : t;
+      return lin ? 2.0 * s + 4.3 * sqrt(s) : s;
+    };
+    double r = tri(rows, rl);
+    if (cl) r = 32.0 * ceil(r / 32.0);
+    double n = ceil((double) rows / t) * ceil((double) cols / t);
+    if (same) n = 0.5 * (n + ceil((double) rows / t));
+    const double rounds = n / (1.5 * b->s->num_sms);
+    const double cost = (rounds > 1.0 ? rounds : 1.0) * (r * tri(cols, cl) + FIXED);
+    if (t == H2B_TILE_MAX || cost < 0.9 * least) {
+      best = t;
+      least = cost;
+    }
+  }
+  return best;
+}
 
 extern "C" int h2b_bem_nearfield(const h2b_bem *bem, const uint32_t *ridx, uint32_t rows,
                                  const uint32_t *cidx, uint32_t cols, int ntrans, double *N,
@@ -541,9 +588,10 @@ extern "C" int h2b_bem_nearfield(const h2b_bem *bem, const uint32_t *ridx, uint3
   const bool dev_out = h2b_is_device_ptr(N);
   const uint64_t ld_dev = dev_out ? ld : out_rows;
 
-  // small outputs: 32 x 32 tiles so that the grid covers the SMs
-  uint64_t t64 = (uint64_t) ((rows + 63) / 64) * ((cols + 63) / 64);
-  uint32_t tile = t64 < 2ull * s->num_sms ? 32 : 64;
+  const bool same = bem->row_basis == bem->col_basis && rows == cols &&
+                    !memcmp(ridx, cidx, sizeof(uint32_t) * rows);
+  if (same) cidx = ridx;  // one set of triangle lists
+  const uint32_t tile = block_tile(bem, rows, cols, same);
 
   // the singular pairs are found on the device (h2b_classify_device): the host plan only lists
   // the tiles and their triangles
@@ -554,6 +602,11 @@ extern "C" int h2b_bem_nearfield(const h2b_bem *bem, const uint32_t *ridx, uint3
                               bem->col_basis, ridx, rows, cidx, cols, 0, (uint32_t) ld_dev,
                               ntrans, tile);
   if (rc == H2B_OK) rc = h2b_nearplan_finalize(&plan);
+  // equal row and column index lists: tiles (I, J) and (J, I) take the same triangle pairs
+  if (rc == H2B_OK && same) {
+    const uint32_t nt = (rows + tile - 1) / tile;
+    h2b_nearplan_mate(&plan, 0, 0, nt, nt);
+  }
   if (rc != H2B_OK) {
     h2b_nearplan_free(&plan);
     h2b_set_error("h2b_bem_nearfield: out of host memory building the plan");
@@ -591,6 +644,8 @@ extern "C" int h2b_bem_nearfield(const h2b_bem *bem, const uint32_t *ridx, uint3
   L.refs = dp.refs;
   L.tiles = dp.tiles;
   L.ntiles = dp.ntiles;
+  L.half = dp.half;
+  L.nhalf = dp.nhalf;
   L.sing = dp.sing;
   L.nsing = dp.nsing;
   L.nvert = dp.nvert;

@@ -219,7 +219,7 @@ extern "C" void h2b_h2matrix_del(h2b_h2matrix *h) {
     devtree_free(h->ct, st);
     dfree(h->d_adm_rc, st); dfree(h->d_adm_cc, st);
     dfree(h->d_near_rc, st); dfree(h->d_near_cc, st); dfree(h->d_near_off, st);
-    dfree(h->d_tiles, st); dfree(h->d_refs, st); dfree(h->d_sing, st);
+    dfree(h->d_tiles, st); dfree(h->d_half, st); dfree(h->d_refs, st); dfree(h->d_sing, st);
     dfree(h->d_xs, st); dfree(h->d_ys, st); dfree(h->d_ws, st); dfree(h->d_wsl, st);
   }
   for (int e = 0; e < 12; e++)
@@ -246,6 +246,37 @@ static int classify_singular(h2b_h2matrix *h, uint64_t all_pairs) {
   return H2B_OK;
 }
 
+// Equal row and column trees (clusters, index lists, boxes) and bases.
+static int same_sides(const h2b_bem *bem, const h2b_tree *tree) {
+  const h2b_ctree &r = tree->row, &c = tree->col;
+  return bem->row_basis == bem->col_basis && r.n == c.n && r.nidx == c.nidx &&
+         !memcmp(r.off, c.off, sizeof(uint32_t) * r.n) &&
+         !memcmp(r.size, c.size, sizeof(uint32_t) * r.n) &&
+         !memcmp(r.sons, c.sons, sizeof(uint32_t) * r.n) &&
+         !memcmp(r.idx, c.idx, sizeof(uint32_t) * r.nidx) &&
+         !memcmp(r.bmin, c.bmin, sizeof(double) * 3 * r.n) &&
+         !memcmp(r.bmax, c.bmax, sizeof(double) * 3 * r.n);
+}
+
+// For every block its transposed block (row and column cluster exchanged), or UINT32_MAX: blocks
+// b with clusters (rc[b], cc[b]) of trees with n clusters.
+static std::vector<uint32_t> transposed_blocks(const std::vector<uint32_t> &rc,
+                                               const std::vector<uint32_t> &cc, uint32_t n) {
+  // blocks by row cluster
+  std::vector<uint32_t> start(n + 1, 0), at(rc.size()), mate(rc.size(), UINT32_MAX);
+  for (uint32_t r : rc) start[r + 1]++;
+  for (uint32_t r = 0; r < n; r++) start[r + 1] += start[r];
+  std::vector<uint32_t> fill(start.begin(), start.end() - 1);
+  for (uint32_t b = 0; b < rc.size(); b++) at[fill[rc[b]]++] = b;
+  for (uint32_t b = 0; b < rc.size(); b++)
+    for (uint32_t i = start[cc[b]]; i < start[cc[b] + 1]; i++)
+      if (cc[at[i]] == rc[b]) {
+        mate[b] = at[i];
+        break;
+      }
+  return mate;
+}
+
 // The structure of an H2 matrix of rank k (every cluster basis padded to k columns); m is the
 // interpolation order of the Chebyshev path (1 for the greenhybrid bases, which use no nodes).
 static h2b_h2matrix *h2matrix_create(const h2b_bem *bem, const h2b_tree *tree, uint32_t m,
@@ -264,6 +295,7 @@ static h2b_h2matrix *h2matrix_create(const h2b_bem *bem, const h2b_tree *tree, u
   h->k = k;
   h->cx = bem->pde == H2B_HELMHOLTZ;
   h->num_sms = bem->s->num_sms;
+  h->same = same_sides(bem, tree);
   int rc = H2B_OK;
   if (cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking) != cudaSuccess) {
     h2b_set_error("h2b_h2matrix_new: %s", cudaGetErrorString(cudaGetLastError()));
@@ -277,10 +309,13 @@ static h2b_h2matrix *h2matrix_create(const h2b_bem *bem, const h2b_tree *tree, u
   // blocks
   std::vector<uint32_t> arc, acc, nrc, ncc;
   std::vector<uint64_t> noff;
+  std::vector<uint32_t> tile0;  // first tile of each nearfield block
   uint64_t ntot = 0;
   h2b_nearplan plan;
   h2b_nearplan_init(&plan);
   plan.skip_sing = 1;  // singular pairs are found on the device below
+  // equal sides share their triangle lists (the plan knows a list by its index pointer)
+  const uint32_t *cidx = h->same ? tree->row.idx : tree->col.idx;
   for (uint32_t b = 0; rc == H2B_OK && b < tree->blocks.n; b++) {
     const uint32_t r = tree->blocks.rc[b], c = tree->blocks.cc[b];
     if (tree->blocks.adm[b]) {
@@ -290,13 +325,28 @@ static h2b_h2matrix *h2matrix_create(const h2b_bem *bem, const h2b_tree *tree, u
       nrc.push_back(r);
       ncc.push_back(c);
       noff.push_back(ntot);
+      tile0.push_back(plan.ntiles);
       const uint32_t rows = tree->row.size[r], cols = tree->col.size[c];
       rc = h2b_nearplan_add_block(&plan, adj, bem->row_basis, bem->col_basis,
                                   tree->row.idx + tree->row.off[r], rows,
-                                  tree->col.idx + tree->col.off[c], cols, ntot, rows, 0, 64);
+                                  cidx + tree->col.off[c], cols, ntot, rows, 0, 64);
       ntot += (uint64_t) rows * cols;
     }
   }
+  // with equal sides the tiles of a nearfield block and of its transposed block take the same
+  // triangle pairs: one tile of each two fills both
+  std::vector<uint32_t> half;
+  if (rc == H2B_OK && h->same) {
+    const std::vector<uint32_t> mate = transposed_blocks(nrc, ncc, tree->row.n);
+    for (uint32_t b = 0; b < nrc.size(); b++)
+      if (mate[b] != UINT32_MAX)
+        h2b_nearplan_mate(&plan, tile0[b], tile0[mate[b]],
+                          (tree->row.size[nrc[b]] + H2B_TILE_MAX - 1) / H2B_TILE_MAX,
+                          (tree->col.size[ncc[b]] + H2B_TILE_MAX - 1) / H2B_TILE_MAX);
+    half.resize(plan.ntiles);
+    half.resize(h2b_nearplan_halves(&plan, half.data()));
+  }
+  h->nhalf = (uint32_t) half.size();
   uint64_t all_pairs = 0;
   if (rc == H2B_OK)
     for (uint32_t t = 0; t < plan.ntiles; t++)
@@ -317,7 +367,7 @@ static h2b_h2matrix *h2matrix_create(const h2b_bem *bem, const h2b_tree *tree, u
     if ((rc = upload(&h->d_adm_rc, arc, h->st)) || (rc = upload(&h->d_adm_cc, acc, h->st)) ||
         (rc = upload(&h->d_near_rc, nrc, h->st)) || (rc = upload(&h->d_near_cc, ncc, h->st)) ||
         (rc = upload(&h->d_near_off, noff, h->st)) || (rc = upload(&h->d_tiles, tiles, h->st)) ||
-        (rc = upload(&h->d_refs, refs, h->st)) ||
+        (rc = upload(&h->d_half, half, h->st)) || (rc = upload(&h->d_refs, refs, h->st)) ||
         (rc = classify_singular(h, all_pairs))) {
     } else if (cudaMallocAsync(&h->d_S, sizeof(double) * W * std::max<uint64_t>((uint64_t) h->nadm * h->k * h->k, 1) + H2B_MV_SLACK, h->st) != cudaSuccess ||
                cudaMallocAsync(&h->d_N, sizeof(double) * W * std::max<uint64_t>(ntot, 1) + H2B_MV_SLACK, h->st) != cudaSuccess ||
@@ -480,16 +530,6 @@ extern "C" h2b_h2matrix *h2b_h2matrix_new_greenhybrid(const h2b_bem *bem, const 
   }
   int rc = green_setup(h->rt, tree->row, k, h->st);
   if (rc == H2B_OK) rc = green_setup(h->ct, tree->col, k, h->st);
-  {
-    const h2b_ctree &r = tree->row, &c = tree->col;
-    h->g_same = bem->row_basis == bem->col_basis && r.n == c.n && r.nidx == c.nidx &&
-                !memcmp(r.off, c.off, sizeof(uint32_t) * r.n) &&
-                !memcmp(r.size, c.size, sizeof(uint32_t) * r.n) &&
-                !memcmp(r.sons, c.sons, sizeof(uint32_t) * r.n) &&
-                !memcmp(r.idx, c.idx, sizeof(uint32_t) * r.nidx) &&
-                !memcmp(r.bmin, c.bmin, sizeof(double) * 3 * r.n) &&
-                !memcmp(r.bmax, c.bmax, sizeof(double) * 3 * r.n);
-  }
   if (rc == H2B_OK && cudaStreamSynchronize(h->st) != cudaSuccess) {
     h2b_set_error("h2b_h2matrix_new_greenhybrid: %s", cudaGetErrorString(cudaGetLastError()));
     rc = H2B_ERR_CUDA;
@@ -955,7 +995,7 @@ static int col_basis(h2b_h2matrix *h) {
   mark(h, 2);
   // column side of the double layer: normal derivatives (assemble_bem3d_dn_lagrange_*)
   int rc;
-  if (h->green && h->g_same && h->g_row_ready && h->bem->layer == H2B_SLP &&
+  if (h->green && h->same && h->g_row_ready && h->bem->layer == H2B_SLP &&
       h->rt.h_woff == h->ct.h_woff) {
     rc = green_copy_col(h);
     h->g_col_copied = 1;
@@ -1000,6 +1040,8 @@ static int launch_near(h2b_h2matrix *h, h2b_h2matrix *h2) {
   L.refs = h->d_refs;
   L.tiles = h->d_tiles;
   L.ntiles = h->ntiles;
+  L.half = h->d_half;
+  L.nhalf = h->nhalf;
   L.sing = h->d_sing;
   L.nsing = h->nsing;
   L.nvert = h->pairs[1];

@@ -60,9 +60,10 @@ struct h2b_h2matrix {
   // one-dimensional rule on [-1, 1], the box widening delta and the ACA accuracy; k = 12 ml^2
   int green = 0;
   int g_ml = 0;
-  // 1: equal row and column trees and bases (the column basis of the single layer is then the
-  // row basis); g_row_ready: the row basis of the current assembly is in place
-  int g_same = 0, g_row_ready = 0;
+  // 1: equal row and column trees and bases (the greenhybrid column basis of the single layer is then
+  // the row basis)
+  int same = 0;
+  int g_row_ready = 0;   // the row basis of the current assembly is in place
   int g_col_copied = 0;  // the column basis was copied (its leaf bases are the row side's)
   double g_tg[9] = {}, g_wg[9] = {}, g_delta = 0.0, g_accur = 0.0;
   int cx = 0, num_sms = 148;
@@ -105,6 +106,8 @@ struct h2b_h2matrix {
   double *d_N = nullptr;
   float *f_S = nullptr, *f_N = nullptr;  // FP32 copies (h2b_h2matrix_make_single)
   h2b_tile *d_tiles = nullptr;
+  uint32_t *d_half = nullptr;  // tiles to run when mates are filled together (nullptr: no mates)
+  uint32_t nhalf = 0;
   h2b_triref *d_refs = nullptr;
   h2b_sing *d_sing = nullptr;
   double *d_xp = nullptr, *d_yp = nullptr, *d_xt = nullptr, *d_yt = nullptr;

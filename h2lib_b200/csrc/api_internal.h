@@ -20,6 +20,7 @@ struct h2b_surface {
   std::vector<uint32_t> t;      // 3*nt
   h2b_adjacency adj{};
   TriRec *d_tri = nullptr;      // nt records
+  QuadRec *d_qrec = nullptr;    // nt records (distant rule of order 2)
   double *d_x = nullptr;        // 3*nv
   uint32_t *d_vt_off = nullptr, *d_vt_tri = nullptr;  // vertex -> triangles (CSR, from adj)
 };
@@ -44,6 +45,8 @@ struct h2b_bem {
 
 struct h2b_devplan {
   h2b_tile *tiles;
+  uint32_t *half;  // tiles to run when mates are filled together (nullptr: no mates)
+  uint32_t nhalf;
   h2b_triref *refs;
   h2b_sing *sing;
   uint32_t ntiles, nsing;

@@ -36,13 +36,22 @@ struct __align__(16) TriRec {
 };
 static_assert(sizeof(TriRec) == 128, "TriRec must be 128 bytes");
 
+// A triangle's part of the q = 2 distant rule: its four points, each with its component along the
+// unit normal, the normal, the Gram determinant and the vertex ids; 22 words of 8 bytes.
+struct __align__(16) QuadRec {
+  double p[4][4];  // x, y, z, <p, n>
+  double n[3], g;
+  uint32_t v[3], pad;
+};
+static_assert(sizeof(QuadRec) == 176, "QuadRec must be 176 bytes");
+
 // A triangle referenced by a nearfield tile: its id and the local output row/column index of each
 // of its three vertices (linear basis) or of the triangle itself in l[0] (constant basis); -1 when
 // the vertex is outside the tile.
 struct TriRef {
   uint32_t t;
   int16_t l[3];
-  int16_t pad;
+  int16_t slots;  // local vertex in slot 0, 1, 2 (two bits each), see h2b_triref
 };
 static_assert(sizeof(TriRef) == 12, "TriRef must be 12 bytes");
 

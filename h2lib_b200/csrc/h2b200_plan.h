@@ -12,11 +12,13 @@ extern "C" {
 
 #define H2B_TILE_MAX 64
 
-/* Same layout as TriRef in device_common.cuh. */
+/* Same layout as TriRef in device_common.cuh.  slots (linear basis): the triangle's local vertex in
+ * slot 0, 1, 2 (two bits each), assigned along the list so that a vertex shared with the triangle
+ * before keeps its slot. */
 typedef struct {
   uint32_t t;
   int16_t l[3];
-  int16_t pad;
+  int16_t slots;
 } h2b_triref;
 
 /* One output tile: rows x cols entries (<= 64 x 64) written at out_off + r + c*ld (or, with
@@ -28,7 +30,7 @@ typedef struct {
   uint32_t ld;
   uint16_t rows, cols;
   uint32_t flags;
-  uint32_t pad;
+  uint32_t mate;  /* 1 + the tile with rows and columns exchanged (same index lists), 0: none */
 } h2b_tile;
 
 /* One singular triangle pair of a tile (tr, sc: absolute positions in the TriRef pool). */
@@ -52,6 +54,8 @@ typedef struct {
   const uint32_t **lkey;
   uint32_t *lkn, *loff, *llen;
   size_t lcap, lcount;
+  uint64_t *order;          /* scratch of the list ordering */
+  size_t corder;
   /* 1: leave the singular pairs to the device classification (h2b_near_classify) */
   int skip_sing;
 } h2b_nearplan;
@@ -82,6 +86,13 @@ int h2b_nearplan_finalize(h2b_nearplan *p);
 int h2b_nearplan_add_reflist(h2b_nearplan *p, h2b_adjacency *adj, int linear,
                              const uint32_t *idx, uint32_t n, uint32_t *off, uint32_t *len);
 uint32_t h2b_pair_code(const uint32_t *tv, const uint32_t *sv);
+/* Marks the tiles of one block (row and column index lists equal: first tile t0, nt tiles per side)
+ * or of two blocks with exchanged row and column lists (t0: nr x nc tiles, t1: nc x nr tiles) as each
+ * other's mates.  Tiles are in add_block's order. */
+void h2b_nearplan_mate(h2b_nearplan *p, uint32_t t0, uint32_t t1, uint32_t nr, uint32_t nc);
+/* The tiles to run when mates are filled together: of two mates only the first, largest products of
+ * list lengths first (eight classes).  list: ntiles entries; returns their number. */
+uint32_t h2b_nearplan_halves(const h2b_nearplan *p, uint32_t *list);
 
 #ifdef __cplusplus
 }

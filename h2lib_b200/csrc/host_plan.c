@@ -87,6 +87,7 @@ h2b_nearplan_free(h2b_nearplan *p)
 {
   free(p->tiles); free(p->refs); free(p->sing);
   free((void *) p->lkey); free(p->lkn); free(p->loff); free(p->llen);
+  free(p->order);
   memset(p, 0, sizeof(*p));
 }
 
@@ -139,6 +140,82 @@ next_gen(h2b_adjacency *adj)
   return adj->gen;
 }
 
+/* Orders the triangles of a linear list by id and assigns their vertices to three slots: the
+ * distant-pair kernel walks along the list and keeps the sums of a vertex in registers while
+ * consecutive triangles share it.  Refined and generated meshes number neighbouring triangles
+ * consecutively, so the walk leaves 0.8 vertices per triangle on a refined sphere (2.3 of a
+ * triangle's vertices lie in the cluster); a greedy strip over the list leaves 0.75. */
+static int
+order_list(h2b_nearplan *p, const h2b_adjacency *adj, uint32_t off, uint32_t n)
+{
+  h2b_triref *r = p->refs + off, *tmp;
+  uint64_t *src, *dst;
+  uint32_t i, held[3] = {UINT32_MAX, UINT32_MAX, UINT32_MAX};
+  const size_t need = 2 * (size_t) n + (sizeof(h2b_triref) * (size_t) n + 7) / 8;
+  if (need > p->corder) {
+    uint64_t *o = (uint64_t *) realloc(p->order, sizeof(uint64_t) * 2 * need);
+    if (!o)
+      return H2B_ERR_NOMEM;
+    p->order = o;
+    p->corder = 2 * need;
+  }
+  /* (id, position) sorted by merging ascending runs: the list comes in one run per vertex */
+  src = p->order;
+  dst = src + n;
+  for (i = 0; i < n; i++)
+    src[i] = (uint64_t) r[i].t << 32 | i;
+  for (;;) {
+    uint32_t o = 0, runs = 0;
+    uint64_t *swap;
+    while (o < n) {
+      uint32_t x = o, m = o + 1, y, e, w = o;
+      while (m < n && src[m] > src[m - 1])
+        m++;
+      for (e = y = m; e < n && (e == m || src[e] > src[e - 1]); e++)
+        ;
+      while (x < m && y < e)
+        dst[w++] = src[x] < src[y] ? src[x++] : src[y++];
+      while (x < m)
+        dst[w++] = src[x++];
+      while (y < e)
+        dst[w++] = src[y++];
+      o = e;
+      runs++;
+    }
+    swap = src;
+    src = dst;
+    dst = swap;
+    if (runs <= 1)
+      break;
+  }
+  tmp = (h2b_triref *) (p->order + 2 * (size_t) n);
+  memcpy(tmp, r, sizeof(*r) * n);
+  for (i = 0; i < n; i++) {
+    const uint32_t *v;
+    int at[3] = {-1, -1, -1}, j, s;
+    uint32_t placed = 0;
+    r[i] = tmp[(uint32_t) src[i]];
+    v = adj->t + 3 * (size_t) r[i].t;
+    for (j = 0; j < 3; j++)
+      for (s = 0; s < 3; s++)
+        if (at[s] < 0 && v[j] == held[s]) {
+          at[s] = j;
+          placed |= 1u << j;
+          break;
+        }
+    for (j = 0; j < 3; j++)
+      if (!(placed >> j & 1u)) {
+        for (s = 0; at[s] >= 0; s++)
+          ;
+        at[s] = j;
+      }
+    for (s = 0; s < 3; s++)
+      held[s] = v[at[s]];
+    r[i].slots = (int16_t) (at[0] | at[1] << 2 | at[2] << 4);
+  }
+  return H2B_OK;
+}
+
 /* Append the triangle list of an index range; returns its offset in p->refs. */
 static int
 add_reflist(h2b_nearplan *p, h2b_adjacency *adj, int linear, const uint32_t *idx, uint32_t n,
@@ -152,7 +229,7 @@ add_reflist(h2b_nearplan *p, h2b_adjacency *adj, int linear, const uint32_t *idx
       h2b_triref *r = &p->refs[p->nrefs++];
       r->t = idx[i];
       r->l[0] = r->l[1] = r->l[2] = (int16_t) i;
-      r->pad = 0;
+      r->slots = 0;
     }
   }
   else {
@@ -178,7 +255,7 @@ add_reflist(h2b_nearplan *p, h2b_adjacency *adj, int linear, const uint32_t *idx
           uint32_t w = adj->t[3 * (size_t) tt + k];
           r->l[k] = (adj->vstamp[w] == gv) ? (int16_t) adj->vloc[w] : (int16_t) -1;
         }
-        r->pad = 0;
+        r->slots = 0;
       }
     }
   }
@@ -251,6 +328,8 @@ cached_reflist(h2b_nearplan *p, h2b_adjacency *adj, int linear, const uint32_t *
   }
   if ((rc = add_reflist(p, adj, linear, idx, n, off, len)) != H2B_OK)
     return rc;
+  if (linear && (rc = order_list(p, adj, *off, *len)) != H2B_OK)
+    return rc;
   p->lkey[i] = idx;
   p->lkn[i] = kn;
   p->loff[i] = *off;
@@ -288,7 +367,7 @@ add_tile(h2b_nearplan *p, h2b_adjacency *adj, int row_linear, int col_linear,
   tl->rows = (uint16_t) rows;
   tl->cols = (uint16_t) cols;
   tl->flags = ntrans ? 1u : 0u;
-  tl->pad = 0;
+  tl->mate = 0;
 
   if (p->skip_sing) {
     p->ntiles++;
@@ -351,6 +430,45 @@ h2b_nearplan_add_block(h2b_nearplan *p, h2b_adjacency *adj, int row_basis, int c
     }
   }
   return H2B_OK;
+}
+
+void
+h2b_nearplan_mate(h2b_nearplan *p, uint32_t t0, uint32_t t1, uint32_t nr, uint32_t nc)
+{
+  uint32_t i, j;
+  for (j = 0; j < nc; j++)
+    for (i = 0; i < nr; i++) {
+      const uint32_t a = t0 + i + j * nr, b = t1 + j + i * nc;
+      if (a == b)
+        continue;
+      p->tiles[a].mate = b + 1;
+      p->tiles[b].mate = a + 1;
+    }
+}
+
+uint32_t
+h2b_nearplan_halves(const h2b_nearplan *p, uint32_t *list)
+{
+  uint32_t cnt[8] = {0}, start[8], i, b, n = 0;
+  uint64_t most = 1;
+#define WORK(T) ((uint64_t) (T).tr_len * (T).sc_len)
+#define SKIP(I) (p->tiles[I].mate && p->tiles[I].mate - 1 < (I))
+  for (i = 0; i < p->ntiles; i++)
+    if (WORK(p->tiles[i]) > most)
+      most = WORK(p->tiles[i]);
+  for (i = 0; i < p->ntiles; i++)
+    if (!SKIP(i))
+      cnt[7 - (WORK(p->tiles[i]) * 7 + most - 1) / most]++;
+  for (b = 0; b < 8; b++) {
+    start[b] = n;
+    n += cnt[b];
+  }
+  for (i = 0; i < p->ntiles; i++)
+    if (!SKIP(i))
+      list[start[7 - (WORK(p->tiles[i]) * 7 + most - 1) / most]++] = i;
+#undef SKIP
+#undef WORK
+  return n;
 }
 
 /* Stable counting sort of the singular pairs by case (1 vertex, 2 edge, 3 identical), so that

@@ -6,6 +6,9 @@
 //     triangle pair (no shared vertex, q^4 tensor points, fully unrolled with the rule in
 //     constant memory); pair results are accumulated in a shared-memory tile and the tile is
 //     written to HBM once with coalesced column-major stores.  Singular pairs are skipped here.
+//     It serves the regular orders other than 2, the FP32 quadrature and row-linear bases with
+//     constant columns; the q = 2 FP64 kernels are near_ring_kernel (linear columns) and
+//     near_pair_kernel (constant bases), which fill a tile and its transposed block's tile together.
 //   * near_sing_kernel — one warp per singular pair (vertex: 2 q2^4 points; edge: 6 q2^3 and
 //     identical: 6 q2^2 kernel evaluations, the rules reduced on the host because X - Y does not
 //     depend on the inner Gauss variables there, see h2b_quad_reduce), lanes stride over the
@@ -451,7 +454,9 @@ __device__ __forceinline__ void dist_pair_tensor_f32(const PairGeo &g, double n0
 struct DistArgs {
   const TriRec *tri;
   const TriRef *refs;
+  const QuadRec *qrec;
   const h2b_tile *tiles;
+  const uint32_t *list;  // the tiles to run (NULL: all)
   double *out0, *out1;
   double kconst, k_re, k_imn;
   int q;  // runtime q for the generic variant
@@ -759,6 +764,566 @@ __global__ void __launch_bounds__(dist_threads<KK>(), dist_minblocks<KK>())
   }
 }
 
+// ---------------------------------------------------------------------------------------------
+// Distant pairs with mates (q = 2, FP64)
+//
+// A nearfield block and its transposed block (rows and columns exchanged, equal index lists) take the
+// same triangle pairs, and the distant rule is the same on both triangles: the pair (t, s) of one
+// and (s, t) of the other share every point pair, its distance, the inverse root and, for
+// Helmholtz kernels, its sine and cosine.  A kernel with MIR = true therefore fills a tile and its
+// mate together: a single layer value is an entry of both; for a double layer the mate's value takes
+// the other triangle's normal, which makes it the adjoint kernel at (x, y), one or two channels
+// more.  (The singular rules are not symmetric under the exchange; those pairs stay separate.)
+
+// Channels of a tile: the kernel's own, then with MIR those of the mate that are not the same.
+template <int KK, bool MIR>
+struct Chan {
+  static constexpr bool SLP = KK == KK_LSLP || KK == KK_HSLP;
+  static constexpr int OWN = KT<KK>::NCH;
+  static constexpr int W = KT<KK>::CPLX ? 2 : 1;
+  static constexpr int ALL = OWN + (MIR && !SLP ? W : 0);
+  // the normals taken: column triangle's (own double layer, mate's adjoint), row triangle's
+  static constexpr bool DC = uses_normal<KK>() && (MIR || !row_normal<KK>());
+  static constexpr bool DR = uses_normal<KK>() && (MIR || row_normal<KK>());
+};
+
+// All channels from r^2 = |x - y|^2, dc = <x - y, n> with the column triangle's normal, dr with the
+// row triangle's (each only where Chan says so).
+template <int KK, bool MIR>
+__device__ __forceinline__ void eval_channels(double r2, double dc, double dr, double k_re,
+                                              double k_imn, double (&kv)[Chan<KK, MIR>::ALL]) {
+  constexpr bool ADJ = row_normal<KK>();
+  const double rinv = rsqrt_nr(r2);
+  if constexpr (!KT<KK>::CPLX) {
+    if constexpr (KK == KK_LSLP || KK == KK_LBOTH) kv[0] = rinv;
+    if constexpr (KK != KK_LSLP) {
+      constexpr int D = KK == KK_LBOTH ? 1 : 0;
+      const double r3 = rinv * rinv * rinv;
+      kv[D] = (ADJ ? -dr : dc) * r3;
+      if constexpr (MIR) kv[D + 1] = (ADJ ? dc : -dr) * r3;
+    }
+  } else {
+    const double r = r2 * rinv, kr = k_re * r;
+    double rn = rinv, s, c;
+    if (k_imn != 0.0) rn *= exp(k_imn * r);
+    sincos(kr, &s, &c);
+    if constexpr (KK == KK_HSLP || KK == KK_HBOTH) {
+      kv[0] = rn * c;
+      kv[1] = rn * s;
+    }
+    if constexpr (KK != KK_HSLP) {
+      constexpr int D = KK == KK_HBOTH ? 2 : 0;
+      const double r3 = rinv * rinv * rn, br = fma(kr, s, c) * r3, bi = fma(-c, kr, s) * r3;
+      const double o = ADJ ? -dr : dc;
+      kv[D] = br * o;
+      kv[D + 1] = bi * o;
+      if constexpr (MIR) {
+        const double m = ADJ ? dc : -dr;
+        kv[D + 2] = br * m;
+        kv[D + 3] = bi * m;
+      }
+    }
+  }
+}
+
+// Accumulator planes: rows of a plane are the tile's rows, PLD apart per column (65 words: the
+// mate's transposed read and the tile's own read are both free of bank conflicts).
+constexpr int PLD = H2B_TILE_MAX + 1, PSZ = PLD * H2B_TILE_MAX;
+
+// Entry o of a complex output (a caller's buffer may be aligned to 8 bytes only).
+__device__ __forceinline__ void put_complex(double *out, uint64_t o, double re, double im) {
+  if ((reinterpret_cast<uintptr_t>(out) & 15u) == 0) {
+    reinterpret_cast<double2 *>(out)[o] = make_double2(re, im);
+  } else {
+    out[2 * o] = re;
+    out[2 * o + 1] = im;
+  }
+}
+
+// A finished tile: entry (r, c) from plane[r + PLD c], or plane[c + PLD r] for the mate.  im: plane of
+// the imaginary parts (complex kernels).
+template <bool CPLX, bool MATE>
+__device__ __forceinline__ void put_tile(double *out, const h2b_tile &tl, const double *re,
+                                         const double *im) {
+  const uint32_t rows = tl.rows, cols = tl.cols;
+  const bool ntrans = tl.flags & 1u;
+  const uint32_t fast = ntrans ? cols : rows;
+  for (uint32_t e = threadIdx.x; e < rows * cols; e += blockDim.x) {
+    const uint32_t hi = e / fast, lo = e - hi * fast, r = ntrans ? hi : lo, c = ntrans ? lo : hi;
+    const uint64_t o = ntrans ? tl.out_off + c + (uint64_t) r * tl.ld
+                              : tl.out_off + r + (uint64_t) c * tl.ld;
+    const uint32_t p = MATE ? c + PLD * r : r + PLD * c;
+    if constexpr (CPLX)
+      put_complex(out, o, re[p], ntrans ? -im[p] : im[p]);
+    else
+      out[o] = re[p];
+  }
+}
+
+// The tile's outputs from its planes, own channels first (linear bases).
+template <int KK, bool MIR>
+__device__ __forceinline__ void put_planes(const DistArgs &a, const h2b_tile &tl,
+                                           const double *pl) {
+  using C = Chan<KK, MIR>;
+  constexpr bool X = KT<KK>::CPLX;
+  put_tile<X, false>(a.out0, tl, pl, pl + PSZ);
+  if constexpr (KT<KK>::NOUT == 2)
+    put_tile<X, false>(a.out1, tl, pl + C::W * PSZ, pl + (C::W + 1) * PSZ);
+  if constexpr (MIR) {
+    if (tl.mate == 0) return;
+    const h2b_tile tm = a.tiles[tl.mate - 1];
+    const double *m = C::SLP ? pl : pl + C::OWN * PSZ;
+    if constexpr (KT<KK>::NOUT == 2) {
+      put_tile<X, true>(a.out0, tm, pl, pl + PSZ);
+      put_tile<X, true>(a.out1, tm, m, m + PSZ);
+    } else {
+      put_tile<X, true>(a.out0, tm, m, m + PSZ);
+    }
+  }
+}
+
+// Linear column basis.  What bounds the scatter of a linear basis is that an FP64 addition to shared
+// memory is a compare-and-swap loop, and a pair has 9 values per channel to add.  Both sides of it
+// are shortened here:
+//   - a warp keeps up to 32 row triangles, one per lane, and walks along the column triangles of its
+//     segment of the list (ordered by id, order_list in host_plan.c).  The sums of the current
+//     triangle's three vertices stay in registers, in slots that a vertex keeps as long as
+//     consecutive triangles share it, and are added to the tile when the walk leaves the vertex:
+//     0.8 instead of 2.3 columns per triangle.
+//   - to add a column, the lanes put their three row values into the warp's buffer and lane i
+//     gathers those of the i-th distinct row vertex (the lists are made once per walk), so that one
+//     addition per row and column reaches the tile, without collisions inside the warp.
+// The column triangle's record comes by one coalesced load a triangle ahead into the warp's own
+// buffer, so that warps only meet at the first and last barrier of a tile.
+//
+// Work is cut into (row group, segment) units; the number of segments is the one that minimises
+// rounds of the CTA's warps times the segment's length, a unit costing about RING_EXTRA triangles
+// more.
+//
+// V and K of 32768 triangles (ellipsoid, leaf 64), ms: a thread per pair with 9 additions per channel
+// 6.66; the walk with additions per lane, no mates 5.62; this kernel 4.29 (FP64 pipe 59 % busy, three
+// warps per scheduler; 15 % of the lanes idle in groups of fewer than 32 row triangles).  Single
+// layer of 16200 triangles 2.02 -> 0.93.
+constexpr uint32_t RING_EXTRA = 3;
+struct RingWarp {
+  double rec[2][22];  // QuadRec of the current and the next column triangle
+  double w[3][4];     // per slot and point: weight times nodal function times Gram determinant, kconst
+  double buf[98];     // row values of a column (3 x 32), a zero, padding
+  uint4 tab[32];      // per distinct row: byte offsets in buf of up to 8 places (96: the zero)
+  double g[32];       // per lane: the row triangle's Gram determinant
+  uint32_t v[3][32];  // and vertex ids
+  uint8_t row[32];    // the distinct rows
+  uint32_t nrow, most, over, pad;  // distinct rows, most places of one, lanes with values outside tab
+};
+
+// Threads and resident CTAs per SM: with up to three planes two CTAs fit an SM's shared memory, six
+// warps each, 170 registers per thread (three channels of 9 sums, the row triangle's points, one
+// kernel evaluation); one plane leaves room for a third of the sums and more warps.
+template <int KK, bool MIR>
+constexpr int ring_threads() { return Chan<KK, MIR>::ALL > 3 ? 256 : Chan<KK, MIR>::ALL == 1 ? 256 : 192; }
+template <int KK, bool MIR>
+constexpr int ring_ctas() { return Chan<KK, MIR>::ALL > 3 ? 1 : 2; }
+
+template <int KK, bool RL, bool MIR>
+__global__ void __launch_bounds__(ring_threads<KK, MIR>(), ring_ctas<KK, MIR>())
+    near_ring_kernel(DistArgs a) {
+  using C = Chan<KK, MIR>;
+  constexpr int NCH = C::ALL, NR = RL ? 3 : 1;
+  constexpr uint32_t T = ring_threads<KK, MIR>(), NW = T / 32;
+  const double(&sd)[6][SIDE_MAXP] = c_side[1];
+  extern __shared__ __align__(16) double sm[];
+  double *planes = sm;                                  // NCH planes
+  double *snod = sm + NCH * PSZ;                        // 3 x 4: weight times nodal function
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  RingWarp &W = reinterpret_cast<RingWarp *>(snod + 12)[warp];
+  const h2b_tile tl = a.tiles[a.list ? a.list[blockIdx.x] : blockIdx.x];
+  for (uint32_t e = tid; e < (uint32_t) (NCH * PSZ); e += T) planes[e] = 0.0;
+  if (tid < 12) snod[tid] = sd[3 + tid / 4][tid & 3u] * a.kconst;
+  const uint32_t ntr = tl.tr_len, nsc = tl.sc_len, ng = (ntr + 31u) / 32u;
+  uint32_t nseg, len;
+  {
+    const uint32_t cand = max(1u, min(lane + 1u, nsc));
+    const uint32_t cost = ((cand * ng + NW - 1) / NW) * ((nsc + cand - 1) / cand + RING_EXTRA);
+    nseg = (__reduce_min_sync(0xffffffffu, cost << 5 | (cand - 1u)) & 31u) + 1u;
+    len = max(1u, (nsc + nseg - 1) / nseg);
+    nseg = (nsc + len - 1) / len;
+  }
+  __syncthreads();
+
+  for (uint32_t u = warp; u < ng * nseg; u += NW) {
+    const uint32_t is = u / ng, ig = u - is * ng;
+    const uint32_t g0 = (uint32_t) ((uint64_t) ig * ntr / ng);
+    const uint32_t ngr = (uint32_t) ((uint64_t) (ig + 1) * ntr / ng) - g0;
+    const bool active = lane < ngr;
+    const TriRef rt = a.refs[tl.tr_off + g0 + (active ? lane : 0u)];
+    const QuadRec &R = a.qrec[rt.t];
+    double x[4][3], nr[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+#pragma unroll
+      for (int d = 0; d < 3; d++) x[q][d] = R.p[q][d];
+    if constexpr (C::DR) {
+#pragma unroll
+      for (int d = 0; d < 3; d++) nr[d] = R.n[d];
+    }
+    __syncwarp();  // the walk before is done with the warp's buffers
+    if (active) W.g[lane] = R.g;
+#pragma unroll
+    for (int i = 0; i < 3; i++) W.v[i][lane] = R.v[i];
+
+    // the lanes' places in the buffer by row vertex.  Values of a 33rd row or a ninth triangle around
+    // a vertex go to the tile lane by lane (bits in over)
+    uint32_t over = 0;
+    if constexpr (RL) {
+      uint32_t *cnt = reinterpret_cast<uint32_t *>(W.buf), *pos = cnt + 64;
+      cnt[lane] = cnt[lane + 32] = 0;
+      W.tab[lane] = make_uint4(0x03000300u, 0x03000300u, 0x03000300u, 0x03000300u);
+      __syncwarp();
+      uint32_t at[3] = {8, 8, 8};
+#pragma unroll
+      for (int i = 0; i < 3; i++)
+        if (active && rt.l[i] >= 0) at[i] = atomicAdd(&cnt[rt.l[i]], 1u);
+      __syncwarp();
+      const uint32_t ca = cnt[lane], cb = cnt[lane + 32], below = (1u << lane) - 1u;
+      const uint32_t ba = __ballot_sync(0xffffffffu, ca > 0), bb = __ballot_sync(0xffffffffu, cb > 0);
+      const uint32_t pa = __popc(ba & below), pb = __popc(ba) + __popc(bb & below);
+      pos[lane] = pa;
+      pos[lane + 32] = pb;
+      if (ca) W.row[pa] = (uint8_t) lane;
+      if (cb && pb < 32u) W.row[pb] = (uint8_t) (lane + 32);
+      const uint32_t most = __reduce_max_sync(0xffffffffu, min(8u, max(ca, cb)));
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < 3; i++)
+        if (active && rt.l[i] >= 0) {
+          const uint32_t p = pos[rt.l[i]];
+          if (at[i] < 8u && p < 32u)
+            reinterpret_cast<uint16_t *>(&W.tab[p])[at[i]] = (uint16_t) (8 * (i * 32 + lane));
+          else
+            over |= 1u << i;
+        }
+      const uint32_t anyover = __any_sync(0xffffffffu, over != 0);
+      __syncwarp();
+      if (lane == 0) {
+        W.nrow = min(32u, (uint32_t) (__popc(ba) + __popc(bb)));
+        W.most = most;
+        W.over = anyover;
+        W.buf[96] = 0.0;
+      }
+    }
+
+    double acc[NCH][NR][3];
+    int cur[3] = {-1, -1, -1};
+#pragma unroll
+    for (int c = 0; c < NCH; c++)
+#pragma unroll
+      for (int i = 0; i < NR; i++) acc[c][i][0] = acc[c][i][1] = acc[c][i][2] = 0.0;
+    // the sums v of a slot to column col of the planes
+    auto flush = [&](int col, const double (&v)[NCH][NR]) {
+      double *dst = planes + PLD * col;
+      const double gr = W.g[lane];
+#pragma unroll
+      for (int c = 0; c < NCH; c++) {
+        if constexpr (!RL) {
+          // constant row basis: a row per lane
+          if (active && rt.l[0] >= 0) atomicAdd(&dst[c * PSZ + rt.l[0]], v[c][0] * gr);
+        } else {
+          __syncwarp();
+#pragma unroll
+          for (int i = 0; i < 3; i++) W.buf[i * 32 + lane] = v[c][i] * gr;
+          __syncwarp();
+          if (lane < W.nrow) {
+            const uint4 mine = W.tab[lane];
+            const char *bb = reinterpret_cast<const char *>(W.buf);
+            auto two = [&](uint32_t o) {
+              return *reinterpret_cast<const double *>(bb + (o & 0xffffu)) +
+                     *reinterpret_cast<const double *>(bb + (o >> 16));
+            };
+            double t = two(mine.x) + two(mine.y) + two(mine.z);
+            if (W.most > 6u) t += two(mine.w);
+            atomicAdd(&dst[c * PSZ + W.row[lane]], t);
+          }
+          if (W.over) {
+#pragma unroll
+            for (int i = 0; i < 3; i++)
+              if (over >> i & 1u)
+                atomicAdd(&dst[c * PSZ + a.refs[tl.tr_off + g0 + lane].l[i]], W.buf[i * 32 + lane]);
+          }
+        }
+      }
+    };
+    // the walk: lane j holds entry e0 + j of the list (triangle, slots); lanes 0 to 21 copy a word of the
+    // next record each
+    const uint32_t first = is * len, last = min(nsc, first + len);
+    uint32_t e0 = first, tri = 0, slots = 0;
+    auto load_refs = [&]() {
+      const TriRef r = a.refs[tl.sc_off + min(e0 + lane, last - 1u)];
+      tri = r.t;
+      const uint32_t p = (uint32_t) r.slots;
+      slots = p << 24;
+#pragma unroll
+      for (int s = 0; s < 3; s++) {
+        const uint32_t j = p >> (2 * s) & 3u;
+        const int l = j == 0 ? r.l[0] : j == 1 ? r.l[1] : r.l[2];
+        slots |= ((uint32_t) l & 255u) << (8 * s);
+      }
+    };
+    auto copy_rec = [&](uint32_t e) {
+      const uint32_t t = __shfl_sync(0xffffffffu, tri, (int) (e - e0));
+      if (lane < 22u)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                         (uint32_t) __cvta_generic_to_shared(&W.rec[e & 1u][lane])),
+                     "l"(reinterpret_cast<const double *>(a.qrec + t) + lane)
+                     : "memory");
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    load_refs();
+    copy_rec(first);
+#pragma unroll 1
+    for (uint32_t e = first;; e++) {
+      // after the last triangle every slot is left
+      const uint32_t sl = e < last ? __shfl_sync(0xffffffffu, slots, (int) (e - e0)) : 0x00ffffffu;
+#pragma unroll 1
+      for (int s = 0; s < 3; s++) {
+        const int nx = (int) (int8_t) (sl >> (8 * s));
+        int was = nx;
+        double v[NCH][NR];
+        auto leave = [&](auto k) {
+          constexpr int K = decltype(k)::value;
+          was = cur[K];
+          cur[K] = nx;
+          if (was == nx) return;
+#pragma unroll
+          for (int c = 0; c < NCH; c++)
+#pragma unroll
+            for (int i = 0; i < NR; i++) {
+              v[c][i] = acc[c][i][K];
+              acc[c][i][K] = 0.0;
+            }
+        };
+        if (s == 0) leave(std::integral_constant<int, 0>());
+        else if (s == 1) leave(std::integral_constant<int, 1>());
+        else leave(std::integral_constant<int, 2>());
+        if (was != nx && was >= 0) flush(was, v);
+      }
+      if (e == last) break;
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncwarp();  // the record is there, and every lane is done with the one before
+      if (e + 1 < last) {
+        if (e + 1 - e0 == 32u) {
+          e0 += 32u;
+          load_refs();
+        }
+        copy_rec(e + 1);
+      }
+      const QuadRec &S = *reinterpret_cast<const QuadRec *>(W.rec[e & 1u]);
+      if (lane < 12u)
+        W.w[lane >> 2][lane & 3u] =
+            snod[(sl >> (24 + 2 * (lane >> 2)) & 3u) * 4 + (lane & 3u)] * S.g;
+      __syncwarp();
+      {
+        const uint32_t tv0 = W.v[0][lane], tv1 = W.v[1][lane], tv2 = W.v[2][lane];
+        const uint32_t sv0 = S.v[0], sv1 = S.v[1], sv2 = S.v[2];
+        if (!active || tv0 == sv0 || tv0 == sv1 || tv0 == sv2 || tv1 == sv0 || tv1 == sv1 ||
+            tv1 == sv2 || tv2 == sv0 || tv2 == sv1 || tv2 == sv2)
+          continue;
+      }
+      double dxc[4] = {0.0, 0.0, 0.0, 0.0};  // <x_q, n> with the column triangle's normal
+      if constexpr (C::DC) {
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+          dxc[q] = fma(x[q][0], S.n[0], fma(x[q][1], S.n[1], x[q][2] * S.n[2]));
+      }
+      // row side first: the four kernel values of a column point are independent chains
+#pragma unroll 1
+      for (int b = 0; b < 4; b++) {
+        const double y0 = S.p[b][0], y1 = S.p[b][1], y2 = S.p[b][2];
+        const double dyc = C::DC ? S.p[b][3] : 0.0;
+        double in[NCH][NR];
+#pragma unroll
+        for (int c = 0; c < NCH; c++)
+#pragma unroll
+          for (int i = 0; i < NR; i++) in[c][i] = 0.0;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          const double dx = x[q][0] - y0, dy = x[q][1] - y1, dz = x[q][2] - y2;
+          const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+          // (the row normal's component from the difference: keeping it per point takes 8 registers)
+          const double dr = C::DR ? fma(dx, nr[0], fma(dy, nr[1], dz * nr[2])) : 0.0;
+          double kv[NCH];
+          eval_channels<KK, MIR>(r2, dxc[q] - dyc, dr, a.k_re, a.k_imn, kv);
+#pragma unroll
+          for (int c = 0; c < NCH; c++)
+#pragma unroll
+            for (int i = 0; i < NR; i++)
+              in[c][i] = fma(sd[RL ? 3 + i : 2][q], kv[c], in[c][i]);
+        }
+#pragma unroll
+        for (int s = 0; s < 3; s++) {
+          const double w = W.w[s][b];
+#pragma unroll
+          for (int c = 0; c < NCH; c++)
+#pragma unroll
+            for (int i = 0; i < NR; i++) acc[c][i][s] = fma(w, in[c][i], acc[c][i][s]);
+        }
+      }
+    }
+  }
+  __syncthreads();
+  put_planes<KK, MIR>(a, tl, planes);
+}
+
+// Constant bases: a pair is an entry.  A thread per pair, lanes on consecutive row triangles (column
+// triangles with ntrans), from staged points; the tile's own entries go straight to memory, the
+// mate's through planes, transposed.  Dense single layer of 8192 triangles: without mates 1.07 ms,
+// with mates 0.57; fused Helmholtz kinds of 49152 triangles, leaf 64: 4.37 -> 2.43.
+template <int KK, bool MIR>
+constexpr int pair_planes() { return !MIR ? 0 : Chan<KK, MIR>::SLP || KT<KK>::NOUT == 1 ? Chan<KK, MIR>::W : 2 * Chan<KK, MIR>::W; }
+template <int KK, bool MIR>
+constexpr int pair_threads() { return pair_planes<KK, MIR>() > 2 ? 512 : 256; }
+
+template <int KK, bool MIR>
+__global__ void __launch_bounds__(pair_threads<KK, MIR>(), pair_planes<KK, MIR>() > 2 ? 1 : 2)
+    near_pair_kernel(DistArgs a) {
+  using C = Chan<KK, MIR>;
+  constexpr int NCH = C::ALL, NPL = pair_planes<KK, MIR>();
+  constexpr bool X = KT<KK>::CPLX;
+  constexpr uint32_t T = pair_threads<KK, MIR>();
+  const double(&sd)[6][SIDE_MAXP] = c_side[1];
+  extern __shared__ __align__(16) double sm[];
+  double *planes = sm;
+  DistStagePts &sg = *reinterpret_cast<DistStagePts *>(sm + NPL * PSZ);
+  const h2b_tile tl = a.tiles[a.list ? a.list[blockIdx.x] : blockIdx.x];
+  const bool ntrans = tl.flags & 1u;
+  // a tile has at most 64 triangles per side: one stage
+  const uint32_t nr = tl.tr_len, nc = tl.sc_len;
+  for (uint32_t e = threadIdx.x; e < nr + nc; e += T) {
+    const bool row = e < nr;
+    const uint32_t i = row ? e : e - nr;
+    const TriRef rf = a.refs[(row ? tl.tr_off : tl.sc_off) + i];
+    const TriRec &S = a.tri[rf.t];
+    stage_points(row ? sg.r : sg.c, i, S, row ? 1.0 : a.kconst);
+#pragma unroll
+    for (int d = 0; d < 3; d++) (row ? sg.rv : sg.cv)[d][i] = S.v[d];
+    (row ? sg.rl : sg.cl)[0][i] = rf.l[0];
+  }
+  __syncthreads();
+  const uint32_t nf = ntrans ? nc : nr, np = nr * nc;
+  uint32_t hi = threadIdx.x / nf, lo = threadIdx.x - hi * nf;
+  const uint32_t dq = T / nf, dr = T - dq * nf;
+  for (uint32_t p = threadIdx.x; p < np; p += T) {
+    const uint32_t ri = ntrans ? hi : lo, ci = ntrans ? lo : hi;
+    hi += dq;
+    lo += dr;
+    if (lo >= nf) {
+      lo -= nf;
+      hi++;
+    }
+    double acc[NCH];
+#pragma unroll
+    for (int c = 0; c < NCH; c++) acc[c] = 0.0;
+    const uint32_t tv0 = sg.rv[0][ri], tv1 = sg.rv[1][ri], tv2 = sg.rv[2][ri];
+    const uint32_t sv0 = sg.cv[0][ci], sv1 = sg.cv[1][ci], sv2 = sg.cv[2][ci];
+    if (!(tv0 == sv0 || tv0 == sv1 || tv0 == sv2 || tv1 == sv0 || tv1 == sv1 || tv1 == sv2 ||
+          tv2 == sv0 || tv2 == sv1 || tv2 == sv2)) {
+      double y[4][3], dyc[4], dyr[4], ncl[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+      for (int b = 0; b < 4; b++) {
+#pragma unroll
+        for (int d = 0; d < 3; d++) y[b][d] = sg.c[PT_X + 3 * b + d][ci];
+        dyc[b] = C::DC ? sg.c[PT_DN + b][ci] : 0.0;
+        dyr[b] = C::DR ? fma(y[b][0], sg.r[PT_N][ri],
+                             fma(y[b][1], sg.r[PT_N + 1][ri], y[b][2] * sg.r[PT_N + 2][ri]))
+                       : 0.0;
+      }
+      if constexpr (C::DC) {
+#pragma unroll
+        for (int d = 0; d < 3; d++) ncl[d] = sg.c[PT_N + d][ci];
+      }
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const double x0 = sg.r[PT_X + 3 * q][ri], x1 = sg.r[PT_X + 3 * q + 1][ri],
+                     x2 = sg.r[PT_X + 3 * q + 2][ri];
+        const double dxc = C::DC ? fma(x0, ncl[0], fma(x1, ncl[1], x2 * ncl[2])) : 0.0;
+        const double dxr = C::DR ? sg.r[PT_DN + q][ri] : 0.0;
+        double in[NCH];
+#pragma unroll
+        for (int c = 0; c < NCH; c++) in[c] = 0.0;
+#pragma unroll
+        for (int b = 0; b < 4; b++) {
+          const double dx = x0 - y[b][0], dy = x1 - y[b][1], dz = x2 - y[b][2];
+          const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+          double kv[NCH];
+          eval_channels<KK, MIR>(r2, dxc - dyc[b], dxr - dyr[b], a.k_re, a.k_imn, kv);
+#pragma unroll
+          for (int c = 0; c < NCH; c++) in[c] = fma(sd[2][b], kv[c], in[c]);
+        }
+#pragma unroll
+        for (int c = 0; c < NCH; c++) acc[c] = fma(sd[2][q], in[c], acc[c]);
+      }
+      const double f2 = sg.c[PT_G][ci] * sg.r[PT_G][ri];
+#pragma unroll
+      for (int c = 0; c < NCH; c++) acc[c] *= f2;
+    }
+    const int lr = sg.rl[0][ri], lc = sg.cl[0][ci];
+    const uint64_t o = ntrans ? tl.out_off + lc + (uint64_t) lr * tl.ld
+                              : tl.out_off + lr + (uint64_t) lc * tl.ld;
+    if constexpr (X) {
+      put_complex(a.out0, o, acc[0], ntrans ? -acc[1] : acc[1]);
+      if constexpr (KT<KK>::NOUT == 2) put_complex(a.out1, o, acc[2], ntrans ? -acc[3] : acc[3]);
+    } else {
+      a.out0[o] = acc[0];
+      if constexpr (KT<KK>::NOUT == 2) a.out1[o] = acc[1];
+    }
+    if constexpr (MIR) {
+      const int e = lr + PLD * lc;
+      constexpr int M = C::SLP ? 0 : C::OWN;  // the mate's channels of the last output
+      if constexpr (KT<KK>::NOUT == 2) {
+#pragma unroll
+        for (int w = 0; w < C::W; w++) {
+          planes[w * PSZ + e] = acc[w];
+          planes[(C::W + w) * PSZ + e] = acc[M + w];
+        }
+      } else {
+#pragma unroll
+        for (int w = 0; w < C::W; w++) planes[w * PSZ + e] = acc[M + w];
+      }
+    }
+  }
+  if constexpr (MIR) {
+    if (tl.mate == 0) return;
+    __syncthreads();
+    const h2b_tile tm = a.tiles[tl.mate - 1];
+    put_tile<X, true>(a.out0, tm, planes, planes + PSZ);
+    if constexpr (KT<KK>::NOUT == 2)
+      put_tile<X, true>(a.out1, tm, planes + C::W * PSZ, planes + (C::W + 1) * PSZ);
+  }
+}
+
+// The QuadRec of every triangle: the points of stage_points.
+__global__ void quad_record_kernel(const TriRec *tri, uint32_t nt, QuadRec *out) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= nt) return;
+  const double(&sd)[6][SIDE_MAXP] = c_side[1];
+  const TriRec &T = tri[t];
+  QuadRec r;
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+#pragma unroll
+    for (int d = 0; d < 3; d++)
+      r.p[q][d] = fma(sd[1][q], T.c[d] - T.b[d], fma(sd[0][q], T.b[d] - T.a[d], T.a[d]));
+    r.p[q][3] = fma(r.p[q][0], T.n[0], fma(r.p[q][1], T.n[1], r.p[q][2] * T.n[2]));
+  }
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    r.n[d] = T.n[d];
+    r.v[d] = T.v[d];
+  }
+  r.g = T.g;
+  r.pad = 0;
+  out[t] = r;
+}
+
 struct SingArgs {
   const TriRec *tri;
   const TriRef *refs;
@@ -991,28 +1556,85 @@ __global__ void __launch_bounds__(SING_THREADS, 1) near_sing_kernel(SingArgs a) 
   }
 }
 
-template <int Q, int KK, bool RL, bool CL, bool F32 = false>
-int launch_dist(const h2b_near_launch *L, cudaStream_t st) {
-  constexpr int PLANES = KT<KK>::NCH;
-  const size_t smem = sizeof(double) * PLANES * H2B_TILE_MAX * H2B_TILE_MAX +
-                      sizeof(DistStageOf<Q, F32>);
-  H2B_CUDA_TRY((h2b_allow_smem<near_dist_kernel<Q, KK, RL, CL, F32>>()));
+DistArgs dist_args(const h2b_near_launch *L) {
   DistArgs a;
   a.tri = (const TriRec *) L->tri;
   a.refs = (const TriRef *) L->refs;
+  a.qrec = (const QuadRec *) L->qrec;
   a.tiles = L->tiles;
+  a.list = nullptr;
   a.out0 = L->out0;
   a.out1 = L->out1;
   a.kconst = L->kconst;
   a.k_re = L->k_re;
   a.k_imn = L->k_imn;
   a.q = (int) L->q;
+  return a;
+}
+
+template <int Q, int KK, bool RL, bool CL, bool F32 = false>
+int launch_dist(const h2b_near_launch *L, cudaStream_t st) {
+  constexpr int PLANES = KT<KK>::NCH;
+  const size_t smem = sizeof(double) * PLANES * H2B_TILE_MAX * H2B_TILE_MAX +
+                      sizeof(DistStageOf<Q, F32>);
+  H2B_CUDA_TRY((h2b_allow_smem<near_dist_kernel<Q, KK, RL, CL, F32>>()));
   if (L->ntiles > 0) {
-    near_dist_kernel<Q, KK, RL, CL, F32><<<L->ntiles, dist_threads<KK>(), smem, st>>>(a);
+    near_dist_kernel<Q, KK, RL, CL, F32>
+        <<<L->ntiles, dist_threads<KK>(), smem, st>>>(dist_args(L));
     h2b_note_launch();
   }
   H2B_CUDA_TRY(cudaGetLastError());
   return H2B_OK;
+}
+
+// MIR: the tiles of L->half fill their mates too; otherwise every tile by itself.
+template <int KK, bool RL, bool MIR>
+int launch_ring(const h2b_near_launch *L, cudaStream_t st) {
+  constexpr int T = ring_threads<KK, MIR>();
+  const size_t smem =
+      sizeof(double) * (Chan<KK, MIR>::ALL * PSZ + 12) + sizeof(RingWarp) * (T / 32);
+  H2B_CUDA_TRY((h2b_allow_smem<near_ring_kernel<KK, RL, MIR>>()));
+  DistArgs a = dist_args(L);
+  a.list = MIR ? L->half : nullptr;
+  const uint32_t n = MIR ? L->nhalf : L->ntiles;
+  if (n > 0) {
+    near_ring_kernel<KK, RL, MIR><<<n, T, smem, st>>>(a);
+    h2b_note_launch();
+  }
+  H2B_CUDA_TRY(cudaGetLastError());
+  return H2B_OK;
+}
+
+template <int KK, bool MIR>
+int launch_pair_kernel(const h2b_near_launch *L, cudaStream_t st) {
+  const size_t smem = sizeof(double) * pair_planes<KK, MIR>() * PSZ + sizeof(DistStagePts);
+  H2B_CUDA_TRY((h2b_allow_smem<near_pair_kernel<KK, MIR>>()));
+  DistArgs a = dist_args(L);
+  a.list = MIR ? L->half : nullptr;
+  const uint32_t n = MIR ? L->nhalf : L->ntiles;
+  if (n > 0) {
+    near_pair_kernel<KK, MIR><<<n, pair_threads<KK, MIR>(), smem, st>>>(a);
+    h2b_note_launch();
+  }
+  H2B_CUDA_TRY(cudaGetLastError());
+  return H2B_OK;
+}
+
+// The q = 2 FP64 kernel of a pair of bases.  Mates need equal bases; the fused Helmholtz kinds with
+// linear bases would need six planes (200 KB), which leaves no room for the warps' buffers.
+template <int KK, bool RL, bool CL>
+int launch_dist2(const h2b_near_launch *L, cudaStream_t st) {
+  if constexpr (RL && CL) {
+    if constexpr (KK != KK_HBOTH)
+      if (L->half) return launch_ring<KK, true, true>(L, st);
+    return launch_ring<KK, true, false>(L, st);
+  } else if constexpr (CL) {
+    return launch_ring<KK, false, false>(L, st);
+  } else if constexpr (RL) {
+    return launch_dist<2, KK, RL, CL>(L, st);
+  } else {
+    return L->half ? launch_pair_kernel<KK, true>(L, st) : launch_pair_kernel<KK, false>(L, st);
+  }
 }
 
 template <int KK, bool RL, bool CL, int PART>
@@ -1079,7 +1701,7 @@ int launch_kk_basis(const h2b_near_launch *L, cudaStream_t st) {
   if (L->q == 2 && L->fp32)
     rc = launch_dist<2, KK, RL, CL, true>(L, st);
   else if (L->q == 2)
-    rc = launch_dist<2, KK, RL, CL>(L, st);
+    rc = launch_dist2<KK, RL, CL>(L, st);
   else
     rc = launch_dist<0, KK, RL, CL>(L, st);
   if (rc != H2B_OK) return rc;
@@ -1654,6 +2276,13 @@ extern "C" int h2b_near_upload_dist_rules(void) {
     for (int r = 0; r < 6; r++)
       for (int p = 0; p < SIDE_MAXP; p++) side_f[q][r][p] = (float) side[q][r][p];
   H2B_CUDA_TRY(cudaMemcpyToSymbol(c_side_f, side_f, sizeof(side_f)));
+  return H2B_OK;
+}
+
+extern "C" int h2b_near_quad_records(const void *tri, uint32_t nt, void *qrec, cudaStream_t st) {
+  quad_record_kernel<<<(nt + 127) / 128, 128, 0, st>>>((const TriRec *) tri, nt, (QuadRec *) qrec);
+  h2b_note_launch();
+  H2B_CUDA_TRY(cudaGetLastError());
   return H2B_OK;
 }
 

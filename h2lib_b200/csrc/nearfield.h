@@ -27,8 +27,11 @@ typedef struct {
   uint32_t q;                    /* regular order: distant pairs use q^4 points */
   const void *tri;               /* TriRec[triangles] */
   const void *refs;              /* TriRef pool */
+  const void *qrec;              /* QuadRec[triangles] */
   const h2b_tile *tiles;
   uint32_t ntiles;
+  const uint32_t *half;          /* tiles to run when mates are filled together (NULL: no mates) */
+  uint32_t nhalf;
   const h2b_sing *sing;          /* sorted by case */
   uint32_t nsing;
   uint32_t nvert;                /* vertex pairs at the start of sing (UINT32_MAX: not known) */
@@ -47,6 +50,8 @@ typedef struct {
 } h2b_near_launch;
 
 int h2b_near_upload_dist_rules(void);
+/* The QuadRec of every triangle (after h2b_near_upload_dist_rules). */
+int h2b_near_quad_records(const void *tri, uint32_t nt, void *qrec, cudaStream_t st);
 /* Singular pairs of a tile list on the device (the pairs that share a vertex, with the vertex
  * permutation code of h2b_pair_code).  vt_off / vt_tri: the surface's vertex -> triangle lists
  * (CSR).  sing == NULL: add the number of pairs of each case c to cursor[c] (c = 1 vertex,
