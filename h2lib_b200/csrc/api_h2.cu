@@ -218,6 +218,7 @@ extern "C" void h2b_h2matrix_del(h2b_h2matrix *h) {
     devtree_free(h->rt, st);
     devtree_free(h->ct, st);
     dfree(h->d_adm_rc, st); dfree(h->d_adm_cc, st);
+    dfree(h->d_st_rc, st); dfree(h->d_st_cc, st); dfree(h->d_spos, st);
     dfree(h->d_near_rc, st); dfree(h->d_near_cc, st); dfree(h->d_near_off, st);
     dfree(h->d_tiles, st); dfree(h->d_half, st); dfree(h->d_refs, st); dfree(h->d_sing, st);
     dfree(h->d_xs, st); dfree(h->d_ys, st); dfree(h->d_ws, st); dfree(h->d_wsl, st);
@@ -280,7 +281,7 @@ static std::vector<uint32_t> transposed_blocks(const std::vector<uint32_t> &rc,
 // The structure of an H2 matrix of rank k (every cluster basis padded to k columns); m is the
 // interpolation order of the Chebyshev path (1 for the greenhybrid bases, which use no nodes).
 static h2b_h2matrix *h2matrix_create(const h2b_bem *bem, const h2b_tree *tree, uint32_t m,
-                                     uint32_t k) {
+                                     uint32_t k, int interpolation) {
   const uint32_t nr = h2b_bem_rows(bem), nc = h2b_bem_cols(bem);
   if (tree->row.nidx != nr || tree->col.nidx != nc) {
     h2b_set_error("h2b_h2matrix_new: tree index sets (%u, %u) do not match the operator (%u, %u)",
@@ -296,6 +297,7 @@ static h2b_h2matrix *h2matrix_create(const h2b_bem *bem, const h2b_tree *tree, u
   h->cx = bem->pde == H2B_HELMHOLTZ;
   h->num_sms = bem->s->num_sms;
   h->same = same_sides(bem, tree);
+  h->sym_coupling = h->same && interpolation;
   int rc = H2B_OK;
   if (cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking) != cudaSuccess) {
     h2b_set_error("h2b_h2matrix_new: %s", cudaGetErrorString(cudaGetLastError()));
@@ -357,6 +359,23 @@ static h2b_h2matrix *h2matrix_create(const h2b_bem *bem, const h2b_tree *tree, u
       rc = H2B_ERR_CUDA;
     }
   h->nadm = (uint32_t) arc.size();
+  // the coupling matrices to store: of two transposed blocks with each other's transposes the first
+  std::vector<uint32_t> src, scc;
+  if (rc == H2B_OK) {
+    std::vector<uint32_t> mate;
+    if (h->sym_coupling) mate = transposed_blocks(arc, acc, tree->row.n);
+    h->h_spos.resize(arc.size());
+    for (uint32_t b = 0; b < arc.size(); b++) {
+      if (h->sym_coupling && mate[b] < b) {
+        h->h_spos[b] = h->h_spos[mate[b]] | 1u;
+        continue;
+      }
+      h->h_spos[b] = 2u * (uint32_t) src.size();
+      src.push_back(arc[b]);
+      scc.push_back(acc[b]);
+    }
+  }
+  h->nstored = (uint32_t) src.size();
   h->nnear = (uint32_t) nrc.size();
   h->near_total = ntot;
   h->ntiles = plan.ntiles;
@@ -365,11 +384,13 @@ static h2b_h2matrix *h2matrix_create(const h2b_bem *bem, const h2b_tree *tree, u
     std::vector<h2b_tile> tiles(plan.tiles, plan.tiles + plan.ntiles);
     std::vector<h2b_triref> refs(plan.refs, plan.refs + plan.nrefs);
     if ((rc = upload(&h->d_adm_rc, arc, h->st)) || (rc = upload(&h->d_adm_cc, acc, h->st)) ||
+        (rc = upload(&h->d_st_rc, src, h->st)) || (rc = upload(&h->d_st_cc, scc, h->st)) ||
+        (rc = upload(&h->d_spos, h->h_spos, h->st)) ||
         (rc = upload(&h->d_near_rc, nrc, h->st)) || (rc = upload(&h->d_near_cc, ncc, h->st)) ||
         (rc = upload(&h->d_near_off, noff, h->st)) || (rc = upload(&h->d_tiles, tiles, h->st)) ||
         (rc = upload(&h->d_half, half, h->st)) || (rc = upload(&h->d_refs, refs, h->st)) ||
         (rc = classify_singular(h, all_pairs))) {
-    } else if (cudaMallocAsync(&h->d_S, sizeof(double) * W * std::max<uint64_t>((uint64_t) h->nadm * h->k * h->k, 1) + H2B_MV_SLACK, h->st) != cudaSuccess ||
+    } else if (cudaMallocAsync(&h->d_S, sizeof(double) * W * std::max<uint64_t>((uint64_t) h->nstored * h->k * h->k, 1) + H2B_MV_SLACK, h->st) != cudaSuccess ||
                cudaMallocAsync(&h->d_N, sizeof(double) * W * std::max<uint64_t>(ntot, 1) + H2B_MV_SLACK, h->st) != cudaSuccess ||
                cudaMallocAsync(&h->d_mverr, sizeof(int), h->st) != cudaSuccess ||
                cudaMemsetAsync(h->d_mverr, 0, sizeof(int), h->st) != cudaSuccess ||
@@ -428,7 +449,7 @@ extern "C" h2b_h2matrix *h2b_h2matrix_new(const h2b_bem *bem, const h2b_tree *tr
     h2b_set_error("h2b_h2matrix_new: interpolation order %u outside 1..5", m);
     return NULL;
   }
-  return h2matrix_create(bem, tree, m, m * m * m);
+  return h2matrix_create(bem, tree, m, m * m * m, 1);
 }
 
 // Per operator: ranks, pivots and transfers of the greenhybrid bases of one tree.
@@ -514,7 +535,7 @@ extern "C" h2b_h2matrix *h2b_h2matrix_new_greenhybrid(const h2b_bem *bem, const 
     }
   }
   const uint32_t ml = m * l, k = 12 * ml * ml;
-  h2b_h2matrix *h = h2matrix_create(bem, tree, 1, k);
+  h2b_h2matrix *h = h2matrix_create(bem, tree, 1, k, 0);
   if (!h) return NULL;
   h->green = 1;
   h->g_ml = (int) ml;
@@ -599,7 +620,7 @@ extern "C" h2b_h2matrix *h2b_h2matrix_new_like(const h2b_bem *bem, const h2b_h2m
   for (DevCTree *t : {&h->rt, &h->ct})
     if (rc == H2B_OK && h->green) rc = green_alloc(*t, h->k, h->st);
   if (rc == H2B_OK &&
-      (cudaMallocAsync(&h->d_S, sizeof(double) * W * std::max<uint64_t>(h->nadm * kk, 1) + H2B_MV_SLACK, h->st) ||
+      (cudaMallocAsync(&h->d_S, sizeof(double) * W * std::max<uint64_t>(h->nstored * kk, 1) + H2B_MV_SLACK, h->st) ||
        cudaMallocAsync(&h->d_N, sizeof(double) * W * std::max<uint64_t>(h->near_total, 1) + H2B_MV_SLACK, h->st) ||
        cudaMallocAsync(&h->d_mverr, sizeof(int), h->st) ||
        cudaMemsetAsync(h->d_mverr, 0, sizeof(int), h->st) ||
@@ -667,12 +688,18 @@ static void build_items(const h2b_h2matrix *h, uint32_t pb, uint32_t fwd_rows, u
                           C.off[c] + c0, R.off[r], h->rt.h_seg[r], H2B_MV_NEAR});
   }
   // coupling blocks, in column panels
+  // of two transposed blocks with each other's transposes the first stands for both
   start[H2B_MV_COUPLING] = (uint32_t) it.size();
-  for (size_t b = 0; b < h->h_arc.size(); b++) {
-    const uint32_t r = h->h_arc[b], c = h->h_acc[b], pc = panel_cols(k);
+  std::vector<char> both(h->nstored, 0);
+  for (uint32_t sp : h->h_spos)
+    if (sp & 1u) both[sp >> 1] = 1;
+  for (uint32_t b = 0; b < h->h_arc.size(); b++) {
+    if (h->h_spos[b] & 1u) continue;
+    const uint32_t r = h->h_arc[b], c = h->h_acc[b], pc = panel_cols(k), at = h->h_spos[b] >> 1;
     for (uint32_t c0 = 0; c0 < k; c0 += pc)
-      it.push_back(MvItem{(uint64_t) b * k * k + (uint64_t) c0 * k, k, std::min(pc, k - c0),
-                          k * c + c0, k * r, h->rt.h_seg[r], H2B_MV_COUPLING});
+      it.push_back(MvItem{(uint64_t) at * k * k + (uint64_t) c0 * k, k, std::min(pc, k - c0),
+                          k * c + c0, k * r, h->rt.h_seg[r],
+                          H2B_MV_COUPLING | (both[at] ? H2B_MV_SYM : 0u)});
   }
   // backward slices, yt_t -> y_t (W_t^T transposed), over every admissible row cluster
   start[H2B_MV_BACKWARD] = (uint32_t) it.size();
@@ -684,14 +711,18 @@ static void build_items(const h2b_h2matrix *h, uint32_t pb, uint32_t fwd_rows, u
   }
   m.n = (uint32_t) it.size();
   for (int q = 0; q < 4; q++) m.start[q] = start[q];
-  m.max_bytes = m.max_rows = m.max_cols_t = m.max_x = 0;
+  m.max_rows = m.max_cols_t = 0;
+  m.per_block = (k + panel_cols(k) - 1) / panel_cols(k);
+  for (int g = 0; g < 3; g++) m.max_bytes[g] = m.max_x[g] = m.max_x2[g] = 0;
   for (const MvItem &e : it) {
     const uint32_t kind = e.flags & H2B_MV_KIND;
     const bool cpx = kind == H2B_MV_NEAR || kind == H2B_MV_COUPLING;
-    m.max_bytes = std::max<uint32_t>(m.max_bytes, e.rows * e.cols * 8u * (cpx ? W : 1u));
+    const int g = kind == H2B_MV_COUPLING ? 1 : kind == H2B_MV_BACKWARD ? 2 : 0;
+    m.max_bytes[g] = std::max<uint32_t>(m.max_bytes[g], e.rows * e.cols * 8u * (cpx ? W : 1u));
     if (!(e.flags & H2B_MV_TRANS)) m.max_rows = std::max(m.max_rows, e.rows);
     else m.max_cols_t = std::max(m.max_cols_t, e.cols);
-    m.max_x = std::max(m.max_x, (e.flags & H2B_MV_TRANS) ? e.rows : e.cols);
+    m.max_x[g] = std::max(m.max_x[g], (e.flags & H2B_MV_TRANS) ? e.rows : e.cols);
+    if (e.flags & H2B_MV_SYM) m.max_x2[g] = std::max(m.max_x2[g], e.rows);
   }
 }
 
@@ -917,7 +948,7 @@ extern "C" int h2b_h2matrix_make_single(h2b_h2matrix *h) {
   if (!h) return H2B_ERR_ARG;
   drop_single(h);
   const uint64_t W = h->cx ? 2 : 1;
-  const uint64_t nN = W * h->near_total, nS = W * (uint64_t) h->nadm * h->k * h->k;
+  const uint64_t nN = W * h->near_total, nS = W * (uint64_t) h->nstored * h->k * h->k;
   const size_t sl = H2B_MV_SLACK;
   if (cudaMallocAsync(&h->f_N, sizeof(float) * std::max<uint64_t>(nN, 1) + sl, h->st) != cudaSuccess ||
       cudaMallocAsync(&h->f_S, sizeof(float) * std::max<uint64_t>(nS, 1) + sl, h->st) != cudaSuccess ||
@@ -1027,7 +1058,7 @@ static int coupling(h2b_h2matrix *h) {
     mark(h, 5);
     return rc;
   }
-  FarCouplingArgs ca{h->d_adm_rc, h->d_adm_cc, h->rt.d_pts, h->ct.d_pts, h->d_S, h->nadm,
+  FarCouplingArgs ca{h->d_st_rc, h->d_st_cc, h->rt.d_pts, h->ct.d_pts, h->d_S, h->nstored,
                      (int) h->m, (int) h->k, h->bem->kconst, h->bem->k_re, -h->bem->k_im};
   int rc = h2b_far_coupling(&ca, h->cx, h->st);
   mark(h, 5);
@@ -1247,6 +1278,33 @@ extern "C" int h2b_h2matrix_info(const h2b_h2matrix *h, uint64_t info[8]) {
   return H2B_OK;
 }
 
+// The coupling matrices of the first n admissible blocks to host memory on stream st: as they are
+// stored, or, where a stored matrix stands for two blocks, put out block by block in pieces of at most
+// 64 MiB of device memory.
+static int copy_coupling(const h2b_h2matrix *h, uint32_t n, double *out, cudaStream_t st) {
+  const uint64_t one = (uint64_t) h->k * h->k * (h->cx ? 2 : 1);
+  if (h->nstored == h->nadm) {
+    H2B_CUDA_TRY(cudaMemcpyAsync(out, h->d_S, sizeof(double) * one * n, cudaMemcpyDeviceToHost, st));
+    return H2B_OK;
+  }
+  const uint32_t per =
+      (uint32_t) std::max<uint64_t>(1, std::min<uint64_t>(n, (64u << 20) / (sizeof(double) * one)));
+  double *buf = nullptr;
+  H2B_CUDA_TRY(cudaMallocAsync((void **) &buf, sizeof(double) * one * per, st));
+  int rc = H2B_OK;
+  for (uint32_t b = 0; rc == H2B_OK && b < n; b += per) {
+    const uint32_t m = std::min(per, n - b);
+    rc = h2b_far_expand(h->d_S, h->d_spos, b, m, (int) h->k, h->cx, buf, st);
+    if (rc == H2B_OK && cudaMemcpyAsync(out + one * b, buf, sizeof(double) * one * m,
+                                        cudaMemcpyDeviceToHost, st) != cudaSuccess) {
+      h2b_set_error("h2b_h2matrix_export: %s", cudaGetErrorString(cudaGetLastError()));
+      rc = H2B_ERR_CUDA;
+    }
+  }
+  cudaFreeAsync(buf, st);
+  return rc;
+}
+
 extern "C" int h2b_h2matrix_export(const h2b_h2matrix *h, int part, uint32_t count, double *out,
                                    uint64_t *ndoubles) {
   if (!h || !ndoubles) return H2B_ERR_ARG;
@@ -1301,6 +1359,12 @@ extern "C" int h2b_h2matrix_export(const h2b_h2matrix *h, int part, uint32_t cou
       return H2B_ERR_ARG;
   }
   *ndoubles = n;
+  if (out && n && part == 4) {
+    const int rc = copy_coupling(h, (uint32_t) (n / (kk * W)), out, h->st);
+    if (rc != H2B_OK) return rc;
+    H2B_CUDA_TRY(cudaStreamSynchronize(h->st));
+    return H2B_OK;
+  }
   if (out && n) {
     H2B_CUDA_TRY(cudaMemcpyAsync(out, src, sizeof(double) * n, cudaMemcpyDeviceToHost, h->st));
     H2B_CUDA_TRY(cudaStreamSynchronize(h->st));
@@ -1339,6 +1403,7 @@ extern "C" int h2b_h2matrix_export_async(h2b_h2matrix *h, int part, uint32_t cou
   // after everything already queued on the matrix's stream, on the copy stream
   H2B_CUDA_TRY(cudaEventRecord(h->ev_copy, h->st));
   H2B_CUDA_TRY(cudaStreamWaitEvent(h->cst, h->ev_copy, 0));
+  if (part == 4) return copy_coupling(h, (uint32_t) (n / ((uint64_t) h->k * h->k * (h->cx ? 2 : 1))), out, h->cst);
   H2B_CUDA_TRY(cudaMemcpyAsync(out, src, sizeof(double) * n, cudaMemcpyDeviceToHost, h->cst));
   return H2B_OK;
 }
@@ -1370,11 +1435,60 @@ extern "C" int h2b_h2matrix_addeval_multi(double alpha_re, double alpha_im,
     return H2B_ERR_ARG;
   }
   const size_t W = h->cx ? 2 : 1;
-  for (uint32_t r = 0; r < nrhs; r++) {
-    int rc = h2b_h2matrix_addeval(alpha_re, alpha_im, h, X + W * ldx * r, Y + W * ldy * r);
-    if (rc != H2B_OK) return rc;
+  const size_t nc = h->ct.nidx, nr = h->rt.nidx;
+  // columns of Y that overlap other columns of X are taken one after the other, as always
+  const uintptr_t x0 = (uintptr_t) X, x1 = (uintptr_t) (X + W * (ldx * (nrhs - 1ull) + nc));
+  const uintptr_t y0 = (uintptr_t) Y, y1 = (uintptr_t) (Y + W * (ldy * (nrhs - 1ull) + nr));
+  const bool apart = nrhs > 1 && (x1 <= y0 || y1 <= x0 || (X == Y && ldx == ldy));
+  if (!apart) {
+    for (uint32_t r = 0; r < nrhs; r++) {
+      int rc = h2b_h2matrix_addeval(alpha_re, alpha_im, h, X + W * ldx * r, Y + W * ldy * r);
+      if (rc != H2B_OK) return rc;
+    }
+    return H2B_OK;
   }
-  return H2B_OK;
+  // The columns in one launch sequence that reads the matrix once (several when a stage's shared
+  // memory holds fewer slices).  The work vectors are the call's own: a stream-ordered
+  // allocation from the device's pool.
+  const uint32_t most = h2b_mvm_max_columns(&h->mvm, 0), seqs = (nrhs + most - 1) / most,
+                 per = (nrhs + seqs - 1) / seqs;
+  const bool dx = h2b_is_device_ptr(X), dy = h2b_is_device_ptr(Y);
+  const size_t nwork = h2b_mvm_work_doubles(&h->mvm, per);
+  double *buf = nullptr;
+  H2B_CUDA_TRY(cudaMallocAsync((void **) &buf, sizeof(double) * (nwork + W * per * (nc + nr)), h->st));
+  double *xd = buf + nwork, *yd = xd + W * per * nc;
+  int rc = H2B_OK;
+  cudaEventRecord(h->ev[9], h->st);
+  for (uint32_t r0 = 0; rc == H2B_OK && r0 < nrhs; r0 += per) {
+    const uint32_t n = std::min(per, nrhs - r0);
+    const double *x = X + W * ldx * r0;
+    double *y = Y + W * ldy * r0;
+    if (!dx && cudaMemcpy2DAsync(xd, sizeof(double) * W * nc, x, sizeof(double) * W * ldx,
+                                 sizeof(double) * W * nc, n, cudaMemcpyHostToDevice,
+                                 h->st) != cudaSuccess)
+      rc = H2B_ERR_CUDA;
+    if (rc == H2B_OK && !dy &&
+        cudaMemcpy2DAsync(yd, sizeof(double) * W * nr, y, sizeof(double) * W * ldy,
+                          sizeof(double) * W * nr, n, cudaMemcpyHostToDevice, h->st) != cudaSuccess)
+      rc = H2B_ERR_CUDA;
+    if (rc == H2B_OK)
+      rc = h2b_mvm_launch_batch(&h->mvm, 0, n, dx ? x : xd, W * (dx ? ldx : nc), dy ? y : yd,
+                                W * (dy ? ldy : nr), alpha_re, alpha_im, buf, nullptr, 1, h->st);
+    if (rc == H2B_OK && !dy &&
+        cudaMemcpy2DAsync(y, sizeof(double) * W * ldy, yd, sizeof(double) * W * nr,
+                          sizeof(double) * W * nr, n, cudaMemcpyDeviceToHost, h->st) != cudaSuccess)
+      rc = H2B_ERR_CUDA;
+    if (rc == H2B_ERR_CUDA)
+      h2b_set_error("h2b_h2matrix_addeval_multi: %s", cudaGetErrorString(cudaGetLastError()));
+  }
+  cudaEventRecord(h->ev[10], h->st);
+  cudaFreeAsync(buf, h->st);
+  const int ec = h2b_h2_check_mv_error(h);  // waits for the stream
+  if (rc == H2B_OK) rc = ec;
+  float t;
+  if (rc == H2B_OK && cudaEventElapsedTime(&t, h->ev[9], h->ev[10]) == cudaSuccess)
+    const_cast<h2b_h2matrix *>(h)->ms[5] = t;
+  return rc;
 }
 
 static int addeval_prec(double alpha_re, double alpha_im, const h2b_h2matrix *h, const double *x,

@@ -63,6 +63,14 @@ struct h2b_h2matrix {
   // 1: equal row and column trees and bases (the greenhybrid column basis of the single layer is then
   // the row basis)
   int same = 0;
+  // 1: the coupling matrices of an admissible block and of its transposed block are each other's
+  // transposes (the kernel at the interpolation points of equal trees): one of each two is formed,
+  // stored and read.  h_spos: per admissible block, its stored matrix's position times two, plus one
+  // when the block is the transpose of that matrix; nstored matrices, of blocks d_st_rc / d_st_cc
+  int sym_coupling = 0;
+  std::vector<uint32_t> h_spos;
+  uint32_t nstored = 0;
+  uint32_t *d_st_rc = nullptr, *d_st_cc = nullptr, *d_spos = nullptr;
   int g_row_ready = 0;   // the row basis of the current assembly is in place
   int g_col_copied = 0;  // the column basis was copied (its leaf bases are the row side's)
   double g_tg[9] = {}, g_wg[9] = {}, g_delta = 0.0, g_accur = 0.0;

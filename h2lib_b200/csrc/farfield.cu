@@ -284,7 +284,32 @@ __global__ void __launch_bounds__(128) coupling_kernel(FarCouplingArgs a) {
   }
 }
 
+// A block's coupling matrix from the stored ones, CTA per block (export only).
+template <typename E>
+__global__ void __launch_bounds__(256) expand_kernel(const E *S, const uint32_t *spos, uint32_t first,
+                                                     int k, E *out) {
+  const uint32_t p = spos[first + blockIdx.x];
+  const E *src = S + (size_t) (p >> 1) * k * k;
+  E *dst = out + (size_t) blockIdx.x * k * k;
+  for (int e = threadIdx.x; e < k * k; e += 256) {
+    const int j = e / k, i = e - j * k;
+    dst[e] = src[p & 1u ? j + i * k : e];
+  }
+}
+
 }  // namespace
+
+extern "C" int h2b_far_expand(const double *S, const uint32_t *spos, uint32_t first, uint32_t n, int k,
+                              int cx, double *out, cudaStream_t st) {
+  if (n == 0) return H2B_OK;
+  if (cx)
+    expand_kernel<double2><<<n, 256, 0, st>>>((const double2 *) S, spos, first, k, (double2 *) out);
+  else
+    expand_kernel<double><<<n, 256, 0, st>>>(S, spos, first, k, out);
+  h2b_note_launch();
+  H2B_CUDA_TRY(cudaGetLastError());
+  return H2B_OK;
+}
 
 template <bool L, bool D, int M>
 static int launch_leaf(const FarLeafArgs *a, size_t smem, cudaStream_t st) {

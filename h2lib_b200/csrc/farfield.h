@@ -77,4 +77,8 @@ extern "C" int h2b_flat_rows(const FlatArgs *a, cudaStream_t st);
 
 extern "C" int h2b_far_leaf_basis(const FarLeafArgs *a, int linear, int dn, cudaStream_t st);
 extern "C" int h2b_far_transfer(const FarTransferArgs *a, cudaStream_t st);
+// out = the k x k matrices of blocks first .. first + n - 1 (W doubles per entry) from the stored ones:
+// spos[b] = position times two, plus one when block b is the transpose of that matrix.
+extern "C" int h2b_far_expand(const double *S, const uint32_t *spos, uint32_t first, uint32_t n, int k,
+                              int cx, double *out, cudaStream_t st);
 extern "C" int h2b_far_coupling(const FarCouplingArgs *a, int cx, cudaStream_t st);

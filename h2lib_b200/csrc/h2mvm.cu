@@ -117,6 +117,9 @@ struct MvLaunch {
   uint32_t stage_bytes;    // bytes per stage (multiple of 128)
   uint32_t panel_bytes;    // panel region of a stage; the x slices of every column follow
   uint32_t xcol_bytes;     // bytes per x slice of one column (multiple of 16, with slack)
+  uint32_t group;          // columns multiplied together (several columns: balanced groups)
+  uint32_t run;            // coupling: consecutive panels per warp
+  uint32_t x2_doubles;     // coupling: doubles per column of a warp's row slices
   uint32_t stages;         // ring stages, a multiple of nw: stage s belongs to consumer warp s % nw
   uint32_t nw;             // consumer warps; warp nw produces
 };
@@ -180,35 +183,53 @@ __device__ __forceinline__ void entry(const T *P, size_t e, double &re, double &
   }
 }
 
-// y[0, R) += P x[0, C) by one warp: lanes take rows (SL slots of 32), the warp runs over the
-// columns; one atomic addition per row.
-template <bool CX, bool PCX, typename T, int SL>
+// The columns of a product that a warp multiplies a panel with at once: their x slices in the stage
+// and their y slices.
+template <int NQ>
+struct Cols {
+  const double *x[NQ];
+  double *y[NQ];
+  int n;
+};
+
+// y_q[0, R) += P x_q[0, C) by one warp for the n <= NQ columns q: lanes take rows (SL slots of 32), the
+// warp runs over the panel's columns, each entry read once for all q; one atomic addition per row
+// and column.
+template <bool CX, bool PCX, typename T, int SL, int NQ>
 __device__ __forceinline__ void warp_gemv_n(const T *__restrict__ P, uint32_t R, uint32_t C,
-                                            const double *__restrict__ xs, double *y,
-                                            uint32_t lane) {
+                                            const Cols<NQ> &v, uint32_t lane) {
   constexpr int W = CX ? 2 : 1;
-  double sr[SL], si[SL];
+  double sr[SL][NQ], si[SL][NQ];
   bool on[SL];
 #pragma unroll
   for (int j = 0; j < SL; j++) {
-    sr[j] = si[j] = 0.0;
     on[j] = lane + 32u * j < R;
+#pragma unroll
+    for (int q = 0; q < NQ; q++) sr[j][q] = si[j][q] = 0.0;
   }
 #pragma unroll 4
   for (uint32_t c = 0; c < C; c++) {
-    const double xr = xs[W * c], xi = CX ? xs[W * c + 1] : 0.0;
+    double xr[NQ], xi[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; q++) {
+      xr[q] = v.x[q][W * c];
+      xi[q] = CX ? v.x[q][W * c + 1] : 0.0;
+    }
     const T *col = P + (size_t) (PCX ? 2 : 1) * c * R;
 #pragma unroll
     for (int j = 0; j < SL; j++) {
       if (on[j]) {
         double pr, pi;
         entry<PCX>(col, lane + 32u * j, pr, pi);
-        if (PCX) {
-          sr[j] = fma(pr, xr, fma(-pi, xi, sr[j]));
-          si[j] = fma(pr, xi, fma(pi, xr, si[j]));
-        } else {
-          sr[j] = fma(pr, xr, sr[j]);
-          if (CX) si[j] = fma(pr, xi, si[j]);
+#pragma unroll
+        for (int q = 0; q < NQ; q++) {
+          if (PCX) {
+            sr[j][q] = fma(pr, xr[q], fma(-pi, xi[q], sr[j][q]));
+            si[j][q] = fma(pr, xi[q], fma(pi, xr[q], si[j][q]));
+          } else {
+            sr[j][q] = fma(pr, xr[q], sr[j][q]);
+            if (CX) si[j][q] = fma(pr, xi[q], si[j][q]);
+          }
         }
       }
     }
@@ -217,70 +238,82 @@ __device__ __forceinline__ void warp_gemv_n(const T *__restrict__ P, uint32_t R,
   for (int j = 0; j < SL; j++) {
     if (on[j]) {
       const uint32_t r = lane + 32u * j;
-      atomicAdd(y + W * r, sr[j]);
-      if (CX) atomicAdd(y + W * r + 1, si[j]);
-    }
-  }
-}
-
-// y[0, C) += P^T x[0, R) by one warp for a real panel: lanes take columns (SL slots of 32) and
-// run over the rows from a lane-dependent start, row (it + lane) mod R at step it, so that the
-// warp's reads of the column-major panel fall in distinct banks.
-template <bool CX, typename T, int SL>
-__device__ __forceinline__ void warp_gemv_t(const T *__restrict__ P, uint32_t R, uint32_t C,
-                                            const double *__restrict__ xs, double *y,
-                                            uint32_t lane) {
-  constexpr int W = CX ? 2 : 1;
-  double sr[SL], si[SL];
-  bool on[SL];
 #pragma unroll
-  for (int j = 0; j < SL; j++) {
-    sr[j] = si[j] = 0.0;
-    on[j] = lane + 32u * j < C;
-  }
-  uint32_t r = lane % R;
-#pragma unroll 4
-  for (uint32_t it = 0; it < R; it++) {
-    const double xr = xs[W * r], xi = CX ? xs[W * r + 1] : 0.0;
-#pragma unroll
-    for (int j = 0; j < SL; j++) {
-      if (on[j]) {
-        const double p = (double) P[r + (size_t) (lane + 32u * j) * R];
-        sr[j] = fma(p, xr, sr[j]);
-        if (CX) si[j] = fma(p, xi, si[j]);
+      for (int q = 0; q < NQ; q++) {
+        if (q >= v.n) break;
+        atomicAdd(v.y[q] + W * r, sr[j][q]);
+        if (CX) atomicAdd(v.y[q] + W * r + 1, si[j][q]);
       }
     }
-    r = r + 1 == R ? 0u : r + 1;
   }
+}
+
+// y_q[0, C) += P^T x_q[0, R) by one warp for the n <= NQ columns q, 32 panel columns at a time.  With cw
+// of them the lanes form G = 32 / cp groups (cp: cw rounded up to a power of two); a lane takes one
+// panel column and its group's part of the rows, and the groups' sums are added by shuffles, so that a
+// panel of few columns (8 for complex rank 125) keeps every lane busy.  Lanes of neighbouring
+// columns read P an odd number of entries apart, which falls in distinct banks: R apart for odd R,
+// R + 1 for even R (a lane starts its rows at its column's number and wraps around).
+template <bool CX, bool PCX, typename T, int NQ>
+__device__ __forceinline__ void warp_gemv_t(const T *__restrict__ P, uint32_t R, uint32_t C,
+                                            const Cols<NQ> &v, uint32_t lane) {
+  constexpr int W = CX ? 2 : 1;
+  for (uint32_t c0 = 0; c0 < C; c0 += 32) {
+    const uint32_t cw = min(32u, C - c0), cp = cw > 1 ? 1u << (32 - __clz(cw - 1)) : 1u;
+    const uint32_t col = lane & (cp - 1u), G = 32u / cp, grp = lane / cp;
+    const uint32_t r0 = grp * R / G, len = (grp + 1) * R / G - r0;
+    const bool on = col < cw;
+    double sr[NQ], si[NQ];
 #pragma unroll
-  for (int j = 0; j < SL; j++) {
-    if (on[j]) {
-      const uint32_t c = lane + 32u * j;
-      atomicAdd(y + W * c, sr[j]);
-      if (CX) atomicAdd(y + W * c + 1, si[j]);
+    for (int q = 0; q < NQ; q++) sr[q] = si[q] = 0.0;
+    if (on && len > 0) {
+      const T *p = P + (size_t) (PCX ? 2 : 1) * ((size_t) (c0 + col) * R + r0);
+      uint32_t r = (R & 1u) ? 0u : col % len;
+#pragma unroll 4
+      for (uint32_t it = 0; it < len; it++) {
+        double pr, pi;
+        entry<PCX>(p, r, pr, pi);
+#pragma unroll
+        for (int q = 0; q < NQ; q++) {
+          const double *x = v.x[q] + W * (r0 + r);
+          const double xr = x[0], xi = CX ? x[1] : 0.0;
+          if (PCX) {
+            sr[q] = fma(pr, xr, fma(-pi, xi, sr[q]));
+            si[q] = fma(pr, xi, fma(pi, xr, si[q]));
+          } else {
+            sr[q] = fma(pr, xr, sr[q]);
+            if (CX) si[q] = fma(pr, xi, si[q]);
+          }
+        }
+        r = r + 1 == len ? 0u : r + 1;
+      }
+    }
+    for (uint32_t o = cp; o < 32u; o <<= 1) {
+#pragma unroll
+      for (int q = 0; q < NQ; q++) {
+        sr[q] += __shfl_xor_sync(0xffffffffu, sr[q], o);
+        if (CX) si[q] += __shfl_xor_sync(0xffffffffu, si[q], o);
+      }
+    }
+    if (on && grp == 0) {
+#pragma unroll
+      for (int q = 0; q < NQ; q++) {
+        if (q >= v.n) break;
+        atomicAdd(v.y[q] + W * (c0 + col), sr[q]);
+        if (CX) atomicAdd(v.y[q] + W * (c0 + col) + 1, si[q]);
+      }
     }
   }
 }
 
-template <bool CX, bool PCX, typename T>
-__device__ __forceinline__ void gemv_n_any(const T *P, uint32_t R, uint32_t C, const double *xs,
-                                           double *y, uint32_t lane) {
+template <bool CX, bool PCX, typename T, int NQ>
+__device__ __forceinline__ void gemv_n_any(const T *P, uint32_t R, uint32_t C, const Cols<NQ> &v,
+                                           uint32_t lane) {
   switch ((R + 31) >> 5) {
-    case 1: warp_gemv_n<CX, PCX, T, 1>(P, R, C, xs, y, lane); break;
-    case 2: warp_gemv_n<CX, PCX, T, 2>(P, R, C, xs, y, lane); break;
-    case 3: warp_gemv_n<CX, PCX, T, 3>(P, R, C, xs, y, lane); break;
-    default: warp_gemv_n<CX, PCX, T, 4>(P, R, C, xs, y, lane); break;
-  }
-}
-
-template <bool CX, typename T>
-__device__ __forceinline__ void gemv_t_any(const T *P, uint32_t R, uint32_t C, const double *xs,
-                                           double *y, uint32_t lane) {
-  switch ((C + 31) >> 5) {
-    case 1: warp_gemv_t<CX, T, 1>(P, R, C, xs, y, lane); break;
-    case 2: warp_gemv_t<CX, T, 2>(P, R, C, xs, y, lane); break;
-    case 3: warp_gemv_t<CX, T, 3>(P, R, C, xs, y, lane); break;
-    default: warp_gemv_t<CX, T, 4>(P, R, C, xs, y, lane); break;
+    case 1: warp_gemv_n<CX, PCX, T, 1, NQ>(P, R, C, v, lane); break;
+    case 2: warp_gemv_n<CX, PCX, T, 2, NQ>(P, R, C, v, lane); break;
+    case 3: warp_gemv_n<CX, PCX, T, 3, NQ>(P, R, C, v, lane); break;
+    default: warp_gemv_n<CX, PCX, T, 4, NQ>(P, R, C, v, lane); break;
   }
 }
 
@@ -292,7 +325,8 @@ __device__ __forceinline__ void gemv_t_any(const T *P, uint32_t R, uint32_t C, c
 // i % S always belongs to the same warp, and no barrier joins the consumer warps.  Every wait is
 // bounded; a warp whose wait runs out sets the error flag and leaves, and the others' bounded
 // waits end the CTA.
-template <bool CX, typename T>
+// NQ: columns multiplied per read of a panel from the stage (1, or MULTI for several columns).
+template <bool CX, typename T, int NQ>
 __global__ void __launch_bounds__(MAXTHREADS) mv_items_kernel(MvLaunch L) {
   extern __shared__ __align__(128) unsigned char smem[];
   constexpr int W = CX ? 2 : 1;
@@ -396,18 +430,32 @@ __global__ void __launch_bounds__(MAXTHREADS) mv_items_kernel(MvLaunch L) {
     const T *P = reinterpret_cast<const T *>(stage + delta);
     const int t = m.flags & H2B_MV_KIND;
     const bool trans = (m.flags & H2B_MV_TRANS) != 0;
-    const size_t xn = (size_t) W * sizeof(double) * (trans ? m.rows : m.cols);
-    for (uint32_t q = 0; q < L.nrhs; q++) {
-      if (!col_on(L.mask, L.nseg, m.seg, q)) continue;  // the column's system is done
-      const char *xl;
-      uint32_t xd, xb;
-      span16(L.X[t] + q * L.sx[t] + (size_t) W * m.xo, xn, xl, xd, xb);
-      const double *xs =
-          reinterpret_cast<const double *>(stage + L.panel_bytes + q * L.xcol_bytes + xd);
-      double *y = L.Y[t] + q * L.sy[t] + (size_t) W * m.yo;
-      if (trans) gemv_t_any<CX, T>(P, m.rows, m.cols, xs, y, lane);
-      else if (CX && complex_panel(t)) gemv_n_any<CX, CX, T>(P, m.rows, m.cols, xs, y, lane);
-      else gemv_n_any<CX, false, T>(P, m.rows, m.cols, xs, y, lane);
+    // the running columns, up to NQ at a time (unused places repeat the last one and write nothing)
+    for (uint32_t q = 0; q < L.nrhs;) {
+      Cols<NQ> v;
+      uint32_t at[NQ];
+      v.n = 0;
+#pragma unroll
+      for (int j = 0; j < NQ; j++) {
+        while (q < L.nrhs && !col_on(L.mask, L.nseg, m.seg, q)) q++;
+        if (q < L.nrhs && (NQ == 1 || (uint32_t) j < L.group)) {
+          at[j] = q++;
+          v.n = j + 1;
+        } else {
+          at[j] = j > 0 ? at[j - 1] : 0u;
+        }
+      }
+      if (v.n == 0) break;
+#pragma unroll
+      for (int j = 0; j < NQ; j++) {
+        const double *x = L.X[t] + at[j] * L.sx[t] + (size_t) W * m.xo;
+        v.x[j] = reinterpret_cast<const double *>(stage + L.panel_bytes + at[j] * L.xcol_bytes +
+                                                  (reinterpret_cast<uintptr_t>(x) & 15u));
+        v.y[j] = L.Y[t] + at[j] * L.sy[t] + (size_t) W * m.yo;
+      }
+      if (trans) warp_gemv_t<CX, false, T, NQ>(P, m.rows, m.cols, v, lane);
+      else if (CX && complex_panel(t)) gemv_n_any<CX, CX, T, NQ>(P, m.rows, m.cols, v, lane);
+      else gemv_n_any<CX, false, T, NQ>(P, m.rows, m.cols, v, lane);
     }
     __syncwarp();
     if (lane == 0)
@@ -416,28 +464,246 @@ __global__ void __launch_bounds__(MAXTHREADS) mv_items_kernel(MvLaunch L) {
   }
 }
 
-// Stage layout: the panel (FP64 panel bytes scaled to the storage type, plus 32 bytes for the
-// alignment and rounding slack) and the x slices of nrhs columns.
+// Coupling panels.  A warp takes a run of consecutive panels of one block (several runs per warp, a
+// block's panels are neighbours in the list) through a stage of its own and keeps the block's row
+// sums in registers (SL slots of 32 rows, NQ columns), so that they reach yt once per run and not once
+// per panel: for complex rank 125 a 16 KiB panel has 8 columns, and adding its 125 rows per panel
+// took 485M FP64 additions to L2 for a product of 49152 triangles with five columns.  A panel
+// that stands for its block and the transposed one (H2B_MV_SYM) is multiplied a second time,
+// transposed, with the row cluster's x, which comes with the run's first panel.  A warp issues its own
+// copies (panel and x slices, completion on its mbarrier) as soon as it has read the panel
+// before: the other warps of the SM cover the wait, and no warp waits for another's copy to be issued
+// (one producer lane for four warps took twice as long on small matrices).  Waits are bounded; nrhs <=
+// NQ.
+// 49152 triangles, m = 5, complex: a product with five columns 9.6 ms as five products, 6.2 with the
+// columns together and panels added one by one, 3.2 with this kernel.  32768 triangles, m = 4, real:
+// 104 us reading every block, 88 reading one of two.
+constexpr uint32_t CP_WARPS = 4;  // warps of a CTA
+template <bool CX, typename T, int SL, int NQ>
+__global__ void __launch_bounds__(CP_WARPS * 32) mv_coupling_kernel(MvLaunch L) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  constexpr int W = CX ? 2 : 1;
+  constexpr int t = H2B_MV_COUPLING;
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+  // the warp's stage (panel, x slices), row slices and barrier
+  unsigned char *stage = smem + (size_t) warp * L.stage_bytes;
+  double *x2 = reinterpret_cast<double *>(smem + (size_t) L.nw * L.stage_bytes) +
+               (size_t) warp * L.nrhs * L.x2_doubles;
+  const uint32_t bar = smem_addr(
+      reinterpret_cast<uint64_t *>(smem + (size_t) L.nw * (L.stage_bytes + 8u * L.nrhs * L.x2_doubles)) + warp);
+  if (lane == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncwarp();
+  // the warp's runs: every wall-th
+  const uint32_t nruns = (L.n + L.run - 1) / L.run, wall = gridDim.x * L.nw;
+  // lane 0: copies panel m and its x slices; head: the row slices too
+  auto issue = [&](const MvItem &m, bool head) {
+    size_t n;
+    const char *pa = panel_addr<CX, T>(L, m, n), *lo, *xl;
+    uint32_t delta, bytes, total = 0, xd, xb;
+    span16(pa, n, lo, delta, bytes);
+    const bool rows2 = head && (m.flags & H2B_MV_SYM);
+    const size_t xn = (size_t) W * sizeof(double) * m.cols, x2n = (size_t) W * sizeof(double) * m.rows;
+    for (uint32_t q = 0; q < L.nrhs; q++) {
+      if (!col_on(L.mask, L.nseg, m.seg, q)) continue;
+      span16(L.X[t] + q * L.sx[t] + (size_t) W * m.xo, xn, xl, xd, xb);
+      total += xb;
+      if (rows2) {
+        span16(L.X[t] + q * L.sx[t] + (size_t) W * m.yo, x2n, xl, xd, xb);
+        total += xb;
+      }
+    }
+    if (total == 0) {  // every column's system is done: nothing to copy
+      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+      return;
+    }
+    total += bytes;
+    // the warp's reads of the stage are ordered before the copies into it
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(total)
+                 : "memory");
+    auto copy = [&](uint32_t dst, const char *src, uint32_t nb) {
+      asm volatile(
+          "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, "
+          "[%3];" ::"r"(dst), "l"(src), "r"(nb), "r"(bar)
+          : "memory");
+    };
+    copy(smem_addr(stage), lo, bytes);
+    for (uint32_t q = 0; q < L.nrhs; q++) {
+      if (!col_on(L.mask, L.nseg, m.seg, q)) continue;
+      span16(L.X[t] + q * L.sx[t] + (size_t) W * m.xo, xn, xl, xd, xb);
+      copy(smem_addr(stage + L.panel_bytes + q * L.xcol_bytes), xl, xb);
+      if (rows2) {
+        span16(L.X[t] + q * L.sx[t] + (size_t) W * m.yo, x2n, xl, xd, xb);
+        copy(smem_addr(x2 + (size_t) q * L.x2_doubles), xl, xb);
+      }
+    }
+  };
+
+  double sr[SL][NQ], si[SL][NQ];
+  uint32_t at[NQ], ncol = 0, yo = UINT32_MAX, rows = 0;
+#pragma unroll
+  for (int q = 0; q < NQ; q++) {
+    at[q] = 0;
+#pragma unroll
+    for (int j = 0; j < SL; j++) sr[j][q] = si[j][q] = 0.0;
+  }
+  auto flush = [&]() {
+#pragma unroll
+    for (int q = 0; q < NQ; q++) {
+      double *y = L.Y[t] + at[q] * L.sy[t] + (size_t) W * yo;
+#pragma unroll
+      for (int j = 0; j < SL; j++) {
+        const uint32_t r = lane + 32u * j;
+        if ((uint32_t) q < ncol && r < rows) {
+          atomicAdd(y + W * r, sr[j][q]);
+          if (CX) atomicAdd(y + W * r + 1, si[j][q]);
+        }
+        sr[j][q] = si[j][q] = 0.0;
+      }
+    }
+  };
+  uint32_t run = blockIdx.x * L.nw + warp, i = run * L.run, phase = 0;
+  if (run >= nruns) return;
+  MvItem m = L.items[L.first + i];
+  if (lane == 0) issue(m, true);
+  for (;;) {
+    // the next panel's descriptor, on its way while this panel is multiplied
+    uint32_t ni = i + 1;
+    if (ni == min(L.n, (run + 1) * L.run)) {
+      run += wall;
+      ni = run < nruns ? run * L.run : L.n;
+    }
+    MvItem nm = m;
+    if (ni < L.n) nm = L.items[L.first + ni];
+    if (!bar_wait(bar, phase)) {
+      // a wait ran out: flag it, wait once more (bounded) for the copies in flight, and leave
+      if (lane == 0) atomicExch(L.err, 1);
+      bar_wait(bar, phase);
+      return;
+    }
+    phase ^= 1u;
+    const bool sym = (m.flags & H2B_MV_SYM) != 0;
+    if (m.yo != yo) {
+      if (yo != UINT32_MAX) flush();
+      yo = m.yo;
+      rows = m.rows;
+      // the running columns (unused places repeat the last one)
+      ncol = 0;
+      uint32_t q = 0;
+#pragma unroll
+      for (int u = 0; u < NQ; u++) {
+        while (q < L.nrhs && !col_on(L.mask, L.nseg, m.seg, q)) q++;
+        if (q < L.nrhs) {
+          at[u] = q++;
+          ncol = u + 1;
+        } else {
+          at[u] = u > 0 ? at[u - 1] : 0u;
+        }
+      }
+    }
+    if (ncol > 0) {
+      size_t n;
+      const char *pa = panel_addr<CX, T>(L, m, n);
+      const T *P = reinterpret_cast<const T *>(stage + (reinterpret_cast<uintptr_t>(pa) & 15u));
+      Cols<NQ> v;
+      v.n = (int) ncol;
+#pragma unroll
+      for (int q = 0; q < NQ; q++) {
+        const double *x = L.X[t] + at[q] * L.sx[t] + (size_t) W * m.xo;
+        v.x[q] = reinterpret_cast<const double *>(stage + L.panel_bytes + at[q] * L.xcol_bytes +
+                                                  (reinterpret_cast<uintptr_t>(x) & 15u));
+      }
+      // enough columns in flight to cover the shared-memory latency
+      constexpr int U = SL * NQ <= 4 ? 8 : SL * NQ <= 8 ? 4 : 2;
+#pragma unroll U
+      for (uint32_t c = 0; c < m.cols; c++) {
+        double xr[NQ], xi[NQ];
+#pragma unroll
+        for (int q = 0; q < NQ; q++) {
+          xr[q] = v.x[q][W * c];
+          xi[q] = CX ? v.x[q][W * c + 1] : 0.0;
+        }
+        const T *col = P + (size_t) W * c * rows;
+#pragma unroll
+        for (int u = 0; u < SL; u++) {
+          if (lane + 32u * u < rows) {
+            double pr, pi;
+            entry<CX>(col, lane + 32u * u, pr, pi);
+#pragma unroll
+            for (int q = 0; q < NQ; q++) {
+              if (CX) {
+                sr[u][q] = fma(pr, xr[q], fma(-pi, xi[q], sr[u][q]));
+                si[u][q] = fma(pr, xi[q], fma(pi, xr[q], si[u][q]));
+              } else {
+                sr[u][q] = fma(pr, xr[q], sr[u][q]);
+              }
+            }
+          }
+        }
+      }
+      if (sym) {
+#pragma unroll
+        for (int q = 0; q < NQ; q++) {
+          const double *x = L.X[t] + at[q] * L.sx[t] + (size_t) W * yo;
+          v.x[q] = reinterpret_cast<const double *>(
+              reinterpret_cast<const unsigned char *>(x2 + at[q] * L.x2_doubles) +
+              (reinterpret_cast<uintptr_t>(x) & 15u));
+          v.y[q] = L.Y[t] + at[q] * L.sy[t] + (size_t) W * m.xo;
+        }
+        warp_gemv_t<CX, CX, T, NQ>(P, rows, m.cols, v, lane);
+      }
+    }
+    __syncwarp();
+    if (ni >= L.n) break;
+    if (lane == 0) issue(nm, nm.yo != m.yo || ni != i + 1);
+    m = nm;
+    i = ni;
+  }
+  flush();
+}
+
+// Columns multiplied per read of a panel when a product has several: four complex columns of a
+// 125-row panel are 32 sums per lane.
+constexpr int MULTI = 4;
+
+// Stage layout of launch g (0 forward + nearfield, 1 coupling, 2 backward): the panel (FP64 panel
+// bytes scaled to the storage type, plus 32 bytes for the alignment and rounding slack) and the x
+// slices of nrhs columns.
 template <typename T>
-uint32_t panel_region(const MvItems &ph) {
-  const size_t b = (size_t) ph.max_bytes * sizeof(T) / sizeof(double) + 32;
+uint32_t panel_region(const MvItems &ph, int g) {
+  const size_t b = (size_t) ph.max_bytes[g] * sizeof(T) / sizeof(double) + 32;
   return (uint32_t) ((b + 127) & ~(size_t) 127);
 }
 
 template <bool CX>
-uint32_t xcol_region(const MvItems &ph) {
-  return (uint32_t) ((sizeof(double) * (CX ? 2 : 1) * ph.max_x + 32 + 15) & ~(size_t) 15);
+uint32_t slice_region(uint32_t n) {
+  return n ? (uint32_t) ((sizeof(double) * (CX ? 2 : 1) * n + 32 + 15) & ~(size_t) 15) : 0u;
+}
+template <bool CX>
+uint32_t xcol_region(const MvItems &ph, int g) {
+  return slice_region<CX>(ph.max_x[g]);
 }
 
 template <bool CX, typename T>
-uint32_t stage_of(const MvItems &ph, uint32_t nrhs) {
-  const size_t b = panel_region<T>(ph) + (size_t) nrhs * xcol_region<CX>(ph);
+uint32_t stage_of(const MvItems &ph, int g, uint32_t nrhs) {
+  const size_t b = panel_region<T>(ph, g) + (size_t) nrhs * xcol_region<CX>(ph, g);
   return (uint32_t) ((b + 127) & ~(size_t) 127);
 }
 
 template <bool CX, typename T>
-size_t smem_of(const MvItems &ph, uint32_t stages, uint32_t nrhs) {
-  return (size_t) stages * (stage_of<CX, T>(ph, nrhs) + sizeof(MvItem) + 16);
+size_t smem_of(const MvItems &ph, int g, uint32_t stages, uint32_t nrhs) {
+  return (size_t) stages * (stage_of<CX, T>(ph, g, nrhs) + sizeof(MvItem) + 16);
+}
+
+// the largest of a product's launches
+template <bool CX, typename T>
+size_t smem_most(const MvItems &ph, uint32_t stages, uint32_t nrhs) {
+  size_t b = 0;
+  for (int g = 0; g < 3; g += 2) b = std::max(b, smem_of<CX, T>(ph, g, stages, nrhs));
+  return b;
 }
 
 // consumer warps and ring stages of a launch shape (stages per consumer warp 1..4)
@@ -446,30 +712,12 @@ void ring_shape(const MvmPlan *p, uint32_t &nw, uint32_t &stages) {
   stages = nw * (uint32_t) std::max(1, std::min(4, p->stages));
 }
 
-template <bool CX, typename T>
-int launch_range(const MvmPlan *p, const MvItems &ph, const MvLaunch &base, uint32_t first,
-                 uint32_t last, cudaStream_t st) {
-  if (last <= first) return H2B_OK;
-  MvLaunch L = base;
-  L.items = ph.items;
-  L.first = first;
-  L.n = last - first;
-  ring_shape(p, L.nw, L.stages);
-  L.panel_bytes = panel_region<T>(ph);
-  L.xcol_bytes = xcol_region<CX>(ph);
-  L.stage_bytes = stage_of<CX, T>(ph, L.nrhs);
-  const size_t smem = smem_of<CX, T>(ph, L.stages, L.nrhs);
-  if (smem > H2B_MAX_DYN_SMEM || ph.max_rows > MAXROWS || ph.max_cols_t > MAXROWS ||
-      ph.max_x > 65536) {
-    h2b_set_error("matvec: item panel of %u bytes / %u rows / %u transposed columns / %u "
-                  "right-hand sides exceeds the kernel's limits (%zu bytes of shared memory)",
-                  ph.max_bytes, ph.max_rows, ph.max_cols_t, L.nrhs, smem);
-    return H2B_ERR_ARG;
-  }
+template <bool CX, typename T, int NQ>
+int launch_items(const MvmPlan *p, const MvLaunch &L, size_t smem, cudaStream_t st) {
   const int threads = (int) (L.nw + 1) * 32;
-  H2B_CUDA_TRY((h2b_allow_smem<mv_items_kernel<CX, T>>()));
+  H2B_CUDA_TRY((h2b_allow_smem<mv_items_kernel<CX, T, NQ>>()));
   int occ = 0;
-  H2B_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, mv_items_kernel<CX, T>,
+  H2B_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, mv_items_kernel<CX, T, NQ>,
                                                              threads, smem));
   if (occ < 1) {
     h2b_set_error("matvec: the item kernel does not fit an SM (%zu bytes of shared memory)", smem);
@@ -478,8 +726,109 @@ int launch_range(const MvmPlan *p, const MvItems &ph, const MvLaunch &base, uint
   const int sms = p->num_sms > 0 ? p->num_sms : 148;
   const int per_sm = std::min(occ, std::max(1, p->ctas_per_sm));
   const uint32_t grid = std::min<uint32_t>(L.n, (uint32_t) (per_sm * sms));
-  mv_items_kernel<CX, T><<<grid, threads, smem, st>>>(L);
+  mv_items_kernel<CX, T, NQ><<<grid, threads, smem, st>>>(L);
   h2b_note_launch();
+  return H2B_OK;
+}
+
+// The items [first, last) of one launch's kinds (g: 0 forward + nearfield, 2 backward).
+template <bool CX, typename T>
+int launch_range(const MvmPlan *p, const MvItems &ph, const MvLaunch &base, uint32_t first,
+                 uint32_t last, cudaStream_t st) {
+  if (last <= first) return H2B_OK;
+  const int g = first >= ph.start[H2B_MV_BACKWARD] ? 2 : 0;
+  MvLaunch L = base;
+  L.items = ph.items;
+  L.first = first;
+  L.n = last - first;
+  ring_shape(p, L.nw, L.stages);
+  L.panel_bytes = panel_region<T>(ph, g);
+  L.xcol_bytes = xcol_region<CX>(ph, g);
+  L.stage_bytes = stage_of<CX, T>(ph, g, L.nrhs);
+  const uint32_t groups = (L.nrhs + MULTI - 1) / MULTI;
+  L.group = (L.nrhs + groups - 1) / groups;
+  const size_t smem = smem_of<CX, T>(ph, g, L.stages, L.nrhs);
+  if (smem > H2B_MAX_DYN_SMEM || ph.max_rows > MAXROWS || ph.max_x[g] > 65536) {
+    h2b_set_error("matvec: item panel of %u bytes / %u rows / %u right-hand sides exceeds the "
+                  "kernel's limits (%zu bytes of shared memory)",
+                  ph.max_bytes[g], ph.max_rows, L.nrhs, smem);
+    return H2B_ERR_ARG;
+  }
+  return L.nrhs > 1 ? launch_items<CX, T, MULTI>(p, L, smem, st)
+                    : launch_items<CX, T, 1>(p, L, smem, st);
+}
+
+// Shared memory of the coupling kernel for n columns.
+template <bool CX, typename T>
+size_t coupling_smem(const MvItems &ph, uint32_t nw, uint32_t n) {
+  const size_t x2 = slice_region<CX>(ph.max_x2[1]);
+  return (size_t) nw * (stage_of<CX, T>(ph, 1, n) + n * x2 + 8);
+}
+
+template <bool CX, typename T, int SL, int NQ>
+int launch_coupling_of(const MvmPlan *p, const MvItems &ph, MvLaunch &L, cudaStream_t st) {
+  const size_t smem = coupling_smem<CX, T>(ph, L.nw, L.nrhs);
+  const int threads = (int) L.nw * 32;
+  H2B_CUDA_TRY((h2b_allow_smem<mv_coupling_kernel<CX, T, SL, NQ>>()));
+  int occ = 0;
+  H2B_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+      &occ, mv_coupling_kernel<CX, T, SL, NQ>, threads, smem));
+  if (smem > H2B_MAX_DYN_SMEM || occ < 1) {
+    h2b_set_error("matvec: the coupling kernel does not fit an SM (%zu bytes of shared memory)", smem);
+    return H2B_ERR_ARG;
+  }
+  const int sms = p->num_sms > 0 ? p->num_sms : 148;
+  // runs: at least six per warp, so that the last round is short, at most a block each
+  const uint32_t all = (uint32_t) (occ * sms) * L.nw;
+  L.run = std::max(1u, std::min(ph.per_block, L.n / (6u * all)));
+  const uint32_t runs = (L.n + L.run - 1) / L.run;
+  const uint32_t grid = std::min<uint32_t>((runs + L.nw - 1) / L.nw, (uint32_t) (occ * sms));
+  mv_coupling_kernel<CX, T, SL, NQ><<<grid, threads, smem, st>>>(L);
+  h2b_note_launch();
+  return H2B_OK;
+}
+
+// Columns of one coupling launch.
+constexpr uint32_t CP_MAX = 5;
+
+template <bool CX, typename T, int SL>
+int launch_coupling_n(const MvmPlan *p, const MvItems &ph, MvLaunch &L, cudaStream_t st) {
+  if (L.nrhs == 1) return launch_coupling_of<CX, T, SL, 1>(p, ph, L, st);
+  if (L.nrhs <= 4) return launch_coupling_of<CX, T, SL, 4>(p, ph, L, st);
+  return launch_coupling_of<CX, T, SL, (int) CP_MAX>(p, ph, L, st);
+}
+
+// The coupling items, up to CP_MAX columns per launch (balanced).  Consumer warps: the shape that
+// keeps the most warps on an SM with at least one stage each.
+template <bool CX, typename T>
+int launch_coupling(const MvmPlan *p, const MvItems &ph, const MvLaunch &base, cudaStream_t st) {
+  const uint32_t first = ph.start[H2B_MV_COUPLING], last = ph.start[H2B_MV_BACKWARD];
+  if (last <= first) return H2B_OK;
+  const uint32_t groups = (base.nrhs + CP_MAX - 1) / CP_MAX, per = (base.nrhs + groups - 1) / groups;
+  for (uint32_t q0 = 0; q0 < base.nrhs; q0 += per) {
+    MvLaunch L = base;
+    L.items = ph.items;
+    L.first = first;
+    L.n = last - first;
+    L.nrhs = std::min(per, base.nrhs - q0);
+    L.X[H2B_MV_COUPLING] += q0 * L.sx[H2B_MV_COUPLING];
+    L.Y[H2B_MV_COUPLING] += q0 * L.sy[H2B_MV_COUPLING];
+    if (L.mask) L.mask += (size_t) q0 * L.nseg;
+    L.nw = CP_WARPS;
+    while (L.nw > 1 && coupling_smem<CX, T>(ph, L.nw, L.nrhs) > 110u * 1024u) L.nw--;
+    L.panel_bytes = panel_region<T>(ph, 1);
+    L.xcol_bytes = xcol_region<CX>(ph, 1);
+    L.stage_bytes = stage_of<CX, T>(ph, 1, L.nrhs);
+    L.x2_doubles = slice_region<CX>(ph.max_x2[1]) / 8u;
+    if (p->k > MAXROWS) {
+      h2b_set_error("matvec: rank %d exceeds %d", p->k, MAXROWS);
+      return H2B_ERR_ARG;
+    }
+    const int rc = p->k <= 32   ? launch_coupling_n<CX, T, 1>(p, ph, L, st)
+                   : p->k <= 64 ? launch_coupling_n<CX, T, 2>(p, ph, L, st)
+                                : launch_coupling_n<CX, T, 4>(p, ph, L, st);
+    if (rc != H2B_OK) return rc;
+  }
   return H2B_OK;
 }
 
@@ -515,8 +864,7 @@ int launch_all(const MvmPlan *p, const double *x, size_t ldx, double *y, size_t 
   const MvItems &it = SINGLE ? p->items_single : p->items;
   // forward + nearfield, coupling (reads xt), backward (reads yt)
   int rc = launch_range<CX, T>(p, it, L, 0, it.start[H2B_MV_COUPLING], st);
-  if (rc == H2B_OK)
-    rc = launch_range<CX, T>(p, it, L, it.start[H2B_MV_COUPLING], it.start[H2B_MV_BACKWARD], st);
+  if (rc == H2B_OK) rc = launch_coupling<CX, T>(p, it, L, st);
   if (rc == H2B_OK) rc = launch_range<CX, T>(p, it, L, it.start[H2B_MV_BACKWARD], it.n, st);
   if (rc != H2B_OK) return rc;
   scatter_multi_kernel<CX><<<gz, 256, 0, st>>>(v, p->ridx, y, ldy, p->nrow, ar, ai);
@@ -600,8 +948,7 @@ int launch_pair(const MvmPlan *p, const MvmPlan *q, const double *x, double *y, 
   const MvItems &iq = SINGLE ? q->items_single : q->items;
   int rc = launch_range<CX, T>(p, it, L, 0, it.start[H2B_MV_COUPLING], st);
   if (rc == H2B_OK) rc = launch_range<CX, T>(p, iq, Lq, 0, iq.start[H2B_MV_COUPLING], st);
-  if (rc == H2B_OK)
-    rc = launch_range<CX, T>(p, it, L, it.start[H2B_MV_COUPLING], it.start[H2B_MV_BACKWARD], st);
+  if (rc == H2B_OK) rc = launch_coupling<CX, T>(p, it, L, st);
   if (rc == H2B_OK) rc = launch_range<CX, T>(p, it, L, it.start[H2B_MV_BACKWARD], it.n, st);
   if (rc != H2B_OK) return rc;
   scatter_multi_kernel<CX><<<gz, 256, 0, st>>>(v, p->ridx, y, 0, p->nrow, 1.0, 0.0);
@@ -613,21 +960,54 @@ int launch_pair(const MvmPlan *p, const MvmPlan *q, const double *x, double *y, 
 
 }  // namespace
 
+template <bool CX, typename T, int SL>
+static int prepare_coupling(void) {
+  H2B_CUDA_TRY((h2b_allow_smem<mv_coupling_kernel<CX, T, SL, 1>>()));
+  H2B_CUDA_TRY((h2b_allow_smem<mv_coupling_kernel<CX, T, SL, 4>>()));
+  H2B_CUDA_TRY((h2b_allow_smem<mv_coupling_kernel<CX, T, SL, (int) CP_MAX>>()));
+  return H2B_OK;
+}
+template <bool CX, typename T>
+static int prepare_ranks(void) {
+  int rc = prepare_coupling<CX, T, 1>();
+  if (rc == H2B_OK) rc = prepare_coupling<CX, T, 2>();
+  return rc == H2B_OK ? prepare_coupling<CX, T, 4>() : rc;
+}
+
 extern "C" int h2b_mvm_prepare(void) {
-  H2B_CUDA_TRY((h2b_allow_smem<mv_items_kernel<false, double>>()));
-  H2B_CUDA_TRY((h2b_allow_smem<mv_items_kernel<true, double>>()));
-  H2B_CUDA_TRY((h2b_allow_smem<mv_items_kernel<false, float>>()));
-  H2B_CUDA_TRY((h2b_allow_smem<mv_items_kernel<true, float>>()));
+  int rc = prepare_ranks<false, double>();
+  if (rc == H2B_OK) rc = prepare_ranks<true, double>();
+  if (rc == H2B_OK) rc = prepare_ranks<false, float>();
+  if (rc == H2B_OK) rc = prepare_ranks<true, float>();
+  if (rc != H2B_OK) return rc;
+  H2B_CUDA_TRY((h2b_allow_smem<mv_items_kernel<false, double, 1>>()));
+  H2B_CUDA_TRY((h2b_allow_smem<mv_items_kernel<false, double, MULTI>>()));
+  H2B_CUDA_TRY((h2b_allow_smem<mv_items_kernel<true, double, 1>>()));
+  H2B_CUDA_TRY((h2b_allow_smem<mv_items_kernel<true, double, MULTI>>()));
+  H2B_CUDA_TRY((h2b_allow_smem<mv_items_kernel<false, float, 1>>()));
+  H2B_CUDA_TRY((h2b_allow_smem<mv_items_kernel<false, float, MULTI>>()));
+  H2B_CUDA_TRY((h2b_allow_smem<mv_items_kernel<true, float, 1>>()));
+  H2B_CUDA_TRY((h2b_allow_smem<mv_items_kernel<true, float, MULTI>>()));
   return H2B_OK;
 }
 
-extern "C" size_t h2b_mvm_smem_bytes(const MvmPlan *p, int single) {
+static size_t smem_any(const MvmPlan *p, int single, uint32_t nrhs) {
   const MvItems &ph = single ? p->items_single : p->items;
   uint32_t nw, stages;
   ring_shape(p, nw, stages);
   if (p->cx)
-    return single ? smem_of<true, float>(ph, stages, 1) : smem_of<true, double>(ph, stages, 1);
-  return single ? smem_of<false, float>(ph, stages, 1) : smem_of<false, double>(ph, stages, 1);
+    return single ? smem_most<true, float>(ph, stages, nrhs) : smem_most<true, double>(ph, stages, nrhs);
+  return single ? smem_most<false, float>(ph, stages, nrhs)
+                : smem_most<false, double>(ph, stages, nrhs);
+}
+
+extern "C" size_t h2b_mvm_smem_bytes(const MvmPlan *p, int single) { return smem_any(p, single, 1); }
+
+extern "C" uint32_t h2b_mvm_max_columns(const MvmPlan *p, int single) {
+  // two groups of MULTI columns; fewer when their slices would leave an SM one CTA only
+  uint32_t n = 2 * MULTI;
+  while (n > 1 && smem_any(p, single, n) > H2B_MAX_DYN_SMEM / 2) n--;
+  return n;
 }
 
 extern "C" int h2b_mvm_launch_single(const MvmPlan *p, const double *x, double *y, double ar,

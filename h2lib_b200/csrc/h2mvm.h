@@ -17,6 +17,8 @@
 #define H2B_MV_BACKWARD 3u
 #define H2B_MV_KIND 3u       // flags & H2B_MV_KIND: the kind
 #define H2B_MV_TRANS 4u      // y += P^T x
+#define H2B_MV_SYM 8u        // y += P x and also x's place of y += P^T times y's place of x: a coupling
+                             // panel that stands for its block and the transposed block
 struct MvItem {
   uint64_t p;                // element offset of the panel in its array
   uint32_t rows, cols;
@@ -31,10 +33,13 @@ struct MvItems {
   const MvItem *items;       // device
   uint32_t n;
   uint32_t start[4];
-  uint32_t max_bytes;        // largest panel in bytes at FP64 storage
+  // per launch (forward + nearfield, coupling, backward):
+  uint32_t max_bytes[3];     // largest panel in bytes at FP64 storage
+  uint32_t max_x[3];         // longest x slice (elements: cols, or rows when transposed)
+  uint32_t max_x2[3];        // longest second x slice (rows of an H2B_MV_SYM item), 0: none
   uint32_t max_rows;         // largest rows of an untransposed item
   uint32_t max_cols_t;       // largest columns of a transposed item
-  uint32_t max_x;            // longest x slice (elements: cols, or rows when transposed)
+  uint32_t per_block;        // panels of a coupling block
 };
 
 // Default largest panel of a work item (bytes at FP64 storage); blocks and slices are split to fit.
@@ -75,6 +80,8 @@ extern "C" size_t h2b_mvm_pair_work_doubles(const MvmPlan *p);
 extern "C" int h2b_mvm_launch_pair(const MvmPlan *p, const MvmPlan *q, int single,
                                    const double *x, double *y, double ar, double ai, double br,
                                    double bi, double *work, cudaStream_t st);
+// The most columns a batched product takes in one launch sequence (shared memory of a stage).
+extern "C" uint32_t h2b_mvm_max_columns(const MvmPlan *p, int single);
 extern "C" size_t h2b_mvm_work_doubles(const MvmPlan *p, uint32_t nrhs);
 extern "C" int h2b_mvm_launch_batch(const MvmPlan *p, int single, uint32_t nrhs, const double *x,
                                     size_t ldx, double *y, size_t ldy, double ar, double ai,
