@@ -1,5 +1,6 @@
 // C-ABI implementation: GMRES on combinations of H2 matrices, residuals, Laplace test data
 // (L2 projection of the harmonic Dirichlet datum, L2 error of the Neumann trace).
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdlib.h>
@@ -367,18 +368,6 @@ __global__ void project_rhs_kernel(HarmArgs a, double *v) {
   for (int l = 0; l < 3; l++) atomicAdd(&v[T.v[l]], s[l] * T.g);
 }
 
-// y = M x for the linear-basis mass matrix (addeval_mass_linear_bem3d, Library/bem3d.c:8878)
-__global__ void mass_kernel(const TriRec *tri, uint32_t nt, const double *x, double *y) {
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nt) return;
-  const TriRec &T = tri[t];
-  const double x0 = x[T.v[0]], x1 = x[T.v[1]], x2 = x[T.v[2]];
-  const double c1 = T.g / 24.0, c2 = T.g / 12.0;
-  atomicAdd(&y[T.v[0]], c2 * x0 + c1 * (x1 + x2));
-  atomicAdd(&y[T.v[1]], c2 * x1 + c1 * (x0 + x2));
-  atomicAdd(&y[T.v[2]], c2 * x2 + c1 * (x0 + x1));
-}
-
 // diagonal of the linear-basis mass matrix: sum over a vertex's triangles of g / 12
 __global__ void mass_diag_kernel(const TriRec *tri, uint32_t nt, double *d) {
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -420,6 +409,114 @@ __global__ void cg_dir_kernel(double *p, const double *r, uint32_t n, const doub
   const double be = sc[2] / sc[0];
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     p[i] = r[i] + be * p[i];
+}
+
+// CG on M x = v from x = 0 with the linear-basis mass matrix, to 1e-15 relative and at most 500
+// steps (solve_cg_avector, Library/krylovsolvers.c:18 as called by projectL2_bem3d_l_avector), in one
+// launch of one thread block cluster: a step is two passes over the vertices with a cluster barrier
+// after each, where separate kernels need six launches and a host read-back of the residual.  The
+// first pass forms the new direction of a vertex and of its neighbours from r and the old direction
+// (two buffers in turn) and gathers M p over the triangles around the vertex; sums of a CTA go to
+// the other CTAs through shared memory.  A thread keeps the first CG_KEEP triangles around its first
+// vertex in registers, so that up to 4096 vertices a step waits for one load and not for a chain of
+// four.  1026 vertices, 54 steps: separate kernels and their read-backs about 1900 us, this one 226
+// (695 without the kept triangles).
+constexpr int CG_CTAS = 8, CG_THREADS = 512, CG_KEEP = 7;
+
+// Sum over the cluster of one value per thread; slot: the parity of the call (a CTA may still read the
+// previous sum).  Contains the cluster barrier that ends the pass.
+__device__ double cluster_total(double v, double (&tot)[2][CG_CTAS], double *red, int slot) {
+  namespace cgr = cooperative_groups;
+  cgr::cluster_group cl = cgr::this_cluster();
+  v = warp_sum(v);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    double t = threadIdx.x < CG_THREADS / 32 ? red[threadIdx.x] : 0.0;
+    t = warp_sum(t);
+    if (threadIdx.x < CG_CTAS)
+      *cl.map_shared_rank(&tot[slot][cl.block_rank()], threadIdx.x) = t;
+  }
+  cl.sync();
+  double s = 0.0;
+#pragma unroll
+  for (int c = 0; c < CG_CTAS; c++) s += tot[slot][c];
+  return s;
+}
+
+__global__ void __cluster_dims__(CG_CTAS, 1, 1) __launch_bounds__(CG_THREADS)
+    mass_cg_kernel(const TriRec *tri, const uint32_t *vt_off, const uint32_t *vt_tri, uint32_t nv,
+                   const double *v, double *x, double *r, double *p0, double *p1, double *ap) {
+  __shared__ double tot[2][CG_CTAS], red[CG_THREADS / 32];
+  const uint32_t t0 = blockIdx.x * CG_THREADS + threadIdx.x, stride = CG_CTAS * CG_THREADS;
+  int slot = 0;
+  double rr = 0.0;
+  for (uint32_t i = t0; i < nv; i += stride) {
+    const double b = v[i];
+    x[i] = 0.0;
+    r[i] = b;
+    p0[i] = 0.0;
+    rr += b * b;
+  }
+  rr = cluster_total(rr, tot, red, slot);
+  const double tol = 1e-15 * sqrt(rr);
+  // the kept triangles: vertex ids (the thread's own vertex where there is none) and Gram determinants
+  uint32_t j[CG_KEEP][3], kept = 0;
+  double gk[CG_KEEP];
+#pragma unroll
+  for (int a = 0; a < CG_KEEP; a++) {
+    const bool on = t0 < nv && vt_off[t0] + a < vt_off[t0 + 1];
+    gk[a] = 0.0;
+    j[a][0] = j[a][1] = j[a][2] = min(t0, nv - 1u);
+    if (on) {
+      const TriRec &T = tri[vt_tri[vt_off[t0] + a]];
+      gk[a] = T.g;
+      for (int d = 0; d < 3; d++) j[a][d] = T.v[d];
+      kept = a + 1;
+    }
+  }
+  double beta = 0.0;
+  for (uint32_t it = 0; sqrt(rr) > tol && it + 1 < 500; it++) {
+    // p = r + beta p_old, M p
+    double *po = it & 1 ? p1 : p0, *pn = it & 1 ? p0 : p1;
+    double pap = 0.0;
+    for (uint32_t i = t0; i < nv; i += stride) {
+      const double pi = r[i] + beta * po[i];
+      double s = 0.0;
+      if (i == t0) {
+        double q[CG_KEEP];
+#pragma unroll
+        for (int a = 0; a < CG_KEEP; a++)
+          q[a] = (r[j[a][0]] + r[j[a][1]] + r[j[a][2]]) +
+                 beta * (po[j[a][0]] + po[j[a][1]] + po[j[a][2]]);
+#pragma unroll
+        for (int a = 0; a < CG_KEEP; a++) s += gk[a] * (pi + q[a]);
+      }
+      for (uint32_t a = vt_off[i] + (i == t0 ? kept : 0u); a < vt_off[i + 1]; a++) {
+        const TriRec &T = tri[vt_tri[a]];
+        const uint32_t j0 = T.v[0], j1 = T.v[1], j2 = T.v[2];
+        const double q0 = r[j0] + beta * po[j0], q1 = r[j1] + beta * po[j1], q2 = r[j2] + beta * po[j2];
+        s += T.g * (pi + (q0 + q1 + q2));
+      }
+      s *= 1.0 / 24.0;
+      pn[i] = pi;
+      ap[i] = s;
+      pap += pi * s;
+    }
+    pap = cluster_total(pap, tot, red, slot ^= 1);
+    const double al = rr / pap;
+    double rn = 0.0;
+    for (uint32_t i = t0; i < nv; i += stride) {
+      x[i] += al * pn[i];
+      const double q = r[i] - al * ap[i];
+      r[i] = q;
+      rn += q * q;
+    }
+    rn = cluster_total(rn, tot, red, slot ^= 1);
+    beta = rn / rr;
+    rr = rn;
+  }
 }
 
 // per-triangle (error^2, norm^2) of the Neumann trace -(x - z).n / |x - z|^3
@@ -662,7 +759,8 @@ __global__ void project_rhs_multi_kernel(HarmArgs a, MultiZ m, double *v) {
   for (int l = 0; l < 3; l++) atomicAdd(&v[(size_t) r * m.nv + T.v[l]], s[l] * T.g);
 }
 
-// mass_kernel on every column (blockIdx.y)
+// y = M x for the linear-basis mass matrix (addeval_mass_linear_bem3d, Library/bem3d.c:8878) on every
+// column (blockIdx.y)
 __global__ void mass_multi_kernel(const TriRec *tri, uint32_t nt, uint32_t nv, const double *x,
                                   double *y) {
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -738,38 +836,18 @@ extern "C" int h2b_project_l2_harmonic(const h2b_bem *bem, const double z[3], do
   const uint32_t nv = s->nv, nt = s->nt;
   DevBuf buf;
   buf.st = st;
-  H2B_CUDA_TRY(cudaMallocAsync(&buf.p, sizeof(double) * (5 * (size_t) nv + 6 * 64 + 4), st));
-  double *v = (double *) buf.p, *x = v + nv, *r = x + nv, *p = r + nv, *ap = p + nv,
-         *rule = ap + nv, *sc = rule + 6 * 64;
+  H2B_CUDA_TRY(cudaMallocAsync(&buf.p, sizeof(double) * (6 * (size_t) nv + 6 * 64), st));
+  double *v = (double *) buf.p, *x = v + nv, *r = x + nv, *p = r + nv, *p1 = p + nv, *ap = p1 + nv,
+         *rule = ap + nv;
   HarmArgs a;
   int rc = harm_args(bem, z, rule, &a, st);
   if (rc != H2B_OK) return rc;
-  H2B_CUDA_TRY(cudaMemsetAsync(v, 0, sizeof(double) * 2 * nv, st));
+  H2B_CUDA_TRY(cudaMemsetAsync(v, 0, sizeof(double) * nv, st));
   project_rhs_kernel<<<(nt + 127) / 128, 128, 0, st>>>(a, v);
-  // CG on M x = v from x = 0 to 1e-15 relative, at most 500 steps (solve_cg_avector,
-  // Library/krylovsolvers.c:18 as called by projectL2_bem3d_l_avector)
-  H2B_CUDA_TRY(cudaMemcpyAsync(r, v, sizeof(double) * nv, cudaMemcpyDeviceToDevice, st));
-  H2B_CUDA_TRY(cudaMemcpyAsync(p, v, sizeof(double) * nv, cudaMemcpyDeviceToDevice, st));
-  double hsc[4];
-  H2B_CUDA_TRY(cudaMemsetAsync(sc, 0, sizeof(double) * 4, st));
-  dot_kernel<<<64, 256, 0, st>>>(r, r, nv, sc);
-  H2B_CUDA_TRY(cudaMemcpyAsync(hsc, sc, sizeof(double), cudaMemcpyDeviceToHost, st));
-  H2B_CUDA_TRY(cudaStreamSynchronize(st));
-  const double norm = sqrt(hsc[0]);
-  double rr = hsc[0];
-  for (uint32_t it = 0; sqrt(rr) > 1e-15 * norm && it + 1 < 500; it++) {
-    H2B_CUDA_TRY(cudaMemsetAsync(ap, 0, sizeof(double) * nv, st));
-    mass_kernel<<<(nt + 127) / 128, 128, 0, st>>>(s->d_tri, nt, p, ap);
-    H2B_CUDA_TRY(cudaMemsetAsync(sc + 1, 0, sizeof(double) * 2, st));
-    dot_kernel<<<64, 256, 0, st>>>(p, ap, nv, sc + 1);
-    cg_update_kernel<<<64, 256, 0, st>>>(x, r, p, ap, nv, sc);
-    dot_kernel<<<64, 256, 0, st>>>(r, r, nv, sc + 2);
-    cg_dir_kernel<<<64, 256, 0, st>>>(p, r, nv, sc);
-    H2B_CUDA_TRY(cudaMemcpyAsync(sc, sc + 2, sizeof(double), cudaMemcpyDeviceToDevice, st));
-    H2B_CUDA_TRY(cudaMemcpyAsync(hsc, sc, sizeof(double), cudaMemcpyDeviceToHost, st));
-    H2B_CUDA_TRY(cudaStreamSynchronize(st));
-    rr = hsc[0];
-  }
+  mass_cg_kernel<<<CG_CTAS, CG_THREADS, 0, st>>>(s->d_tri, s->d_vt_off, s->d_vt_tri, nv, v, x, r, p,
+                                                 p1, ap);
+  h2b_note_launch();
+  H2B_CUDA_TRY(cudaGetLastError());
   H2B_CUDA_TRY(cudaMemcpyAsync(w, x, sizeof(double) * nv, cudaMemcpyDefault, st));
   H2B_CUDA_TRY(cudaStreamSynchronize(st));
   return H2B_OK;
