@@ -127,33 +127,58 @@ __device__ __forceinline__ void put_part(const GmresDev &g, const Sys &v, uint32
   v.part[(size_t) lb * g.ldpart * 2 + 2 * j + 1] = im;
 }
 
+// The vector kernels of a step take the columns of V in CGRP groups: thread (r, cg) has row r of the
+// CTA's TPB rows and the columns j = cg mod CGRP, so a thread's chain of loads is a quarter as long and
+// a small system (a few CTAs) keeps four times the loads in flight.  A step's vector kernels on
+// 1026 rows, k to 50: one thread per row 24.5 us, CGRP = 4 16.7; 96 systems of 570 rows on average
+// 36.6 and 34.0.
+constexpr int CGRP = 4;
+constexpr int VTHREADS = TPB * CGRP;
+
+// CTA -> (system, local row i, column group).  Returns false (uniformly per CTA) when the system is
+// not selected.
+template <bool CX>
+__device__ __forceinline__ bool step_view(const GmresDev &g, Sys &v, uint32_t &i, uint32_t &lb,
+                                          uint32_t &cg) {
+  const uint32_t s = g.blk[blockIdx.x];
+  v = sys_view<CX>(g, s);
+  lb = blockIdx.x - g.sys[s].blk0;
+  i = lb * TPB + (threadIdx.x & (TPB - 1));
+  cg = threadIdx.x / TPB;
+  return selected(v.state, GMRES_SEL_ACTIVE);
+}
+
 // part[lb][j] = sum over this CTA's rows of pj(j), for j = 0..k: one warp reduction per j into
-// shared memory and a single barrier, instead of a block-wide reduction (two barriers) per j.
+// shared memory and a single barrier.  A warp takes the columns of its group, eight at a time: their
+// loads are issued together and their shuffle trees interleave.
 template <bool CX, typename F>
 __device__ __forceinline__ void block_dots(const GmresDev &g, const Sys &v, uint32_t lb,
                                            uint32_t k, F pj) {
   __shared__ double ws[2][TPB / 32][GMRES_KMAX + 1];
-  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  // eight columns at a time: their loads are issued together and their eight shuffle trees
-  // interleave, instead of one load and one dependent tree per column (each column's sum is
-  // the same tree either way)
+  const uint32_t lane = threadIdx.x & 31, w = (threadIdx.x >> 5) & (TPB / 32 - 1);
+  const uint32_t cg = threadIdx.x / TPB;
   constexpr uint32_t CH = 8;
-  for (uint32_t j0 = 0; j0 <= k; j0 += CH) {
+  for (uint32_t j0 = cg; j0 <= k; j0 += CH * CGRP) {
     cd p[CH];
 #pragma unroll
-    for (uint32_t u = 0; u < CH; u++) p[u] = j0 + u <= k ? pj(j0 + u) : cd{0.0, 0.0};
+    for (uint32_t u = 0; u < CH; u++) {
+      const uint32_t j = j0 + u * CGRP;
+      p[u] = j <= k ? pj(j) : cd{0.0, 0.0};
+    }
 #pragma unroll
     for (uint32_t u = 0; u < CH; u++) {
+      const uint32_t j = j0 + u * CGRP;
+      if (j > k) break;  // uniform in the warp
       const double sr = warp_sum(p[u].re);
       const double si = CX ? warp_sum(p[u].im) : 0.0;
-      if (lane == 0 && j0 + u <= k) {
-        ws[0][w][j0 + u] = sr;
-        ws[1][w][j0 + u] = si;
+      if (lane == 0) {
+        ws[0][w][j] = sr;
+        ws[1][w][j] = si;
       }
     }
   }
   __syncthreads();
-  for (uint32_t j = threadIdx.x; j <= k; j += blockDim.x) {
+  for (uint32_t j = threadIdx.x; j <= k; j += VTHREADS) {
     double sr = 0.0, si = 0.0;
 #pragma unroll
     for (int q = 0; q < TPB / 32; q++) {
@@ -164,18 +189,44 @@ __device__ __forceinline__ void block_dots(const GmresDev &g, const Sys &v, uint
   }
 }
 
+// sum over the columns j <= k of V[i, j] u[j], every thread of a row gets it.  skip: a column left out
+// (UINT32_MAX: none).  us: u in shared memory.
+template <bool CX>
+__device__ __forceinline__ cd row_times(const Sys &v, uint32_t i, uint32_t cg, uint32_t k,
+                                        const double *us, uint32_t skip) {
+  __shared__ double ps[2][CGRP][TPB];
+  const uint32_t r = threadIdx.x & (TPB - 1);
+  cd t = {0.0, 0.0};
+  if (i < v.n) {
+    const uint32_t jmax = i < k ? i : k;  // V[i, j] = 0 for j > i
+#pragma unroll 8
+    for (uint32_t j = cg; j <= jmax; j += CGRP)
+      if (j != skip) t = cadd(t, cmul(vij<CX>(v, i, j), cd{us[2 * j], us[2 * j + 1]}));
+  }
+  ps[0][cg][r] = t.re;
+  if (CX) ps[1][cg][r] = t.im;
+  __syncthreads();
+  cd s = {0.0, 0.0};
+#pragma unroll
+  for (int c = 0; c < CGRP; c++) {
+    s.re += ps[0][c][r];
+    if (CX) s.im += ps[1][c][r];
+  }
+  return s;
+}
+
 // The new Krylov vector a = A q (in abuf) is moved into column k+1 of qr, and the partial sums
 // part[b][j] = sum_{i in block b} conj(V[i,j]) a[i] (j <= k) of w = V_{0..k}^H a are formed.
 template <bool CX>
-__global__ void __launch_bounds__(TPB) vth_kernel(GmresDev g) {
+__global__ void __launch_bounds__(VTHREADS) vth_kernel(GmresDev g) {
   Sys v;
-  uint32_t i, lb;
-  if (!vec_view<CX>(g, GMRES_SEL_ACTIVE, v, i, lb)) return;
+  uint32_t i, lb, cg;
+  if (!step_view<CX>(g, v, i, lb, cg)) return;
   const uint32_t k = v.state->k;
   double *col = v.qr + (size_t) (CX ? 2 : 1) * (k + 1) * v.n;
   const bool in = i < v.n;
   const cd x = in ? ld<CX>(v.abuf, i) : cd{0.0, 0.0};
-  if (in) st<CX>(col, i, x);
+  if (in && cg == 0) st<CX>(col, i, x);
   block_dots<CX>(g, v, lb, k, [&](uint32_t j) {
     return in ? cmul(cconj(vij<CX>(v, i, j)), x) : cd{0.0, 0.0};
   });
@@ -187,26 +238,21 @@ __global__ void __launch_bounds__(TPB) vth_kernel(GmresDev g) {
 // by the Householder factor gamma), taken before the scaling: gamma is a common factor of them,
 // applied once the bookkeeping has computed it.
 template <bool CX>
-__global__ void __launch_bounds__(TPB) apply_v_dots_kernel(GmresDev g) {
+__global__ void __launch_bounds__(VTHREADS) apply_v_dots_kernel(GmresDev g) {
   __shared__ double us[2 * GMRES_KMAX];
   Sys v;
-  uint32_t i, lb;
-  if (!vec_view<CX>(g, GMRES_SEL_ACTIVE, v, i, lb)) return;
+  uint32_t i, lb, cg;
+  if (!step_view<CX>(g, v, i, lb, cg)) return;
   const uint32_t k = v.state->k;
-  for (uint32_t j = threadIdx.x; j <= k; j += TPB) {
+  for (uint32_t j = threadIdx.x; j <= k; j += VTHREADS) {
     us[2 * j] = v.u[2 * j];
     us[2 * j + 1] = v.u[2 * j + 1];
   }
-  __syncthreads();
   double *a = v.qr + (size_t) (CX ? 2 : 1) * (k + 1) * v.n;
-  cd ai = {0.0, 0.0};
-  if (i < v.n) {
-    ai = ld<CX>(a, i);
-    const uint32_t jmax = i < k ? i : k;  // V[i, j] = 0 for j > i
-    for (uint32_t j = 0; j <= jmax; j++)
-      ai = csub(ai, cmul(vij<CX>(v, i, j), cd{us[2 * j], us[2 * j + 1]}));
-    st<CX>(a, i, ai);
-  }
+  const cd a0 = i < v.n ? ld<CX>(a, i) : cd{0.0, 0.0};
+  __syncthreads();  // u is there, and every thread of the row has read a
+  const cd ai = csub(a0, row_times<CX>(v, i, cg, k, us, UINT32_MAX));
+  if (i < v.n && cg == 0) st<CX>(a, i, ai);
   const bool below = i < v.n && i > k + 1;
   block_dots<CX>(g, v, lb, k + 1, [&](uint32_t j) {
     if (j == 0) return cd{(i < v.n && i >= k + 1) ? cabs2(ai) : 0.0, 0.0};
@@ -215,31 +261,41 @@ __global__ void __launch_bounds__(TPB) apply_v_dots_kernel(GmresDev g) {
 }
 
 // After the bookkeeping of a step (k is the new dimension): the new reflector's rows below k are
-// scaled by gamma (column k of qr; its row k holds the stored rotation), then q = e_k - V_{0..k} u.
-// Each thread scales its own row before it reads it.
+// scaled by gamma (column k of qr; its row k holds the stored rotation), then q = e_k - V_{0..k} u; abuf
+// is cleared for the next operator application.
 template <bool CX>
-__global__ void __launch_bounds__(TPB) scale_make_q_kernel(GmresDev g) {
+__global__ void __launch_bounds__(VTHREADS) scale_make_q_kernel(GmresDev g) {
   __shared__ double us[2 * GMRES_KMAX];
   Sys v;
-  uint32_t i, lb;
-  if (!vec_view<CX>(g, GMRES_SEL_ACTIVE, v, i, lb)) return;
+  uint32_t i, lb, cg;
+  if (!step_view<CX>(g, v, i, lb, cg)) return;
   const uint32_t k = v.state->k;
   const cd gamma = {v.state->gamma_re, v.state->gamma_im};
-  for (uint32_t j = threadIdx.x; j <= k; j += TPB) {
+  for (uint32_t j = threadIdx.x; j <= k; j += VTHREADS) {
     us[2 * j] = v.u[2 * j];
     us[2 * j + 1] = v.u[2 * j + 1];
   }
   __syncthreads();
-  if (i >= v.n) return;
+  // the columns before k; column k is scaled by the row's first thread, which adds its part
+  const cd t = row_times<CX>(v, i, cg, k, us, k);
+  if (i >= v.n || cg != 0) return;
+  cd vk = {i == k ? 1.0 : 0.0, 0.0};
   if (i > k) {
     double *col = v.qr + (size_t) (CX ? 2 : 1) * k * v.n;
-    st<CX>(col, i, cmul(ld<CX>(col, i), gamma));
+    vk = cmul(ld<CX>(col, i), gamma);
+    st<CX>(col, i, vk);
   }
   cd q = {i == k ? 1.0 : 0.0, 0.0};
-  const uint32_t jmax = i < k ? i : k;
-  for (uint32_t j = 0; j <= jmax; j++) q = csub(q, cmul(vij<CX>(v, i, j), cd{us[2 * j], us[2 * j + 1]}));
+  q = csub(csub(q, t), cmul(vk, cd{us[2 * k], us[2 * k + 1]}));
   st<CX>(v.q, i, q);
+  st<CX>(v.abuf, i, cd{0.0, 0.0});
 }
+
+// Bookkeeping kernels: one CTA of SMALL_THREADS threads per system, SGRP threads to an index of the
+// triangular products (each takes every SGRP-th term); sequential only where the algorithm is (Givens,
+// triangular solve).
+constexpr int SGRP = 2;
+constexpr int SMALL_THREADS = SGRP * GMRES_KMAX;
 
 // z[j] = sum over the system's blocks of part[b][j], j <= k.  Lanes take consecutive columns
 // (coalesced reads of a block's partial sums), warps take interleaved blocks, so every thread has
@@ -247,7 +303,7 @@ __global__ void __launch_bounds__(TPB) scale_make_q_kernel(GmresDev g) {
 // synchronises before reading z.
 __device__ void sum_parts_all(const GmresDev &g, const Sys &v, uint32_t k, double *zr,
                               double *zi, uint32_t j0 = 0) {
-  constexpr int NW = GMRES_KMAX / 32;  // warps of the bookkeeping CTA (GMRES_KMAX threads)
+  constexpr int NW = SMALL_THREADS / 32;  // warps of the bookkeeping CTA
   __shared__ double wsr[NW][GMRES_KMAX], wsi[NW][GMRES_KMAX];
   const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   for (uint32_t j = lane; j <= k; j += 32) {
@@ -276,9 +332,13 @@ __device__ void sum_parts_all(const GmresDev &g, const Sys &v, uint32_t k, doubl
 __device__ __forceinline__ cd Tij(const GmresDev &g, const Sys &v, uint32_t i, uint32_t j) {
   return {v.T[2 * ((size_t) i + (size_t) j * g.kmax)], v.T[2 * ((size_t) i + (size_t) j * g.kmax) + 1]};
 }
+// T is upper triangular; entry (i, j) is also kept at (j, i), so that threads over either index read
+// consecutive words
 __device__ __forceinline__ void setT(const GmresDev &g, const Sys &v, uint32_t i, uint32_t j, cd x) {
   v.T[2 * ((size_t) i + (size_t) j * g.kmax)] = x.re;
   v.T[2 * ((size_t) i + (size_t) j * g.kmax) + 1] = x.im;
+  v.T[2 * ((size_t) j + (size_t) i * g.kmax)] = x.re;
+  v.T[2 * ((size_t) j + (size_t) i * g.kmax) + 1] = x.im;
 }
 
 // Householder scalars of a column with entries diag (first) and squared norm norm2
@@ -339,9 +399,7 @@ __device__ cd findapply_givens(cd *a, cd *b, bool unitary) {
   return rho;
 }
 
-__device__ void apply_givens(cd rho, cd *a, cd *b, bool unitary) {
-  const cd aa = *a, bb = *b;
-  cd s, c;
+__device__ void givens_cs(cd rho, cd &c, cd &s) {
   if (cabs2(rho) < 1.0) {
     s = rho;
     c = {sqrt(1.0 - cabs2(s)), 0.0};
@@ -352,14 +410,19 @@ __device__ void apply_givens(cd rho, cd *a, cd *b, bool unitary) {
     c = {1.0, 0.0};
     s = {0.0, 0.0};
   }
+}
+
+__device__ __forceinline__ void rotate_givens(cd c, cd s, cd *a, cd *b, bool unitary) {
+  const cd aa = *a, bb = *b;
   *a = cadd(cmul(c, aa), cmul(s, bb));
   *b = unitary ? csub(cmul(cconj(c), bb), cmul(cconj(s), aa)) : csub(cmul(c, bb), cmul(s, aa));
 }
 
-// Bookkeeping kernels: one CTA of SMALL_THREADS threads (>= kmax) per system; O(k) work per
-// thread for the triangular products, sequential only where the algorithm is (Givens, triangular
-// solve).
-constexpr int SMALL_THREADS = GMRES_KMAX;
+__device__ void apply_givens(cd rho, cd *a, cd *b, bool unitary) {
+  cd c, s;
+  givens_cs(rho, c, s);
+  rotate_givens(c, s, a, b, unitary);
+}
 
 __device__ double block_sum_small(double v, double *red) {
   v = warp_sum(v);
@@ -375,13 +438,15 @@ template <bool CX>
 __global__ void __launch_bounds__(SMALL_THREADS) small_kernel(GmresDev g, int phase, int sel) {
   __shared__ double zr[GMRES_KMAX], zi[GMRES_KMAX], red[SMALL_THREADS / 32];
   __shared__ double wr[GMRES_KMAX], wi[GMRES_KMAX];
-  __shared__ double hs[4];  // phase 1: gamma, alpha
+  __shared__ double hs[6];  // phase 1: gamma, alpha, tau
+  __shared__ double pr[SGRP][GMRES_KMAX], pi[SGRP][GMRES_KMAX];  // the groups' sums
+  __shared__ double cr[GMRES_KMAX], ci[GMRES_KMAX];  // phase 1: cosines of the stored rotations
   __shared__ double yr[GMRES_KMAX], yi[GMRES_KMAX];  // phase 1: conj(V[k+1, j])
   const Sys v = sys_view<CX>(g, blockIdx.x);
   GmresState *s = v.state;
   if (!selected(s, sel)) return;
   const uint32_t k = s->k;
-  const uint32_t t = threadIdx.x;
+  const uint32_t t = threadIdx.x, r = t & (GMRES_KMAX - 1), sg = t / GMRES_KMAX;
   __syncthreads();  // every thread has read k before anyone may change it
   if (phase == 0) {
     // after vth: w = V^H a; u = T^H w
@@ -391,57 +456,63 @@ __global__ void __launch_bounds__(SMALL_THREADS) small_kernel(GmresDev g, int ph
       v.w[2 * t] = zr[t];
       v.w[2 * t + 1] = zi[t];
     }
+    cd u = {0.0, 0.0};
+    if (r <= k) {
+#pragma unroll 8
+      for (uint32_t i = sg; i <= r; i += SGRP)
+        u = cadd(u, cmul(cconj(Tij(g, v, r, i)), cd{zr[i], zi[i]}));
+    }
+    pr[sg][r] = u.re;
+    pi[sg][r] = u.im;
+    __syncthreads();
     if (t <= k) {
-      cd u = {0.0, 0.0};
-      for (uint32_t i = 0; i <= t; i++) u = cadd(u, cmul(cconj(Tij(g, v, i, t)), cd{zr[i], zi[i]}));
-      v.u[2 * t] = u.re;
-      v.u[2 * t + 1] = u.im;
+      v.u[2 * t] = pr[0][t] + pr[1][t];
+      v.u[2 * t + 1] = pi[0][t] + pi[1][t];
     }
   } else if (phase == 1) {
     // after apply_v_dots: the Householder scalars of column k+1 from ||a[k+1..n)||^2 (part slot
     // 0); the T column k+1 from the reflector products (part slots 1..k+1, times gamma); u for q;
     // the Givens rotations of the new Hessenberg column (entry k+1 = alpha); k += 1.
-    {
-      // y_j = conj(V[k+1, j]) (j <= k), read before anything waits on the Householder scalars
-      if (t <= k) {
-        const cd y = cconj(vij<CX>(v, k + 1, t));
-        yr[t] = y.re;
-        yi[t] = y.im;
-      }
-      double part = 0.0;
-      for (uint32_t b = t; b < v.nblk; b += SMALL_THREADS)
-        part += v.part[(size_t) b * g.ldpart * 2];
-      const double norm2 = block_sum_small(part, red);
-      if (t == 0) {
-        const double *a = v.qr + (size_t) (CX ? 2 : 1) * (k + 1) * v.n;
-        householder(k + 1 < v.n ? ld<CX>(a, k + 1) : cd{0.0, 0.0}, norm2, s, k + 1, v);
-        hs[0] = s->gamma_re;
-        hs[1] = s->gamma_im;
-        hs[2] = s->alpha_re;
-        hs[3] = s->alpha_im;
-      }
-      __syncthreads();
-    }
-    const cd tau = {v.tau[2 * (k + 1)], v.tau[2 * (k + 1) + 1]};
-    sum_parts_all(g, v, k, zr, zi, 1u);
-    __syncthreads();
-    if (t <= k) {  // gamma z + conj(v_t[k+1])
-      cd z = cmul(cd{zr[t], zi[t]}, cd{hs[0], hs[1]});
-      z = cadd(z, cd{yr[t], yi[t]});
-      zr[t] = z.re;
-      zi[t] = z.im;
-    }
-    __syncthreads();
-    // T column k+1: T[t, k+1] = -tau sum_{j=t..k} T[t, j] z_j, T[k+1, k+1] = tau; and
-    // u = T y with y_{k+1} = 1: both sums run over row t of T in one pass
+    // y_j = conj(V[k+1, j]) (j <= k)
     if (t <= k) {
-      cd acc = {0.0, 0.0}, uy = {0.0, 0.0};
-#pragma unroll 4
-      for (uint32_t j = t; j <= k; j++) {
-        const cd tv = Tij(g, v, t, j);
-        acc = cadd(acc, cmul(tv, cd{zr[j], zi[j]}));
+      const cd y = cconj(vij<CX>(v, k + 1, t));
+      yr[t] = y.re;
+      yi[t] = y.im;
+    }
+    sum_parts_all(g, v, k + 1, zr, zi);
+    __syncthreads();
+    // The T column k+1 is T[t, k+1] = -tau sum_{j=t..k} T[t, j] (gamma z_j + y_j), T[k+1, k+1] = tau,
+    // and u = T y with y_{k+1} = 1: both sums run over row t of T without the Householder scalars,
+    // which the last thread forms meanwhile (zr[0] = ||a[k+1..n)||^2, z_j in zr[1 + j])
+    cd acc = {0.0, 0.0}, uy = {0.0, 0.0};
+    if (r <= k) {
+#pragma unroll 8
+      for (uint32_t j = r + sg; j <= k; j += SGRP) {
+        const cd tv = Tij(g, v, r, j);
+        acc = cadd(acc, cmul(tv, cd{zr[j + 1], zi[j + 1]}));
         uy = cadd(uy, cmul(tv, cd{yr[j], yi[j]}));
       }
+    }
+    if (sg == 1) {
+      pr[0][r] = acc.re, pi[0][r] = acc.im;
+      pr[1][r] = uy.re, pi[1][r] = uy.im;
+    }
+    if (t == SMALL_THREADS - 1) {
+      const double *a = v.qr + (size_t) (CX ? 2 : 1) * (k + 1) * v.n;
+      householder(k + 1 < v.n ? ld<CX>(a, k + 1) : cd{0.0, 0.0}, zr[0], s, k + 1, v);
+      hs[0] = s->gamma_re;
+      hs[1] = s->gamma_im;
+      hs[2] = s->alpha_re;
+      hs[3] = s->alpha_im;
+      hs[4] = v.tau[2 * (k + 1)];
+      hs[5] = v.tau[2 * (k + 1) + 1];
+    }
+    __syncthreads();
+    const cd tau = {hs[4], hs[5]};
+    if (t <= k) {
+      acc = cadd(acc, cd{pr[0][t], pi[0][t]});
+      uy = cadd(uy, cd{pr[1][t], pi[1][t]});
+      acc = cadd(cmul(acc, cd{hs[0], hs[1]}), uy);
       const cd tn = cmul(cd{-tau.re, -tau.im}, acc);
       setT(g, v, t, k + 1, tn);
       uy = cadd(uy, tn);
@@ -453,8 +524,9 @@ __global__ void __launch_bounds__(SMALL_THREADS) small_kernel(GmresDev g, int ph
       v.u[2 * t + 1] = tau.im;
     }
     // Givens rotations on the new Hessenberg column (rows 0..k+1 of column k+1): the column and
-    // the stored rotations (diagonal of the previous columns) are staged in shared memory, so the
-    // sequential sweep by one thread never waits on global memory.
+    // the cosines and sines of the stored rotations (diagonal of the previous columns) are put in
+    // shared memory by all threads, so the sequential sweep by one thread is four products per
+    // rotation: no square root, division or global load in its chain.
     double *col = v.qr + (size_t) (CX ? 2 : 1) * (k + 1) * v.n;
     __syncthreads();  // zr / zi (read by the T loop above) are reused below
     if (t <= k + 1) {
@@ -463,20 +535,26 @@ __global__ void __launch_bounds__(SMALL_THREADS) small_kernel(GmresDev g, int ph
       wi[t] = c.im;
     }
     if (t < k) {
-      const cd r = ld<CX>(v.qr + (size_t) (CX ? 2 : 1) * (t + 1) * v.n, t + 1);
-      zr[t] = r.re;
-      zi[t] = r.im;
+      cd c, sn;
+      givens_cs(ld<CX>(v.qr + (size_t) (CX ? 2 : 1) * (t + 1) * v.n, t + 1), c, sn);
+      cr[t] = c.re;
+      ci[t] = c.im;
+      zr[t] = sn.re;
+      zi[t] = sn.im;
     }
     __syncthreads();
     if (t == 0) {
+      cd x = {wr[0], wi[0]};
+#pragma unroll 4
       for (uint32_t i = 0; i < k; i++) {
-        cd a = {wr[i], wi[i]}, b = {wr[i + 1], wi[i + 1]};
-        apply_givens(cd{zr[i], zi[i]}, &a, &b, g.unitary != 0);
-        wr[i] = a.re;
-        wi[i] = a.im;
-        wr[i + 1] = b.re;
-        wi[i + 1] = b.im;
+        cd y = {wr[i + 1], wi[i + 1]};
+        rotate_givens(cd{cr[i], ci[i]}, cd{zr[i], zi[i]}, &x, &y, g.unitary != 0);
+        wr[i] = x.re;
+        wi[i] = x.im;
+        x = y;
       }
+      wr[k] = x.re;
+      wi[k] = x.im;
       cd a = {wr[k], wi[k]}, b = {wr[k + 1], wi[k + 1]};
       const cd rho = findapply_givens(&a, &b, g.unitary != 0);
       wr[k] = a.re;
@@ -626,13 +704,16 @@ __global__ void __launch_bounds__(TPB) init0_kernel(GmresDev g, const double *b,
   if (threadIdx.x == 0) put_part(g, v, lb, 0, s, 0.0);
 }
 
-// column 0: scale rows > 0 by gamma, row 0 = alpha; q = H_0 e_0 = e_0 - tau_0 v_0
+// column 0: scale rows > 0 by gamma, row 0 = alpha; q = H_0 e_0 = e_0 - tau_0 v_0.  abuf, which init0
+// has read, is cleared for the next step of every system (the operator wrote all of it).
 template <bool CX>
 __global__ void __launch_bounds__(TPB) scale0_kernel(GmresDev g, int sel) {
   Sys v;
   uint32_t i, lb;
-  if (!vec_view<CX>(g, sel, v, i, lb)) return;
+  const bool on = vec_view<CX>(g, sel, v, i, lb);
   if (i >= v.n) return;
+  st<CX>(v.abuf, i, cd{0.0, 0.0});
+  if (!on) return;
   const cd gamma = {v.state->gamma_re, v.state->gamma_im};
   const cd tau = {v.tau[0], v.tau[1]};
   if (i == 0) {
@@ -648,17 +729,17 @@ __global__ void __launch_bounds__(TPB) scale0_kernel(GmresDev g, int sel) {
 template <bool CX>
 int step_impl(const GmresDev &g, const GmresOp &op, cudaStream_t st) {
   const uint32_t nb = g.nblocks;
-  // a = A q into the staging vector, then into column k+1 of qr (k is read on the device)
-  zero_abuf_kernel<CX><<<nb, TPB, 0, st>>>(g);
+  // a = A q into the staging vector (cleared by the step or restart before), then into column k+1 of
+  // qr (k is read on the device)
   int rc = (op.apply_lo ? op.apply_lo : op.apply)(op.ctx, g.q, g.abuf, 1.0, 0.0, st);
   if (rc != H2B_OK) return rc;
   // w = V^H a; u = T^H w; a -= V u with the next column's norm and dot products; Householder
   // scalars, T column, Givens (k += 1); scaled reflector and q
-  vth_kernel<CX><<<nb, TPB, 0, st>>>(g);
+  vth_kernel<CX><<<nb, VTHREADS, 0, st>>>(g);
   small_kernel<CX><<<g.nsys, SMALL_THREADS, 0, st>>>(g, 0, GMRES_SEL_ACTIVE);
-  apply_v_dots_kernel<CX><<<nb, TPB, 0, st>>>(g);
+  apply_v_dots_kernel<CX><<<nb, VTHREADS, 0, st>>>(g);
   small_kernel<CX><<<g.nsys, SMALL_THREADS, 0, st>>>(g, 1, GMRES_SEL_ACTIVE);
-  scale_make_q_kernel<CX><<<nb, TPB, 0, st>>>(g);
+  scale_make_q_kernel<CX><<<nb, VTHREADS, 0, st>>>(g);
   H2B_CUDA_TRY(cudaGetLastError());
   return H2B_OK;
 }
