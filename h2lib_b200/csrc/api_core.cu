@@ -6,6 +6,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <algorithm>
 #include <atomic>
 #include <mutex>
 #include <vector>
@@ -184,13 +185,35 @@ extern "C" h2b_surface *h2b_surface_new(uint32_t vertices, const double *x, uint
                       cudaMemcpyHostToDevice, s->stream) != cudaSuccess ||
       cudaMemcpyAsync(s->d_vt_tri, s->adj.tri, sizeof(uint32_t) * 3ull * triangles,
                       cudaMemcpyHostToDevice, s->stream) != cudaSuccess ||
-      cudaStreamSynchronize(s->stream) != cudaSuccess) {
+      cudaStreamSynchronize(s->stream) != cudaSuccess) {  // rec is read
     h2b_set_error("h2b_surface_new: %s", cudaGetErrorString(cudaGetLastError()));
     h2b_surface_del(s);
     return NULL;
   }
   s->device = dev;
   s->num_sms = sms;
+  // neighbour lists: about 18 per triangle on usual meshes
+  uint64_t room = 0;
+  for (uint32_t v = 0; v < vertices; v++) {
+    const uint64_t d = s->adj.off[v + 1] - s->adj.off[v];
+    room += d * d;
+  }
+  if (room <= 64ull * triangles && room < UINT32_MAX) {
+    uint32_t *cursor = nullptr;
+    const cudaStream_t st = s->stream;
+    if (cudaMallocAsync(&cursor, sizeof(uint32_t), st) != cudaSuccess ||
+        cudaMallocAsync(&s->d_nb_off, sizeof(uint32_t) * (size_t) triangles, st) != cudaSuccess ||
+        cudaMallocAsync(&s->d_nb_len, sizeof(uint32_t) * (size_t) triangles, st) != cudaSuccess ||
+        cudaMallocAsync(&s->d_nb, sizeof(uint2) * room, st) != cudaSuccess ||
+        cudaMemsetAsync(cursor, 0, sizeof(uint32_t), st) != cudaSuccess ||
+        h2b_near_neighbours(s->d_tri, triangles, s->d_vt_off, s->d_vt_tri, cursor, s->d_nb_off,
+                            s->d_nb_len, s->d_nb, st) != H2B_OK ||
+        cudaFreeAsync(cursor, st) != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess) {
+      h2b_set_error("h2b_surface_new: %s", cudaGetErrorString(cudaGetLastError()));
+      h2b_surface_del(s);
+      return NULL;
+    }
+  }
   return s;
 }
 
@@ -201,6 +224,9 @@ extern "C" void h2b_surface_del(h2b_surface *s) {
   if (s->d_tri) cudaFreeAsync(s->d_tri, s->stream);
   if (s->d_qrec) cudaFreeAsync(s->d_qrec, s->stream);
   if (s->d_x) cudaFreeAsync(s->d_x, s->stream);
+  if (s->d_nb_off) cudaFreeAsync(s->d_nb_off, s->stream);
+  if (s->d_nb_len) cudaFreeAsync(s->d_nb_len, s->stream);
+  if (s->d_nb) cudaFreeAsync(s->d_nb, s->stream);
   if (s->d_vt_off) cudaFreeAsync(s->d_vt_off, s->stream);
   if (s->d_vt_tri) cudaFreeAsync(s->d_vt_tri, s->stream);
   if (s->stream) cudaStreamDestroy(s->stream);
@@ -392,37 +418,56 @@ uint32_t h2b_bem_cols(const h2b_bem *b) {
   return b->col_basis == H2B_BASIS_LINEAR ? b->s->nv : b->s->nt;
 }
 
-// Upload a finished plan; device arrays returned in *dp (freed by h2b_devplan_free).
-int h2b_devplan_upload(const h2b_nearplan *p, cudaStream_t st, h2b_devplan *dp) {
+// The tiles of one block (rows x cols indices in tiles of `tile`) on the device: the host lists the
+// triangles of each side's parts, the tiles themselves are written by a kernel (a dense matrix of
+// 8192 indices has 16384 of them, which took 0.4 ms on the host).  Device arrays in *dp, freed by
+// h2b_devplan_free.
+static int block_plan(const h2b_bem *bem, const uint32_t *ridx, uint32_t rows, const uint32_t *cidx,
+                      uint32_t cols, uint32_t ld, int ntrans, uint32_t tile, bool same, cudaStream_t st,
+                      h2b_devplan *dp) {
   memset(dp, 0, sizeof(*dp));
-  dp->ntiles = p->ntiles;
-  dp->nsing = p->nsing;
-  dp->nvert = p->nsing ? p->case_start[2] - p->case_start[1] : 0;
-  if (p->ntiles) {
-    H2B_CUDA_TRY(cudaMallocAsync(&dp->tiles, sizeof(h2b_tile) * p->ntiles, st));
-    H2B_CUDA_TRY(cudaMemcpyAsync(dp->tiles, p->tiles, sizeof(h2b_tile) * p->ntiles,
-                                 cudaMemcpyHostToDevice, st));
+  h2b_adjacency *adj = const_cast<h2b_adjacency *>(&bem->s->adj);
+  const uint32_t nr = (rows + tile - 1) / tile, nc = (cols + tile - 1) / tile;
+  if ((uint64_t) nr * nc > UINT32_MAX / 2) {
+    h2b_set_error("h2b_bem_nearfield: %u x %u entries are too many for one call", rows, cols);
+    return H2B_ERR_ARG;
   }
-  bool mates = false;
-  for (uint32_t i = 0; i < p->ntiles && !mates; i++) mates = p->tiles[i].mate != 0;
-  if (mates) {
-    std::vector<uint32_t> half(p->ntiles);
-    dp->nhalf = h2b_nearplan_halves(p, half.data());
-    H2B_CUDA_TRY(cudaMallocAsync(&dp->half, sizeof(uint32_t) * dp->nhalf, st));
-    H2B_CUDA_TRY(cudaMemcpyAsync(dp->half, half.data(), sizeof(uint32_t) * dp->nhalf,
-                                 cudaMemcpyHostToDevice, st));
+  struct Plan : h2b_nearplan {
+    Plan() { h2b_nearplan_init(this); }
+    ~Plan() { h2b_nearplan_free(this); }
+  } plan;
+  std::vector<uint32_t> lists(2ull * (nr + nc));
+  const int rl = bem->row_basis == H2B_BASIS_LINEAR, cl = bem->col_basis == H2B_BASIS_LINEAR;
+  int rc = H2B_OK;
+  for (uint32_t i = 0; rc == H2B_OK && i < nr; i++)
+    rc = h2b_nearplan_tile_list(&plan, adj, rl, ridx + (size_t) i * tile,
+                                std::min(tile, rows - i * tile), &lists[i], &lists[nr + i]);
+  for (uint32_t j = 0; rc == H2B_OK && j < nc; j++)
+    rc = h2b_nearplan_tile_list(&plan, adj, cl, cidx + (size_t) j * tile,
+                                std::min(tile, cols - j * tile), &lists[2 * nr + j],
+                                &lists[2 * nr + nc + j]);
+  if (rc != H2B_OK) {
+    h2b_set_error("h2b_bem_nearfield: out of host memory building the plan");
+    return rc;
   }
-  if (p->nrefs) {
-    H2B_CUDA_TRY(cudaMallocAsync(&dp->refs, sizeof(h2b_triref) * p->nrefs, st));
-    H2B_CUDA_TRY(cudaMemcpyAsync(dp->refs, p->refs, sizeof(h2b_triref) * p->nrefs,
-                                 cudaMemcpyHostToDevice, st));
+  dp->ntiles = nr * nc;
+  dp->nhalf = same ? nr * (nr + 1) / 2 : 0;
+  uint32_t *d_lists = nullptr;
+  if (cudaMallocAsync((void **) &dp->tiles, sizeof(h2b_tile) * dp->ntiles, st) != cudaSuccess ||
+      (same && cudaMallocAsync((void **) &dp->half, sizeof(uint32_t) * dp->nhalf, st) != cudaSuccess) ||
+      cudaMallocAsync((void **) &dp->refs, sizeof(h2b_triref) * std::max(1u, plan.nrefs), st) != cudaSuccess ||
+      cudaMemcpyAsync(dp->refs, plan.refs, sizeof(h2b_triref) * plan.nrefs, cudaMemcpyHostToDevice,
+                      st) != cudaSuccess ||
+      cudaMallocAsync((void **) &d_lists, sizeof(uint32_t) * lists.size(), st) != cudaSuccess ||
+      cudaMemcpyAsync(d_lists, lists.data(), sizeof(uint32_t) * lists.size(),
+                      cudaMemcpyHostToDevice, st) != cudaSuccess) {
+    h2b_set_error("h2b_bem_nearfield: %s", cudaGetErrorString(cudaGetLastError()));
+    rc = H2B_ERR_CUDA;
   }
-  if (p->nsing) {
-    H2B_CUDA_TRY(cudaMallocAsync(&dp->sing, sizeof(h2b_sing) * p->nsing, st));
-    H2B_CUDA_TRY(cudaMemcpyAsync(dp->sing, p->sing, sizeof(h2b_sing) * p->nsing,
-                                 cudaMemcpyHostToDevice, st));
-  }
-  return H2B_OK;
+  if (rc == H2B_OK)
+    rc = h2b_near_grid_tiles(d_lists, nr, nc, rows, cols, tile, ld, ntrans, dp->tiles, dp->half, st);
+  if (d_lists) cudaFreeAsync(d_lists, st);
+  return rc;
 }
 
 int h2b_classify_device(const h2b_surface *s, const void *refs, const h2b_tile *tiles,
@@ -432,11 +477,12 @@ int h2b_classify_device(const h2b_surface *s, const void *refs, const h2b_tile *
   uint32_t *d_cur = nullptr;
   H2B_CUDA_TRY(cudaMallocAsync(&d_cur, sizeof(uint32_t) * 8, st));
   int rc = H2B_OK;
-  uint32_t host[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  // d_cur[0..3]: pairs per case of the count pass, [4..7]: the write pass's cursors
+  uint32_t host[4] = {0, 0, 0, 0};
   if (cudaMemsetAsync(d_cur, 0, sizeof(uint32_t) * 8, st) != cudaSuccess) rc = H2B_ERR_CUDA;
   if (rc == H2B_OK)
-    rc = h2b_near_classify(s->d_tri, refs, tiles, ntiles, s->d_vt_off, s->d_vt_tri, d_cur, nullptr,
-                           nullptr, st);
+    rc = h2b_near_classify(s->d_tri, refs, tiles, ntiles, s->d_nb_off, s->d_nb_len, s->d_nb, d_cur,
+                           nullptr, nullptr, st);
   if (rc == H2B_OK &&
       (cudaMemcpyAsync(host, d_cur, sizeof(uint32_t) * 4, cudaMemcpyDeviceToHost, st) !=
            cudaSuccess ||
@@ -449,23 +495,12 @@ int h2b_classify_device(const h2b_surface *s, const void *refs, const h2b_tile *
     cudaFreeAsync(d_cur, st);
     return H2B_ERR_ARG;
   }
-  if (rc == H2B_OK) {
-    // base offsets of the cases in host[4..7]
-    host[4] = 0;
-    host[5] = 0;
-    host[6] = host[1];
-    host[7] = host[1] + host[2];
-    if (nsing &&
-        (cudaMallocAsync((void **) d_sing, sizeof(h2b_sing) * nsing, st) != cudaSuccess ||
-         cudaMemsetAsync(d_cur, 0, sizeof(uint32_t) * 4, st) != cudaSuccess ||
-         cudaMemcpyAsync(d_cur + 4, host + 4, sizeof(uint32_t) * 4, cudaMemcpyHostToDevice, st) !=
-             cudaSuccess))
-      rc = H2B_ERR_CUDA;
-  }
+  if (rc == H2B_OK && nsing &&
+      cudaMallocAsync((void **) d_sing, sizeof(h2b_sing) * nsing, st) != cudaSuccess)
+    rc = H2B_ERR_CUDA;
   if (rc == H2B_OK && nsing)
-    rc = h2b_near_classify(s->d_tri, refs, tiles, ntiles, s->d_vt_off, s->d_vt_tri, d_cur,
-                           d_cur + 4, *d_sing, st);
-  if (rc == H2B_OK && cudaStreamSynchronize(st) != cudaSuccess) rc = H2B_ERR_CUDA;
+    rc = h2b_near_classify(s->d_tri, refs, tiles, ntiles, s->d_nb_off, s->d_nb_len, s->d_nb, d_cur + 4,
+                           d_cur, *d_sing, st);
   if (rc == H2B_ERR_CUDA)
     h2b_set_error("singular-pair classification: %s", cudaGetErrorString(cudaGetLastError()));
   cudaFreeAsync(d_cur, st);
@@ -593,28 +628,8 @@ extern "C" int h2b_bem_nearfield(const h2b_bem *bem, const uint32_t *ridx, uint3
   if (same) cidx = ridx;  // one set of triangle lists
   const uint32_t tile = block_tile(bem, rows, cols, same);
 
-  // the singular pairs are found on the device (h2b_classify_device): the host plan only lists
-  // the tiles and their triangles
-  h2b_nearplan plan;
-  h2b_nearplan_init(&plan);
-  plan.skip_sing = 1;
-  rc = h2b_nearplan_add_block(&plan, const_cast<h2b_adjacency *>(&s->adj), bem->row_basis,
-                              bem->col_basis, ridx, rows, cidx, cols, 0, (uint32_t) ld_dev,
-                              ntrans, tile);
-  if (rc == H2B_OK) rc = h2b_nearplan_finalize(&plan);
-  // equal row and column index lists: tiles (I, J) and (J, I) take the same triangle pairs
-  if (rc == H2B_OK && same) {
-    const uint32_t nt = (rows + tile - 1) / tile;
-    h2b_nearplan_mate(&plan, 0, 0, nt, nt);
-  }
-  if (rc != H2B_OK) {
-    h2b_nearplan_free(&plan);
-    h2b_set_error("h2b_bem_nearfield: out of host memory building the plan");
-    return rc;
-  }
   h2b_devplan dp;
-  rc = h2b_devplan_upload(&plan, st, &dp);
-  h2b_nearplan_free(&plan);
+  rc = block_plan(bem, ridx, rows, cidx, cols, (uint32_t) ld_dev, ntrans, tile, same, st, &dp);
   if (rc != H2B_OK) {
     h2b_devplan_free(&dp, st);
     return rc;

@@ -23,6 +23,10 @@ struct h2b_surface {
   QuadRec *d_qrec = nullptr;    // nt records (distant rule of order 2)
   double *d_x = nullptr;        // 3*nv
   uint32_t *d_vt_off = nullptr, *d_vt_tri = nullptr;  // vertex -> triangles (CSR, from adj)
+  // triangle -> triangles around it with their permutation codes (h2b_near_neighbours); nullptr on
+  // meshes whose lists would be long (vertices with very many triangles)
+  uint32_t *d_nb_off = nullptr, *d_nb_len = nullptr;
+  uint2 *d_nb = nullptr;
 };
 
 struct h2b_bem {
@@ -59,12 +63,12 @@ int h2b_bem_kernel_kind(const h2b_bem *b);
 void h2b_fill_launch(const h2b_bem *b, h2b_near_launch *L);
 uint32_t h2b_bem_rows(const h2b_bem *b);
 uint32_t h2b_bem_cols(const h2b_bem *b);
-int h2b_devplan_upload(const h2b_nearplan *p, cudaStream_t st, h2b_devplan *dp);
 void h2b_devplan_free(h2b_devplan *dp, cudaStream_t st);
 // Singular pairs of uploaded tiles, found on the device in two passes (count, then write grouped
 // by Sauter-Schwab case: vertex, edge, identical; order inside a case not fixed).  *d_sing: a
 // stream-ordered device array of cnt[1] + cnt[2] + cnt[3] pairs (nullptr when there are none);
-// cnt[c]: pairs of case c = 1..3.  Synchronises st.
+// cnt[c]: pairs of case c = 1..3.  Synchronises
+// st after the count; the pairs are written on st.
 int h2b_classify_device(const h2b_surface *s, const void *refs, const h2b_tile *tiles,
                         uint32_t ntiles, cudaStream_t st, h2b_sing **d_sing, uint32_t cnt[4]);
 int h2b_check_err_flag(const h2b_bem *b, cudaStream_t st);

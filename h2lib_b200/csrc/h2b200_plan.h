@@ -85,6 +85,10 @@ int h2b_nearplan_finalize(h2b_nearplan *p);
  * constant: the triangles themselves), appended to p->refs. */
 int h2b_nearplan_add_reflist(h2b_nearplan *p, h2b_adjacency *adj, int linear,
                              const uint32_t *idx, uint32_t n, uint32_t *off, uint32_t *len);
+/* The same list as a tile's side takes it: ordered by id with slots (linear), and shared with the other
+ * tiles on the same index pointer. */
+int h2b_nearplan_tile_list(h2b_nearplan *p, h2b_adjacency *adj, int linear, const uint32_t *idx,
+                           uint32_t n, uint32_t *off, uint32_t *len);
 uint32_t h2b_pair_code(const uint32_t *tv, const uint32_t *sv);
 /* Marks the tiles of one block (row and column index lists equal: first tile t0, nt tiles per side)
  * or of two blocks with exchanged row and column lists (t0: nr x nc tiles, t1: nc x nr tiles) as each

@@ -338,6 +338,13 @@ cached_reflist(h2b_nearplan *p, h2b_adjacency *adj, int linear, const uint32_t *
   return H2B_OK;
 }
 
+int
+h2b_nearplan_tile_list(h2b_nearplan *p, h2b_adjacency *adj, int linear, const uint32_t *idx,
+                       uint32_t n, uint32_t *off, uint32_t *len)
+{
+  return cached_reflist(p, adj, linear, idx, n, off, len);
+}
+
 static int
 add_tile(h2b_nearplan *p, h2b_adjacency *adj, int row_linear, int col_linear,
          const uint32_t *ridx, uint32_t rows, const uint32_t *cidx, uint32_t cols,

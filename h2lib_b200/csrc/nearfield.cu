@@ -1876,69 +1876,131 @@ __global__ void __launch_bounds__(256) unique_pairs_kernel(const TriRec *tri, co
 }
 
 
+// The triangles around each triangle: a triangle around several vertices of t is taken at the first
+// of them.  A CTA reserves room for its triangles' vertex lists with one addition to the cursor.
+__global__ void __launch_bounds__(128) neighbours_kernel(const TriRec *tri, uint32_t nt,
+                                                         const uint32_t *vt_off,
+                                                         const uint32_t *vt_tri, uint32_t *cursor,
+                                                         uint32_t *off, uint32_t *len, uint2 *nb) {
+  __shared__ uint32_t wsum[4], base;
+  const uint32_t t = blockIdx.x * 128 + threadIdx.x, lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+  uint32_t tv[3] = {0, 0, 0}, room = 0;
+  if (t < nt)
+    for (int k = 0; k < 3; k++) {
+      tv[k] = tri[t].v[k];
+      room += vt_off[tv[k] + 1] - vt_off[tv[k]];
+    }
+  uint32_t pre = room;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t v = __shfl_up_sync(0xffffffffu, pre, o);
+    if (lane >= (uint32_t) o) pre += v;
+  }
+  if (lane == 31) wsum[w] = pre;
+  __syncthreads();
+  if (threadIdx.x == 0) base = atomicAdd(cursor, wsum[0] + wsum[1] + wsum[2] + wsum[3]);
+  __syncthreads();
+  if (t >= nt) return;
+  uint32_t at = base + pre - room, n = 0;
+  for (uint32_t q = 0; q < w; q++) at += wsum[q];
+  off[t] = at;
+  for (int k = 0; k < 3; k++)
+    for (uint32_t a = vt_off[tv[k]]; a < vt_off[tv[k] + 1]; a++) {
+      const uint32_t s = vt_tri[a];
+      const uint32_t sv[3] = {tri[s].v[0], tri[s].v[1], tri[s].v[2]};
+      bool seen = false;
+      for (int k2 = 0; k2 < k; k2++) seen |= sv[0] == tv[k2] || sv[1] == tv[k2] || sv[2] == tv[k2];
+      if (!seen) nb[at + n++] = make_uint2(s, pair_code_dev(tv, sv));
+    }
+  len[t] = n;
+}
+
 // One CTA per tile.  The tile's column triangles go into a shared-memory hash table (triangle id
-// -> position in the column list); a thread per row triangle t visits the triangles around t's
-// vertices (the surface's vertex -> triangle lists) and looks each one up, so the pairs found are
-// exactly the tile's pairs that share a vertex, without testing the others.  A triangle around
-// several vertices of t is taken at the first of them.  Counts per case are gathered in shared
-// memory: the count pass adds them to cursor[c]; the write pass reserves the tile's range of
-// case c with one atomic and writes its pairs there.  Column lists longer than half the table
-// take classify_all_pairs.
+// -> position in the column list); the triangles around each row triangle (the surface's neighbour
+// lists, eight lanes to a row triangle) are looked up in it, so the pairs found are exactly the
+// tile's pairs that share a vertex, without testing the others.  Counts per case are gathered in
+// shared memory: the count pass adds them to cursor[c]; the write pass reserves the tile's range of
+// case c with one atomic and writes its pairs there.  Column lists longer than half the table take
+// classify_all_pairs.  Dense constant basis, 8192 triangles: walking the vertices' lists and forming
+// the codes per tile, one thread per row triangle, 181 + 355 us for the two passes; from the neighbour lists
+// 74 + 149.
 constexpr int CL_HASH = 1024;  // slots, a power of two
 __device__ __forceinline__ uint32_t cl_slot(uint32_t t) { return (t * 2654435761u) >> 22; }
 
 template <bool WRITE>
 __global__ void __launch_bounds__(256) classify_kernel(const TriRec *tri, const TriRef *refs,
                                                        const h2b_tile *tiles,
-                                                       const uint32_t *vt_off,
-                                                       const uint32_t *vt_tri, uint32_t *cursor,
-                                                       const uint32_t *base, h2b_sing *out) {
+                                                       const uint32_t *nb_off,
+                                                       const uint32_t *nb_len, const uint2 *nb,
+                                                       uint32_t *cursor, const uint32_t *counts,
+                                                       h2b_sing *out) {
   __shared__ uint32_t hkey[CL_HASH];
   __shared__ uint32_t hval[CL_HASH];
-  __shared__ uint32_t cnt[4], cur[4], rsv[4];
+  __shared__ uint32_t cnt[4], cur[4], rsv[4], base[4];
+  if (WRITE && threadIdx.x == 0) {
+    base[1] = 0;
+    base[2] = counts[1];
+    base[3] = counts[1] + counts[2];
+  }
   const h2b_tile tl = tiles[blockIdx.x];
   const uint32_t ntr = tl.tr_len, nsc = tl.sc_len;
-  if (nsc > (uint32_t) CL_HASH / 2) {
+  if (!nb || nsc > (uint32_t) CL_HASH / 2) {
     classify_all_pairs<WRITE>(tri, refs, tl, cursor, base, out);
     return;
   }
-  for (uint32_t e = threadIdx.x; e < (uint32_t) CL_HASH; e += blockDim.x) hkey[e] = UINT32_MAX;
+  // a table of at least twice the list's length
+  uint32_t mask = 63u;
+  while (mask + 1u < 2u * nsc) mask = 2u * mask + 1u;
+  for (uint32_t e = threadIdx.x; e <= mask; e += blockDim.x) hkey[e] = UINT32_MAX;
   if (threadIdx.x < 4) cnt[threadIdx.x] = cur[threadIdx.x] = 0;
   __syncthreads();
   for (uint32_t e = threadIdx.x; e < nsc; e += blockDim.x) {
     const uint32_t t = refs[tl.sc_off + e].t;
-    uint32_t h = cl_slot(t);
-    while (atomicCAS(&hkey[h], UINT32_MAX, t) != UINT32_MAX) h = (h + 1) & (CL_HASH - 1);
+    uint32_t h = cl_slot(t) & mask;
+    while (atomicCAS(&hkey[h], UINT32_MAX, t) != UINT32_MAX) h = (h + 1) & mask;
     hval[h] = e;
   }
   __syncthreads();
+  const uint32_t sub = threadIdx.x & 7u, lane = threadIdx.x & 31u;
   // pass 0 counts the tile's pairs per case; pass 1 (write pass only) writes them
   for (int pass = 0; pass < (WRITE ? 2 : 1); pass++) {
-    for (uint32_t i = threadIdx.x; i < ntr; i += blockDim.x) {
-      const uint32_t t = refs[tl.tr_off + i].t;
-      const uint32_t tv[3] = {tri[t].v[0], tri[t].v[1], tri[t].v[2]};
+    for (uint32_t i0 = 0; i0 < ntr; i0 += 32) {
+      const uint32_t i = i0 + threadIdx.x / 8;
+      uint32_t o = 0, n = 0;
+      if (i < ntr) {
+        const uint32_t t = refs[tl.tr_off + i].t;
+        o = nb_off[t];
+        n = nb_len[t];
+      }
+      const uint32_t most = __reduce_max_sync(0xffffffffu, n);
+      for (uint32_t a = 0; a < most; a += 8) {
+        uint32_t c = 0, code = 0, at = 0;
+        if (a + sub < n) {
+          const uint2 e = nb[o + a + sub];
+          uint32_t h = cl_slot(e.x) & mask;
+          while (hkey[h] != e.x && hkey[h] != UINT32_MAX) h = (h + 1) & mask;
+          if (hkey[h] == e.x) {
+            code = e.y;
+            c = code & 3u;
+            at = hval[h];
+          }
+        }
 #pragma unroll
-      for (int k = 0; k < 3; k++) {
-        for (uint32_t a = vt_off[tv[k]]; a < vt_off[tv[k] + 1]; a++) {
-          const uint32_t s = vt_tri[a];
-          const uint32_t sv[3] = {tri[s].v[0], tri[s].v[1], tri[s].v[2]};
-          bool seen = false;
-#pragma unroll
-          for (int k2 = 0; k2 < k; k2++) seen |= sv[0] == tv[k2] || sv[1] == tv[k2] || sv[2] == tv[k2];
-          if (seen) continue;
-          uint32_t h = cl_slot(s);
-          while (hkey[h] != s && hkey[h] != UINT32_MAX) h = (h + 1) & (CL_HASH - 1);
-          if (hkey[h] != s) continue;
-          const uint32_t code = pair_code_dev(tv, sv), c = code & 3u;
-          if (pass == 0) {
-            atomicAdd(&cnt[c], 1u);
-          } else {
+        for (uint32_t q = 1; q <= 3; q++) {
+          const unsigned m = __ballot_sync(0xffffffffu, c == q);
+          if (m == 0) continue;
+          const uint32_t leader = __ffs(m) - 1;
+          uint32_t b = 0;
+          if (lane == leader) b = atomicAdd(pass == 0 ? &cnt[q] : &cur[q], (uint32_t) __popc(m));
+          if (pass == 0) continue;
+          b = __shfl_sync(0xffffffffu, b, leader);
+          if (WRITE && c == q) {
             h2b_sing sg;
             sg.tile = blockIdx.x;
             sg.tr = tl.tr_off + i;
-            sg.sc = tl.sc_off + hval[h];
+            sg.sc = tl.sc_off + at;
             sg.code = code;
-            out[base[c] + rsv[c] + atomicAdd(&cur[c], 1u)] = sg;
+            out[base[q] + rsv[q] + b + __popc(m & ((1u << lane) - 1u))] = sg;
           }
         }
       }
@@ -1952,20 +2014,65 @@ __global__ void __launch_bounds__(256) classify_kernel(const TriRec *tri, const 
   }
 }
 
+__global__ void grid_tiles_kernel(const uint32_t *lists, uint32_t nr, uint32_t nc, uint32_t rows,
+                                  uint32_t cols, uint32_t tile, uint32_t ld, int ntrans,
+                                  h2b_tile *tiles, uint32_t *half) {
+  const uint64_t a = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x;
+  if (a >= (uint64_t) nr * nc) return;
+  const uint32_t j = (uint32_t) (a / nr), i = (uint32_t) (a - (uint64_t) j * nr);
+  const uint32_t *coff = lists + 2 * nr;
+  h2b_tile t;
+  t.tr_off = lists[i];
+  t.tr_len = lists[nr + i];
+  t.sc_off = coff[j];
+  t.sc_len = coff[nc + j];
+  const uint32_t r0 = i * tile, c0 = j * tile;
+  t.out_off = ntrans ? c0 + (uint64_t) r0 * ld : r0 + (uint64_t) c0 * ld;
+  t.ld = ld;
+  t.rows = (uint16_t) min(tile, rows - r0);
+  t.cols = (uint16_t) min(tile, cols - c0);
+  t.flags = ntrans ? 1u : 0u;
+  t.mate = half && i != j ? j + i * nr + 1u : 0u;
+  tiles[a] = t;
+  if (half && i >= j)
+    half[(uint64_t) j * nr - (uint64_t) j * (j - 1ull) / 2 + (i - j)] = (uint32_t) a;
+}
+
 }  // namespace
 
+extern "C" int h2b_near_neighbours(const void *tri, uint32_t nt, const uint32_t *vt_off,
+                                   const uint32_t *vt_tri, uint32_t *cursor, uint32_t *off,
+                                   uint32_t *len, uint2 *nb, cudaStream_t st) {
+  neighbours_kernel<<<(nt + 127) / 128, 128, 0, st>>>((const TriRec *) tri, nt, vt_off, vt_tri,
+                                                      cursor, off, len, nb);
+  h2b_note_launch();
+  H2B_CUDA_TRY(cudaGetLastError());
+  return H2B_OK;
+}
+
 extern "C" int h2b_near_classify(const void *tri, const void *refs, const h2b_tile *tiles,
-                                 uint32_t ntiles, const uint32_t *vt_off, const uint32_t *vt_tri,
-                                 uint32_t *cursor, const uint32_t *base, h2b_sing *sing,
-                                 cudaStream_t st) {
+                                 uint32_t ntiles, const uint32_t *nb_off, const uint32_t *nb_len,
+                                 const uint2 *nb, uint32_t *cursor, const uint32_t *counts,
+                                 h2b_sing *sing, cudaStream_t st) {
   if (ntiles == 0) return H2B_OK;
   if (sing)
     classify_kernel<true><<<ntiles, 256, 0, st>>>((const TriRec *) tri, (const TriRef *) refs,
-                                                  tiles, vt_off, vt_tri, cursor, base, sing);
+                                                  tiles, nb_off, nb_len, nb, cursor, counts, sing);
   else
     classify_kernel<false><<<ntiles, 256, 0, st>>>((const TriRec *) tri, (const TriRef *) refs,
-                                                   tiles, vt_off, vt_tri, cursor, nullptr,
+                                                   tiles, nb_off, nb_len, nb, cursor, nullptr,
                                                    nullptr);
+  h2b_note_launch();
+  H2B_CUDA_TRY(cudaGetLastError());
+  return H2B_OK;
+}
+
+extern "C" int h2b_near_grid_tiles(const uint32_t *lists, uint32_t nr, uint32_t nc, uint32_t rows,
+                                   uint32_t cols, uint32_t tile, uint32_t ld, int ntrans,
+                                   h2b_tile *tiles, uint32_t *half, cudaStream_t st) {
+  const uint64_t n = (uint64_t) nr * nc;
+  grid_tiles_kernel<<<(uint32_t) ((n + 127) / 128), 128, 0, st>>>(lists, nr, nc, rows, cols, tile,
+                                                                  ld, ntrans, tiles, half);
   h2b_note_launch();
   H2B_CUDA_TRY(cudaGetLastError());
   return H2B_OK;

@@ -52,14 +52,27 @@ typedef struct {
 int h2b_near_upload_dist_rules(void);
 /* The QuadRec of every triangle (after h2b_near_upload_dist_rules). */
 int h2b_near_quad_records(const void *tri, uint32_t nt, void *qrec, cudaStream_t st);
-/* Singular pairs of a tile list on the device (the pairs that share a vertex, with the vertex
- * permutation code of h2b_pair_code).  vt_off / vt_tri: the surface's vertex -> triangle lists
- * (CSR).  sing == NULL: add the number of pairs of each case c to cursor[c] (c = 1 vertex,
- * 2 edge, 3 identical).  Otherwise write the pairs of case c to sing[base[c] + cursor[c]++]
- * (cursor zeroed by the caller); the order inside a case is not fixed. */
+/* The triangles around each triangle (those that share a vertex with it, itself included), with the
+ * vertex permutation code of h2b_pair_code: triangle t's are (id, code) at nb[off[t]] ..
+ * nb[off[t] + len[t]).  vt_off / vt_tri: the surface's vertex -> triangle lists (CSR); cursor: a
+ * device counter set to 0; nb: room for the sum over the vertices of their squared triangle counts. */
+int h2b_near_neighbours(const void *tri, uint32_t nt, const uint32_t *vt_off, const uint32_t *vt_tri,
+                        uint32_t *cursor, uint32_t *off, uint32_t *len, uint2 *nb, cudaStream_t st);
+/* Singular pairs of a tile list on the device (the pairs that share a vertex).  nb_off, nb_len, nb:
+ * h2b_near_neighbours (NULL: every pair of a tile is tested).  sing == NULL: add the number of pairs
+ * of each case c to cursor[c] (c = 1 vertex, 2 edge, 3 identical).  Otherwise write the pairs of case
+ * c to sing[base[c] + cursor[c]++] (cursor zeroed by the caller); the order inside a case is not
+ * fixed. */
 int h2b_near_classify(const void *tri, const void *refs, const h2b_tile *tiles, uint32_t ntiles,
-                      const uint32_t *vt_off, const uint32_t *vt_tri, uint32_t *cursor,
-                      const uint32_t *base, h2b_sing *sing, cudaStream_t st);
+                      const uint32_t *nb_off, const uint32_t *nb_len, const uint2 *nb,
+                      uint32_t *cursor, const uint32_t *counts, h2b_sing *sing, cudaStream_t st);
+/* The tiles of one block cut into nr x nc tiles of `tile` rows and columns, tile (i, j) at i + j nr;
+ * lists: row list offsets (nr) and lengths (nr), column list offsets (nc) and lengths (nc) in the
+ * TriRef pool.  half != NULL (equal row and column lists): tiles (i, j) and (j, i) are mates, and half
+ * receives the nr (nr + 1) / 2 tiles with i >= j. */
+int h2b_near_grid_tiles(const uint32_t *lists, uint32_t nr, uint32_t nc, uint32_t rows, uint32_t cols,
+                        uint32_t tile, uint32_t ld, int ntrans, h2b_tile *tiles, uint32_t *half,
+                        cudaStream_t st);
 int h2b_near_launch_kernels(const h2b_near_launch *L, cudaStream_t st);
 /* Distinct triangle pairs of a tile list, by vertices shared (counts[0] distant, [1] common
  * vertex, [2] common edge, [3] identical), from a bitmap of nt^2 bits in device memory (freed
