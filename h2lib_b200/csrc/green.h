@@ -64,8 +64,10 @@ struct GreenCouplingArgs {
   uint32_t n;
   int K, q, rlinear, clinear, dlp;
   double kconst;
-  uint32_t max_elems;  // bound on a block's column triangles over its pivots (K x the largest
+  uint32_t max_elems;  // bound on a block's triangles over its column pivots (K x the largest
                        // vertex degree, or K for constant bases)
+  uint32_t max_rows;   // the same over its row pivots
+  const QuadRec *qrec; // points of the order-2 rule
 };
 
 extern "C" {

@@ -2211,10 +2211,15 @@ __global__ void __launch_bounds__(256) green_coupling_kernel(GreenCouplingArgs a
   }
 }
 
-// The same entries with the column triangles staged once per block: for every pivot column its
-// triangles' four rule points, their weights times the basis function, Gram determinant and
-// 1/(4 pi), and the normal (q = 2).  A thread then reads its column's triangles from shared
-// memory instead of forming their points once per row triangle.
+// The same entries for q = 2.  The triangles of the block's pivot rows and columns are staged once: per
+// column triangle the four points, their weights times the basis function, Gram determinant and
+// 1/(4 pi), and the normal; per row triangle its id and corner.  A unit of work is (row triangle,
+// pivot column), its sum over the column's triangles; the row triangles of a pivot are added up in
+// order afterwards.  Only entries inside the ranks are units (a mean rank of 11 of K = 48 leaves 5 % of
+// the padded block), and about 64 row triangles times 11 columns keep the CTA's lanes busy, where a
+// thread per padded entry had a fifth of a warp's lanes at work.  The partial sums of GCW words at most
+// are kept, columns in groups.  16200 triangles, K = 48: 1106 -> 425 us.
+constexpr uint32_t GCW = 1024;
 template <bool RL, bool CL, bool DLP>
 __global__ void __launch_bounds__(256) green_coupling_staged_kernel(GreenCouplingArgs a) {
   extern __shared__ __align__(16) unsigned char gsm[];
@@ -2225,92 +2230,124 @@ __global__ void __launch_bounds__(256) green_coupling_staged_kernel(GreenCouplin
   const uint32_t *pr = a.rpiv + (size_t) rc * K, *pc = a.cpiv + (size_t) cc * K;
   double *S = a.S + (size_t) b * K * K;
   const double(&sd)[6][SIDE_MAXP] = c_side[1];
-  uint32_t *coff = reinterpret_cast<uint32_t *>(gsm);           // K + 1 (padded to 16 bytes)
-  double *cy = reinterpret_cast<double *>(gsm + 16 * ((4 * (K + 1) + 15) / 16));
-  const uint32_t emax = (uint32_t) a.max_elems;
-  double *cw = cy + (size_t) emax * 3 * P;                        // emax x P weights
-  double *cn = cw + (size_t) emax * P;                            // emax x 3 normals
-  if (threadIdx.x == 0) {
+  const uint32_t emax = a.max_elems;
+  double *cy = reinterpret_cast<double *>(gsm);      // emax x P x 3 points
+  double *cw = cy + (size_t) emax * 3 * P;           // emax x P weights
+  double *cn = cw + (size_t) emax * P;               // emax x 3 normals
+  double *part = cn + (size_t) emax * 3;             // GCW partial sums
+  uint32_t *coff = reinterpret_cast<uint32_t *>(part + GCW);  // K + 1
+  uint32_t *roff = coff + K + 1;                     // K + 1
+  uint32_t *rt = roff + K + 1;                       // rmax: triangle times four plus corner
+  if (threadIdx.x < 64) {
+    // offsets of the pivots' triangles (warp 0: columns, warp 1: rows)
+    const bool row = threadIdx.x >= 32;
+    const uint32_t lane = threadIdx.x & 31u, n = row ? kr : kc;
+    const bool lin = row ? RL : CL;
+    uint32_t *off = row ? roff : coff;
     uint32_t o = 0;
-    for (uint32_t j = 0; j < kc; j++) {
-      coff[j] = o;
-      o += CL ? a.vt_off[pc[j] + 1] - a.vt_off[pc[j]] : 1u;
+    for (uint32_t j0 = 0; j0 < n; j0 += 32) {
+      const uint32_t j = j0 + lane;
+      uint32_t d = 0;
+      if (j < n) {
+        const uint32_t bj = row ? pr[j] : pc[j];
+        d = lin ? a.vt_off[bj + 1] - a.vt_off[bj] : 1u;
+      }
+      uint32_t s = d;
+#pragma unroll
+      for (int sh = 1; sh < 32; sh <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, s, sh);
+        if (lane >= (uint32_t) sh) s += v;
+      }
+      if (j < n) off[j] = o + s - d;
+      o += __shfl_sync(0xffffffffu, s, 31);
     }
-    coff[kc] = o;
+    if (lane == 0) off[n] = o;
   }
+  // entries past the ranks
+  for (uint32_t e = threadIdx.x; e < K * K; e += blockDim.x)
+    if (e % K >= kr || e / K >= kc) S[e] = 0.0;
   __syncthreads();
   for (uint32_t j = threadIdx.x; j < kc; j += blockDim.x) {
-    const uint32_t bj = pc[j];
-    const uint32_t u0 = CL ? a.vt_off[bj] : 0u, u1 = CL ? a.vt_off[bj + 1] : 1u;
-    for (uint32_t u = u0; u < u1; u++) {
-      const uint32_t f = coff[j] + (u - u0);
-      const TriRec &Sx = a.tri[CL ? a.vt_tri[u] : bj];
-      const int cs = CL ? (Sx.v[0] == bj ? 0 : (Sx.v[1] == bj ? 1 : 2)) : 0;
-      const double gk = Sx.g * a.kconst;
+    const uint32_t bj = pc[j], u0 = CL ? a.vt_off[bj] : 0u, n = coff[j + 1] - coff[j];
+    for (uint32_t u = 0; u < n; u++) {
+      const uint32_t f = coff[j] + u;
+      const QuadRec &Q = a.qrec[CL ? a.vt_tri[u0 + u] : bj];
+      const int cs = CL ? (Q.v[0] == bj ? 0 : (Q.v[1] == bj ? 1 : 2)) : 0;
+      const double gk = Q.g * a.kconst;
       for (int p = 0; p < P; p++) {
-        const double ty = sd[0][p], sy = sd[1][p];
-        const double ay = 1.0 - ty, by = ty - sy, cy_ = sy;
-        for (int d = 0; d < 3; d++)
-          cy[((size_t) f * P + p) * 3 + d] = Sx.a[d] * ay + Sx.b[d] * by + Sx.c[d] * cy_;
+        for (int d = 0; d < 3; d++) cy[((size_t) f * P + p) * 3 + d] = Q.p[p][d];
         cw[(size_t) f * P + p] = (CL ? sd[3 + cs][p] : sd[2][p]) * gk;
       }
-      for (int d = 0; d < 3; d++) cn[(size_t) f * 3 + d] = Sx.n[d];
+      for (int d = 0; d < 3; d++) cn[(size_t) f * 3 + d] = Q.n[d];
+    }
+  }
+  for (uint32_t i = threadIdx.x; i < kr; i += blockDim.x) {
+    const uint32_t bi = pr[i], u0 = RL ? a.vt_off[bi] : 0u, n = roff[i + 1] - roff[i];
+    for (uint32_t u = 0; u < n; u++) {
+      const uint32_t t = RL ? a.vt_tri[u0 + u] : bi;
+      const QuadRec &Q = a.qrec[t];
+      rt[roff[i] + u] = 4u * t + (RL ? (Q.v[0] == bi ? 0u : (Q.v[1] == bi ? 1u : 2u)) : 3u);
     }
   }
   __syncthreads();
-  for (uint32_t e = threadIdx.x; e < K * K; e += blockDim.x) {
-    const uint32_t i = e % K, j = e / K;
-    double acc = 0.0;
-    if (i < kr && j < kc) {
-      const uint32_t bi = pr[i];
-      const uint32_t t0 = RL ? a.vt_off[bi] : 0u, t1 = RL ? a.vt_off[bi + 1] : 1u;
-      const uint32_t f0 = coff[j], f1 = coff[j + 1];
-      for (uint32_t ti = t0; ti < t1; ti++) {
-        const TriRec &T = a.tri[RL ? a.vt_tri[ti] : bi];
-        const int ct = RL ? (T.v[0] == bi ? 0 : (T.v[1] == bi ? 1 : 2)) : 0;
-        double xa[P][3], wa[P];
+  const uint32_t nR = roff[kr], jc = max(1u, GCW / max(1u, nR));  // columns per group
+  for (uint32_t j0 = 0; j0 < kc; j0 += jc) {
+    const uint32_t nj = min(jc, kc - j0);
+    for (uint32_t e = threadIdx.x; e < nR * nj; e += blockDim.x) {
+      const uint32_t jj = e / nR, fr = e - jj * nR;
+      const uint32_t code = rt[fr], ct = code & 3u;
+      const QuadRec &T = a.qrec[code >> 2];
+      double xa[P][3], wa[P];
+#pragma unroll
+      for (int p = 0; p < P; p++) {
+#pragma unroll
+        for (int d = 0; d < 3; d++) xa[p][d] = T.p[p][d];
+        wa[p] = (RL ? sd[3 + ct][p] : sd[2][p]) * T.g;
+      }
+      const uint32_t f0 = coff[j0 + jj], f1 = coff[j0 + jj + 1];
+      double sum = 0.0;
+      for (uint32_t f = f0; f < f1; f++) {
+        const double *y = cy + (size_t) f * P * 3, *w = cw + (size_t) f * P;
+        double n0 = 0.0, n1 = 0.0, n2 = 0.0;
+        if (DLP) n0 = cn[3 * (size_t) f], n1 = cn[3 * (size_t) f + 1], n2 = cn[3 * (size_t) f + 2];
 #pragma unroll
         for (int p = 0; p < P; p++) {
-          const double tx = sd[0][p], sx = sd[1][p];
-          const double ax = 1.0 - tx, bx = tx - sx, cx = sx;
+          const double y0 = y[3 * p], y1 = y[3 * p + 1], y2 = y[3 * p + 2];
+          double pb = 0.0;
 #pragma unroll
-          for (int d = 0; d < 3; d++) xa[p][d] = T.a[d] * ax + T.b[d] * bx + T.c[d] * cx;
-          wa[p] = RL ? sd[3 + ct][p] : sd[2][p];
-        }
-        double part = 0.0;
-        for (uint32_t f = f0; f < f1; f++) {
-          const double *y = cy + (size_t) f * P * 3, *w = cw + (size_t) f * P;
-          const double n0 = cn[3 * (size_t) f], n1 = cn[3 * (size_t) f + 1],
-                       n2 = cn[3 * (size_t) f + 2];
-#pragma unroll
-          for (int p = 0; p < P; p++) {
-            const double y0 = y[3 * p], y1 = y[3 * p + 1], y2 = y[3 * p + 2];
-            double pb = 0.0;
-#pragma unroll
-            for (int r = 0; r < P; r++) {
-              const double d0 = xa[r][0] - y0, d1 = xa[r][1] - y1, d2 = xa[r][2] - y2;
-              const double ri = rsqrt_nr(fma(d0, d0, fma(d1, d1, d2 * d2)));
-              const double fv = DLP ? fma(d0, n0, fma(d1, n1, d2 * n2)) * (ri * ri * ri) : ri;
-              pb = fma(wa[r], fv, pb);
-            }
-            part = fma(w[p], pb, part);
+          for (int r = 0; r < P; r++) {
+            const double d0 = xa[r][0] - y0, d1 = xa[r][1] - y1, d2 = xa[r][2] - y2;
+            const double ri = rsqrt_nr(fma(d0, d0, fma(d1, d1, d2 * d2)));
+            const double fv = DLP ? fma(d0, n0, fma(d1, n1, d2 * n2)) * (ri * ri * ri) : ri;
+            pb = fma(wa[r], fv, pb);
           }
+          sum = fma(w[p], pb, sum);
         }
-        acc += part * T.g;
       }
+      part[e] = sum;
     }
-    S[i + (size_t) j * K] = acc;
+    __syncthreads();
+    for (uint32_t e = threadIdx.x; e < kr * nj; e += blockDim.x) {
+      const uint32_t jj = e / kr, i = e - jj * kr;
+      double s = 0.0;
+      for (uint32_t f = roff[i]; f < roff[i + 1]; f++) s += part[jj * nR + f];
+      S[i + (size_t) (j0 + jj) * K] = s;
+    }
+    __syncthreads();
   }
 }
 
-size_t green_coupling_smem(int K, uint32_t max_elems) {
-  return 16 * ((4 * ((size_t) K + 1) + 15) / 16) + sizeof(double) * (size_t) max_elems * (12 + 4 + 3);
+size_t green_coupling_smem(const GreenCouplingArgs *a) {
+  return sizeof(double) * ((size_t) a->max_elems * (12 + 4 + 3) + GCW) +
+         sizeof(uint32_t) * (2 * ((size_t) a->K + 1) + a->max_rows);
 }
 
+// The staged kernel where a group holds at least one column (row pivots with at most GCW triangles) and
+// its stage fits; usual meshes have about 290 triangles over 48 pivots.
 template <bool RL, bool CL, bool DLP>
 static int launch_green_coupling(const GreenCouplingArgs *a, cudaStream_t st) {
-  const size_t smem = green_coupling_smem(a->K, a->max_elems);
-  if (a->q == 2 && smem <= H2B_MAX_DYN_SMEM) {
+  const size_t smem = green_coupling_smem(a);
+  if (a->q == 2 && smem <= H2B_MAX_DYN_SMEM && a->max_rows <= GCW) {
     H2B_CUDA_TRY((h2b_allow_smem<green_coupling_staged_kernel<RL, CL, DLP>>()));
     green_coupling_staged_kernel<RL, CL, DLP><<<a->n, 256, smem, st>>>(*a);
   } else if (a->q == 2) {
