@@ -133,7 +133,7 @@ extern "C" int h2b_solve_gmres_noalloc(uint32_t nterms, const h2b_h2matrix *cons
   H2B_CUDA_TRY(cudaMemcpyAsync(dx, x, sizeof(double) * W * n, cudaMemcpyDefault, st));
 
   // host-driven loop: one step launch sequence per iteration, the residual estimate read back
-  GmresOp op{&combo, combo_apply_na, nullptr};
+  GmresOp op{&combo, combo_apply_na, nullptr, nullptr};
   GmresState hs;
   auto read_state = [&]() -> int {
     H2B_CUDA_TRY(cudaMemcpyAsync(&hs, g.state, sizeof(GmresState), cudaMemcpyDeviceToHost, st));

@@ -210,7 +210,10 @@ static int solve_segments(Combo &combo, uint32_t nseg, const uint32_t *seg_off, 
   combo.work = (double *) work.p;
   combo.mask = forest ? g.mask : nullptr;
   combo.nseg = nseg;
-  GmresOp op{(void *) &combo, combo_apply, mixed ? combo_apply_single : nullptr};
+  // the products of (re)starts take only the systems that restart
+  Combo rcombo = combo;
+  if (forest) rcombo.mask = g.rmask;
+  GmresOp op{(void *) &combo, combo_apply, mixed ? combo_apply_single : nullptr, (void *) &rcombo};
   std::vector<GmresState> hs(nsys);
   int rc = h2b_gmres_run(&g, &op, db, dx, maxiter, st, hs.data());
   if (rc != H2B_OK) return rc;

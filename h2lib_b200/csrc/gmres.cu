@@ -750,7 +750,7 @@ int init_impl(const GmresDev &g, const GmresOp &op, const double *b, double *x, 
   const uint32_t nb = g.nblocks;
   // qr[:,0] = b - A x
   zero_abuf_kernel<CX><<<nb, TPB, 0, st>>>(g);
-  int rc = op.apply(op.ctx, x, g.abuf, 1.0, 0.0, st);
+  int rc = op.apply(op.rctx ? op.rctx : op.ctx, x, g.abuf, 1.0, 0.0, st);
   if (rc != H2B_OK) return rc;
   init0_kernel<CX><<<nb, TPB, 0, st>>>(g, b, sel);
   small_kernel<CX><<<g.nsys, SMALL_THREADS, 0, st>>>(g, 4, sel);
@@ -814,6 +814,7 @@ __global__ void decide_kernel(GmresDev g, cudaGraphConditionalHandle hi) {
   for (uint32_t s = threadIdx.x; s < g.nsys; s += blockDim.x) {
     GmresState *y = g.state + s;
     y->restart = (y->active && (y->k + 1 >= g.kmax || y->verify)) ? 1u : 0u;
+    g.rmask[s] = y->restart;
     if (y->restart) any = 1;
   }
   __syncthreads();
@@ -887,7 +888,8 @@ size_t h2b_gmres_workspace(int cx, uint32_t nsys, const uint32_t *sizes, uint32_
          + 2 * W * n                         // q, abuf
          + 2 * nb * ld                       // part
          + (sizeof(GmresState) * nsys + sizeof(GmresCtl) + sizeof(GmresSys) * nsys +
-            sizeof(uint32_t) * (nb + nsys)) / sizeof(double) + 64;
+            sizeof(uint32_t) * (nb + nsys + (nsys > 1 ? nsys : 0))) / sizeof(double)
+         + 64;  // alignment, and the second mask of a single system
 }
 
 void h2b_gmres_layout(GmresDev *g, double *p, int cx, uint32_t nsys, const uint32_t *sizes,
@@ -929,6 +931,7 @@ void h2b_gmres_layout(GmresDev *g, double *p, int cx, uint32_t nsys, const uint3
   g->sys = (const GmresSys *) c; c += sizeof(GmresSys) * nsys;
   g->blk = (const uint32_t *) c;
   g->mask = (uint32_t *) c + nb;
+  g->rmask = g->mask + nsys;
 }
 
 extern "C" int h2b_gmres_step(const GmresDev *g, const GmresOp *op, cudaStream_t st) {
@@ -1022,7 +1025,7 @@ extern "C" int h2b_gmres_run(const GmresDev *g, const GmresOp *op, const double 
   } ef{exec};
   H2B_CUDA_TRY(cudaMemsetAsync(g->state, 0, sizeof(GmresState) * g->nsys, st));
   // the first residual needs every system's product
-  H2B_CUDA_TRY(cudaMemsetAsync(g->mask, 1, sizeof(uint32_t) * g->nsys, st));
+  H2B_CUDA_TRY(cudaMemsetAsync(g->mask, 1, sizeof(uint32_t) * g->nsys * 2, st));  // and rmask
   H2B_CUDA_TRY(cudaMemsetAsync(g->T, 0, sizeof(double) * 2 * (size_t) g->nsys * g->kmax * g->kmax, st));
   if ((rc = h2b_gmres_bnorm(g, b, st)) != H2B_OK) return rc;
   if ((rc = h2b_gmres_init(g, op, b, x, GMRES_SEL_ALL, st)) != H2B_OK) return rc;

@@ -56,15 +56,18 @@ struct GmresDev {
   GmresState *state;         // nsys
   GmresCtl *ctl;
   uint32_t *mask;            // nsys: 1 while the system is active (read by a masked operator)
+  uint32_t *rmask;           // nsys: 1 where the current iteration restarts the system
 };
 
 // y += alpha * A x on stream st (x, y: the global vectors).  apply_lo (optional) is a cheaper,
 // less accurate application used for the Arnoldi steps of a mixed-precision solve; residuals at
-// (re)starts always use apply.
+// (re)starts always use apply, with rctx where it is given (an operator masked by rmask: only the
+// systems that restart).
 struct GmresOp {
   void *ctx;
   int (*apply)(void *ctx, const double *x, double *y, double ar, double ai, cudaStream_t st);
   int (*apply_lo)(void *ctx, const double *x, double *y, double ar, double ai, cudaStream_t st);
+  void *rctx;
 };
 
 // Doubles of device work space for nsys systems of total size n (without b and x), and the
