@@ -87,20 +87,25 @@ __global__ void __launch_bounds__(128) flatten_paths_kernel(FlatArgs a) {
 // is multiplied one axis at a time:
 //   t1[a][b][jz] = sum_c w[a][b][c] Pz[c][jz],  t2[a][jy][jz] = sum_b t1[a][b][jz] Py[b][jy],
 //   W_f[jx][jy][jz] = sum_a t2[a][jy][jz] Px[a][jx]
-// -- 3 m^4 multiply-adds per row instead of the k^2 = m^6 of the full product.  The rows are
-// staged in shared memory in chunks of RB; a thread takes one fibre of m inputs and writes its m
-// outputs, so every input is read once per step.
+// -- 3 m^4 multiply-adds per row instead of the k^2 = m^6 of the full product.  A thread takes one
+// fibre of m inputs, the first time from memory, and writes its m outputs to the inputs' places in
+// shared memory, so every input is read once per step and one buffer of RB rows is enough.  What
+// bounds it is the wait for the rows and between the steps, so the CTAs are small and many
+// (FLAT_CTAS of 128 threads with 80 registers per SM; 64 registers spill the 25 factors of m = 5).
+// A basis of 49152 triangles, m = 5: 249 us with 256 threads, rows staged first and two buffers; in
+// place 201, with 128 threads 150; rows read by the first step 132.  32768 triangles, m = 4: 31 -> 24.
 template <int M>
 struct FlatShape {
   static constexpr int K = M * M * M;
-  // rows per chunk: two K-double buffers per row within 96 KiB (at most H2B_FLAT_ROWS)
-  static constexpr int RB = (96 * 1024) / (16 * K) < H2B_FLAT_ROWS ? (96 * 1024) / (16 * K)
-                                                                   : H2B_FLAT_ROWS;
+  // rows per chunk: K doubles per row within 48 KiB (at most H2B_FLAT_ROWS)
+  static constexpr int RB = (48 * 1024) / (8 * K) < H2B_FLAT_ROWS ? (48 * 1024) / (8 * K)
+                                                                  : H2B_FLAT_ROWS;
   static_assert(RB >= 1, "rank too large for the staged flatten");
 };
 
+constexpr int FLAT_CTAS = 6, FLAT_ROW_THREADS = 128;
 template <int M>
-__global__ void __launch_bounds__(FLAT_TPB) flatten_rows_kernel(FlatArgs a) {
+__global__ void __launch_bounds__(FLAT_ROW_THREADS, FLAT_CTAS) flatten_rows_kernel(FlatArgs a) {
   constexpr int K = FlatShape<M>::K, RB = FlatShape<M>::RB, MM = M * M;
   extern __shared__ double sm[];
   __shared__ double L[3][M][M];  // the pair's three transfer products
@@ -109,34 +114,32 @@ __global__ void __launch_bounds__(FLAT_TPB) flatten_rows_kernel(FlatArgs a) {
   const uint32_t l = a.pairs[2 * (size_t) pid], f = a.pairs[2 * (size_t) pid + 1];
   for (int e = (int) threadIdx.x; e < 3 * MM; e += (int) blockDim.x)
     (&L[0][0][0])[e] = a.P[(size_t) pid * 3 * MM + e];
-  double *A = sm, *B = sm + (size_t) RB * K;
+  double *A = sm;
   const uint32_t rf = a.off[l] - a.off[f] + r0;  // first row inside f
   const double *Ws = a.W + a.woff[l] + (size_t) r0 * K;
   double *Wf = a.W + a.woff[f] + (size_t) rf * K;
   for (uint32_t c0 = 0; c0 < nr; c0 += RB) {
     const uint32_t nc = min((uint32_t) RB, nr - c0);
     __syncthreads();  // L is ready; the previous chunk's last step has read A
-    // W_l^T rows are contiguous (ld K)
-    for (uint32_t e = threadIdx.x; e < nc * K; e += blockDim.x) A[e] = Ws[(size_t) c0 * K + e];
-    __syncthreads();
-    // z: fibre g = (row, a, b) of A -> B[row][a][b][jz]
-    for (uint32_t g = threadIdx.x; g < nc * MM; g += blockDim.x) {
+    const double *Z = Ws + (size_t) c0 * K;  // W_l^T rows are contiguous (ld K)
+    // z: fibre g = (row, a, b) of W_l -> A[row][a][b][jz]
+    for (uint32_t g = threadIdx.x; g < nc * MM; g += FLAT_ROW_THREADS) {
       double in[M];
 #pragma unroll
-      for (int c = 0; c < M; c++) in[c] = A[(size_t) g * M + c];
+      for (int c = 0; c < M; c++) in[c] = Z[(size_t) g * M + c];
 #pragma unroll
       for (int jz = 0; jz < M; jz++) {
         double acc = 0.0;
 #pragma unroll
         for (int c = 0; c < M; c++) acc = fma(in[c], L[2][c][jz], acc);
-        B[(size_t) g * M + jz] = acc;
+        A[(size_t) g * M + jz] = acc;
       }
     }
     __syncthreads();
-    // y: fibre g = (row, a, jz) of B (stride M) -> A[row][a][jy][jz]
-    for (uint32_t g = threadIdx.x; g < nc * MM; g += blockDim.x) {
+    // y: fibre g = (row, a, jz) of A (stride M) -> A[row][a][jy][jz]
+    for (uint32_t g = threadIdx.x; g < nc * MM; g += FLAT_ROW_THREADS) {
       const uint32_t jz = g % M, ra = g / M;
-      const double *x = B + (size_t) ra * MM + jz;
+      const double *x = A + (size_t) ra * MM + jz;
       double in[M];
 #pragma unroll
       for (int b = 0; b < M; b++) in[b] = x[b * M];
@@ -151,7 +154,7 @@ __global__ void __launch_bounds__(FLAT_TPB) flatten_rows_kernel(FlatArgs a) {
     __syncthreads();
     // x: fibre g = (row, jy, jz) of A (stride M^2) -> W_f rows, consecutive threads writing
     // consecutive (jy, jz)
-    for (uint32_t g = threadIdx.x; g < nc * MM; g += blockDim.x) {
+    for (uint32_t g = threadIdx.x; g < nc * MM; g += FLAT_ROW_THREADS) {
       const uint32_t yz = g % MM, row = g / MM;
       const double *x = A + (size_t) row * K + yz;
       double in[M];
@@ -219,9 +222,9 @@ static int launch_flatten(const FlatArgs *a, int rows, cudaStream_t st) {
   if (!rows) {
     flatten_paths_kernel<M><<<a->nleaves, 128, 0, st>>>(*a);
   } else {
-    constexpr size_t smem = sizeof(double) * 2 * FlatShape<M>::RB * FlatShape<M>::K;
+    constexpr size_t smem = sizeof(double) * FlatShape<M>::RB * FlatShape<M>::K;
     H2B_CUDA_TRY(h2b_allow_smem<flatten_rows_kernel<M>>());
-    flatten_rows_kernel<M><<<a->nitems, FLAT_TPB, smem, st>>>(*a);
+    flatten_rows_kernel<M><<<a->nitems, FLAT_ROW_THREADS, smem, st>>>(*a);
   }
   h2b_note_launch();
   H2B_CUDA_TRY(cudaGetLastError());
