@@ -21,6 +21,7 @@
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
+#include <vector>
 
 #include "device_common.cuh"
 #include "gmres.h"
@@ -807,31 +808,17 @@ __global__ void precheck_kernel(GmresDev g, cudaGraphConditionalHandle hw) {
   }
 }
 
-__global__ void decide_kernel(GmresDev g, cudaGraphConditionalHandle hi) {
-  __shared__ int any;
-  if (threadIdx.x == 0) any = 0;
+// The end of a step: which systems go on, and which of those restart before the next one (their
+// restart is the IF node behind this kernel; one kernel for both: 2 us and a launch less per step).
+__global__ void control_kernel(GmresDev g, cudaGraphConditionalHandle hw,
+                               cudaGraphConditionalHandle hi) {
+  __shared__ int any, again;
+  if (threadIdx.x == 0) any = again = 0;
   __syncthreads();
   for (uint32_t s = threadIdx.x; s < g.nsys; s += blockDim.x) {
     GmresState *y = g.state + s;
-    y->restart = (y->active && (y->k + 1 >= g.kmax || y->verify)) ? 1u : 0u;
-    g.rmask[s] = y->restart;
-    if (y->restart) any = 1;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    g.ctl->any_restart = any;
-    cudaGraphSetConditional(hi, any ? 1u : 0u);
-  }
-}
-
-__global__ void control_kernel(GmresDev g, cudaGraphConditionalHandle hw) {
-  __shared__ int any;
-  if (threadIdx.x == 0) any = 0;
-  __syncthreads();
-  for (uint32_t s = threadIdx.x; s < g.nsys; s += blockDim.x) {
-    GmresState *y = g.state + s;
-    y->restart = 0;
-    if (!y->active) {  // stopped earlier, or by the FP64 residual of a restart in this step
+    y->restart = g.rmask[s] = 0;
+    if (!y->active) {  // stopped earlier, or by the FP64 residual of the restart before this step
       if (g.mask) g.mask[s] = 0;
       continue;
     }
@@ -846,12 +833,18 @@ __global__ void control_kernel(GmresDev g, cudaGraphConditionalHandle hw) {
     }
     if (g.mask) g.mask[s] = y->active;
     if (y->active) any = 1;
+    if (y->active && (y->k + 1 >= g.kmax || y->verify)) {
+      y->restart = g.rmask[s] = 1;
+      again = 1;
+    }
   }
   __syncthreads();
   if (threadIdx.x == 0) {
     g.ctl->budget--;
     g.ctl->any_active = any;
+    g.ctl->any_restart = again;
     cudaGraphSetConditional(hw, (any && g.ctl->budget > 0) ? 1u : 0u);
+    cudaGraphSetConditional(hi, again ? 1u : 0u);
   }
 }
 
@@ -968,7 +961,7 @@ extern "C" int h2b_gmres_loop_graph(const GmresDev *g, const GmresOp *op, const 
   GmresDev gv = *g;
   int rc;
   // top: precheck -> WHILE
-  cudaGraphNode_t pre, wnode, dec, inode;
+  cudaGraphNode_t pre, wnode, inode;
   if ((rc = add_ctl_node(&pre, top, nullptr, 0, (void *) precheck_kernel, &gv, &hw)) != H2B_OK)
     return rc;
   cudaGraphNodeParams wp = {};
@@ -978,32 +971,37 @@ extern "C" int h2b_gmres_loop_graph(const GmresDev *g, const GmresOp *op, const 
   wp.conditional.size = 1;
   H2B_CUDA_TRY(cudaGraphAddNode(&wnode, top, &pre, 1, &wp));
   cudaGraph_t body = wp.conditional.phGraph_out[0];
-  // body: decide -> IF(restart) -> step -> control
+  // body: step -> control -> IF(restart)
   H2B_CUDA_TRY(cudaGraphConditionalHandleCreate(&hi, body, 0, 0));
-  if ((rc = add_ctl_node(&dec, body, nullptr, 0, (void *) decide_kernel, &gv, &hi)) != H2B_OK)
-    return rc;
+  H2B_CUDA_TRY(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0,
+                                             cudaStreamCaptureModeThreadLocal));
+  rc = g->cx ? step_impl<true>(*g, *op, st) : step_impl<false>(*g, *op, st);
+  std::vector<cudaGraphNode_t> last;
+  if (rc == H2B_OK) {
+    control_kernel<<<1, CTL_THREADS, 0, st>>>(gv, hw, hi);
+    cudaStreamCaptureStatus status;
+    const cudaGraphNode_t *deps = nullptr;
+    size_t ndeps = 0;
+    if (cudaGetLastError() != cudaSuccess ||
+        cudaStreamGetCaptureInfo(st, &status, nullptr, nullptr, &deps, &ndeps) != cudaSuccess)
+      rc = H2B_ERR_CUDA;
+    else
+      last.assign(deps, deps + ndeps);
+  }
+  cudaGraph_t captured = nullptr;
+  cudaError_t ce = cudaStreamEndCapture(st, &captured);
+  if (rc != H2B_OK) return rc;
+  H2B_CUDA_TRY(ce);
   cudaGraphNodeParams ip = {};
   ip.type = cudaGraphNodeTypeConditional;
   ip.conditional.handle = hi;
   ip.conditional.type = cudaGraphCondTypeIf;
   ip.conditional.size = 1;
-  H2B_CUDA_TRY(cudaGraphAddNode(&inode, body, &dec, 1, &ip));
-  cudaGraph_t ifbody = ip.conditional.phGraph_out[0];
-  H2B_CUDA_TRY(cudaStreamBeginCaptureToGraph(st, ifbody, nullptr, nullptr, 0,
+  H2B_CUDA_TRY(cudaGraphAddNode(&inode, body, last.data(), last.size(), &ip));
+  H2B_CUDA_TRY(cudaStreamBeginCaptureToGraph(st, ip.conditional.phGraph_out[0], nullptr, nullptr, 0,
                                              cudaStreamCaptureModeThreadLocal));
   rc = g->cx ? finish_impl<true>(*g, *op, b, x, GMRES_SEL_RESTART, st)
              : finish_impl<false>(*g, *op, b, x, GMRES_SEL_RESTART, st);
-  cudaGraph_t captured = nullptr;
-  cudaError_t ce = cudaStreamEndCapture(st, &captured);
-  if (rc != H2B_OK) return rc;
-  H2B_CUDA_TRY(ce);
-  H2B_CUDA_TRY(cudaStreamBeginCaptureToGraph(st, body, &inode, nullptr, 1,
-                                             cudaStreamCaptureModeThreadLocal));
-  rc = g->cx ? step_impl<true>(*g, *op, st) : step_impl<false>(*g, *op, st);
-  if (rc == H2B_OK) {
-    control_kernel<<<1, CTL_THREADS, 0, st>>>(gv, hw);
-    if (cudaGetLastError() != cudaSuccess) rc = H2B_ERR_CUDA;
-  }
   ce = cudaStreamEndCapture(st, &captured);
   if (rc != H2B_OK) return rc;
   H2B_CUDA_TRY(ce);
