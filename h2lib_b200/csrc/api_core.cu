@@ -541,10 +541,12 @@ int h2b_check_err_flag(const h2b_bem *b, cudaStream_t st) {
 // each, measured between one and two) times the lanes a tile's triangle pairs take.  A tile side of
 // s vertices touches about 2 s + 4.3 sqrt(s) triangles (the inner ones and those along the border,
 // counted on refined spheres), rows in groups of 32 lanes, so smaller tiles evaluate border pairs more
-// often but spread a small block over the SMs; with constant bases tiles share no pairs.  FIXED is
-// the fixed cost of a tile in pairs (clearing, staging and writing it).  60 x 57 linear block: four
-// tiles of 32 take 46 us, 8 x 8 tiles 16 us.  578 x 578 complex double layer: tiles of 16 take
-// 613 us, of 32 533 us.
+// often but spread a small block over the SMs; with constant bases tiles share no pairs.  Linear
+// columns with q = 2 spread a tile over a cluster of up to eight CTAs as well (near_ring_kernel; the
+// same rule as its launch).  FIXED is the fixed cost of a tile in pairs (clearing, staging and writing
+// it).  60 x 57 linear block: four tiles of 32 take 46 us, 8 x 8 tiles 16 us, with clusters 10.
+// 578 x 578 complex double layer, us: a CTA per tile of 16 613, of 32 533 to 642; a
+// cluster per tile of 64 421.
 static uint32_t block_tile(const h2b_bem *b, uint32_t rows, uint32_t cols, bool same) {
   constexpr double FIXED = 400.0;
   const bool rl = b->row_basis == H2B_BASIS_LINEAR, cl = b->col_basis == H2B_BASIS_LINEAR;
@@ -559,8 +561,11 @@ static uint32_t block_tile(const h2b_bem *b, uint32_t rows, uint32_t cols, bool 
     if (cl) r = 32.0 * ceil(r / 32.0);
     double n = ceil((double) rows / t) * ceil((double) cols / t);
     if (same) n = 0.5 * (n + ceil((double) rows / t));
+    double work = r * tri(cols, cl);
+    if (cl && b->q == 2)
+      for (int share = 1; share < 8 && 2.0 * n <= 6.0 * b->s->num_sms; share *= 2) n *= 2, work /= 2;
     const double rounds = n / (1.5 * b->s->num_sms);
-    const double cost = (rounds > 1.0 ? rounds : 1.0) * (r * tri(cols, cl) + FIXED);
+    const double cost = (rounds > 1.0 ? rounds : 1.0) * (work + FIXED);
     if (t == H2B_TILE_MAX || cost < 0.9 * least) {
       best = t;
       least = cost;

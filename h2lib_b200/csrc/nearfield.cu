@@ -24,6 +24,7 @@
 // Library/helmholtzbem3d.c:27/140.  The quadrature point difference x - y is formed directly as
 // (A_t - A_s) + t_x (B_t - A_t) + s_x (C_t - B_t) - t_y (B_s - A_s) - s_y (C_s - B_s), which is
 // the reference's A(1-t) + B(t-s) + C s map on both triangles, without forming x and y first.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <string.h>
@@ -841,15 +842,17 @@ __device__ __forceinline__ void put_complex(double *out, uint64_t o, double re, 
 }
 
 // A finished tile: entry (r, c) from plane[r + PLD c], or plane[c + PLD r] for the mate.  im: plane of
-// the imaginary parts (complex kernels).
+// the imaginary parts (complex kernels).  Of the plane's columns only the nc from c0 on.
 template <bool CPLX, bool MATE>
 __device__ __forceinline__ void put_tile(double *out, const h2b_tile &tl, const double *re,
-                                         const double *im) {
+                                         const double *im, uint32_t c0 = 0,
+                                         uint32_t nc = H2B_TILE_MAX) {
   const uint32_t rows = tl.rows, cols = tl.cols;
   const bool ntrans = tl.flags & 1u;
   const uint32_t fast = ntrans ? cols : rows;
   for (uint32_t e = threadIdx.x; e < rows * cols; e += blockDim.x) {
     const uint32_t hi = e / fast, lo = e - hi * fast, r = ntrans ? hi : lo, c = ntrans ? lo : hi;
+    if ((MATE ? r : c) - c0 >= nc) continue;
     const uint64_t o = ntrans ? tl.out_off + c + (uint64_t) r * tl.ld
                               : tl.out_off + r + (uint64_t) c * tl.ld;
     const uint32_t p = MATE ? c + PLD * r : r + PLD * c;
@@ -860,24 +863,24 @@ __device__ __forceinline__ void put_tile(double *out, const h2b_tile &tl, const 
   }
 }
 
-// The tile's outputs from its planes, own channels first (linear bases).
+// The tile's outputs from nc columns of its planes, own channels first (linear bases).
 template <int KK, bool MIR>
 __device__ __forceinline__ void put_planes(const DistArgs &a, const h2b_tile &tl,
-                                           const double *pl) {
+                                           const double *pl, uint32_t c0, uint32_t nc) {
   using C = Chan<KK, MIR>;
   constexpr bool X = KT<KK>::CPLX;
-  put_tile<X, false>(a.out0, tl, pl, pl + PSZ);
+  put_tile<X, false>(a.out0, tl, pl, pl + PSZ, c0, nc);
   if constexpr (KT<KK>::NOUT == 2)
-    put_tile<X, false>(a.out1, tl, pl + C::W * PSZ, pl + (C::W + 1) * PSZ);
+    put_tile<X, false>(a.out1, tl, pl + C::W * PSZ, pl + (C::W + 1) * PSZ, c0, nc);
   if constexpr (MIR) {
     if (tl.mate == 0) return;
     const h2b_tile tm = a.tiles[tl.mate - 1];
     const double *m = C::SLP ? pl : pl + C::OWN * PSZ;
     if constexpr (KT<KK>::NOUT == 2) {
-      put_tile<X, true>(a.out0, tm, pl, pl + PSZ);
-      put_tile<X, true>(a.out1, tm, m, m + PSZ);
+      put_tile<X, true>(a.out0, tm, pl, pl + PSZ, c0, nc);
+      put_tile<X, true>(a.out1, tm, m, m + PSZ, c0, nc);
     } else {
-      put_tile<X, true>(a.out0, tm, m, m + PSZ);
+      put_tile<X, true>(a.out0, tm, m, m + PSZ, c0, nc);
     }
   }
 }
@@ -904,7 +907,15 @@ __device__ __forceinline__ void put_planes(const DistArgs &a, const h2b_tile &tl
 // 6.66; the walk with additions per lane, no mates 5.62; this kernel 4.29 (FP64 pipe 59 % busy, three
 // warps per scheduler; 15 % of the lanes idle in groups of fewer than 32 row triangles).  Single
 // layer of 16200 triangles 2.02 -> 0.93.
-constexpr uint32_t RING_EXTRA = 3;
+//
+// Where the tiles are fewer than the CTAs that fit (RING_FILL times over), the CTAs of a cluster of up
+// to RING_CLUSTER share a tile's units, add each other's planes column by column through distributed
+// shared memory and write a share of the columns each: more SMs have work, and a block can be cut into
+// larger tiles, which evaluate fewer border pairs twice.  Double layer of 578 vertices, complex: one
+// CTA per tile of 32 642 us; tiles of 64, clusters filling the SMs once 510, twice 449, three times
+// 421.  V and K of 1352 triangles 309 -> 174 (eight times: 209).  The two kinds are separate kernels:
+// one for both spills the fused layers' registers (4290 -> 4320 us above).
+constexpr uint32_t RING_EXTRA = 3, RING_CLUSTER = 8, RING_FILL = 3;
 struct RingWarp {
   double rec[2][22];  // QuadRec of the current and the next column triangle
   double w[3][4];     // per slot and point: weight times nodal function times Gram determinant, kconst
@@ -924,7 +935,7 @@ constexpr int ring_threads() { return Chan<KK, MIR>::ALL > 3 ? 256 : Chan<KK, MI
 template <int KK, bool MIR>
 constexpr int ring_ctas() { return Chan<KK, MIR>::ALL > 3 ? 1 : 2; }
 
-template <int KK, bool RL, bool MIR>
+template <int KK, bool RL, bool MIR, bool SHARED>
 __global__ void __launch_bounds__(ring_threads<KK, MIR>(), ring_ctas<KK, MIR>())
     near_ring_kernel(DistArgs a) {
   using C = Chan<KK, MIR>;
@@ -936,21 +947,34 @@ __global__ void __launch_bounds__(ring_threads<KK, MIR>(), ring_ctas<KK, MIR>())
   double *snod = sm + NCH * PSZ;                        // 3 x 4: weight times nodal function
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
   RingWarp &W = reinterpret_cast<RingWarp *>(snod + 12)[warp];
-  const h2b_tile tl = a.tiles[a.list ? a.list[blockIdx.x] : blockIdx.x];
+  // SHARED: the CTAs of a cluster share a tile.  The CTA's place, read again where it is used
+  // (registers)
+  auto blk = []() {
+    uint32_t v = 0;
+    if constexpr (SHARED) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(v));
+    return v;
+  };
+  auto nblk = []() {
+    uint32_t v = 1;
+    if constexpr (SHARED) asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(v));
+    return v;
+  };
+  const uint32_t it = blockIdx.x / nblk();
+  const h2b_tile tl = a.tiles[a.list ? a.list[it] : it];
   for (uint32_t e = tid; e < (uint32_t) (NCH * PSZ); e += T) planes[e] = 0.0;
   if (tid < 12) snod[tid] = sd[3 + tid / 4][tid & 3u] * a.kconst;
   const uint32_t ntr = tl.tr_len, nsc = tl.sc_len, ng = (ntr + 31u) / 32u;
   uint32_t nseg, len;
   {
     const uint32_t cand = max(1u, min(lane + 1u, nsc));
-    const uint32_t cost = ((cand * ng + NW - 1) / NW) * ((nsc + cand - 1) / cand + RING_EXTRA);
+    const uint32_t cost = ((cand * ng + NW * nblk() - 1) / (NW * nblk())) * ((nsc + cand - 1) / cand + RING_EXTRA);
     nseg = (__reduce_min_sync(0xffffffffu, cost << 5 | (cand - 1u)) & 31u) + 1u;
     len = max(1u, (nsc + nseg - 1) / nseg);
     nseg = (nsc + len - 1) / len;
   }
   __syncthreads();
 
-  for (uint32_t u = warp; u < ng * nseg; u += NW) {
+  for (uint32_t u = warp * nblk() + blk(); u < ng * nseg; u += NW * nblk()) {
     const uint32_t is = u / ng, ig = u - is * ng;
     const uint32_t g0 = (uint32_t) ((uint64_t) ig * ntr / ng);
     const uint32_t ngr = (uint32_t) ((uint64_t) (ig + 1) * ntr / ng) - g0;
@@ -1169,8 +1193,28 @@ __global__ void __launch_bounds__(ring_threads<KK, MIR>(), ring_ctas<KK, MIR>())
       }
     }
   }
-  __syncthreads();
-  put_planes<KK, MIR>(a, tl, planes);
+  if constexpr (!SHARED) {
+    __syncthreads();
+    put_planes<KK, MIR>(a, tl, planes, 0, tl.cols);
+  } else {
+    const uint32_t nb = nblk(), b = blk();
+    cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    // each CTA of the cluster adds and writes a share of the columns
+    cl.sync();
+    const uint32_t c0 = b * tl.cols / nb, nc = (b + 1) * tl.cols / nb - c0;
+    for (uint32_t e = tid; e < nc * tl.rows; e += T) {
+      const uint32_t c = e / tl.rows, p = e - c * tl.rows + PLD * (c0 + c);
+  #pragma unroll
+      for (int ch = 0; ch < NCH; ch++) {
+        double v = planes[ch * PSZ + p];
+        for (uint32_t k = 1; k < nb; k++)
+          v += cl.map_shared_rank(planes, (b + k) % nb)[ch * PSZ + p];
+        planes[ch * PSZ + p] = v;
+      }
+    }
+    cl.sync();
+    put_planes<KK, MIR>(a, tl, planes, c0, nc);
+  }
 }
 
 // Constant bases: a pair is an entry.  A thread per pair, lanes on consecutive row triangles (column
@@ -1587,18 +1631,38 @@ int launch_dist(const h2b_near_launch *L, cudaStream_t st) {
   return H2B_OK;
 }
 
-// MIR: the tiles of L->half fill their mates too; otherwise every tile by itself.
+// MIR: the tiles of L->half fill their mates too; otherwise every tile by itself.  (block_tile in
+// api_core.cu counts on the cluster rule.)
 template <int KK, bool RL, bool MIR>
 int launch_ring(const h2b_near_launch *L, cudaStream_t st) {
   constexpr int T = ring_threads<KK, MIR>();
   const size_t smem =
       sizeof(double) * (Chan<KK, MIR>::ALL * PSZ + 12) + sizeof(RingWarp) * (T / 32);
-  H2B_CUDA_TRY((h2b_allow_smem<near_ring_kernel<KK, RL, MIR>>()));
+  H2B_CUDA_TRY((h2b_allow_smem<near_ring_kernel<KK, RL, MIR, false>>()));
+  H2B_CUDA_TRY((h2b_allow_smem<near_ring_kernel<KK, RL, MIR, true>>()));
   DistArgs a = dist_args(L);
   a.list = MIR ? L->half : nullptr;
   const uint32_t n = MIR ? L->nhalf : L->ntiles;
   if (n > 0) {
-    near_ring_kernel<KK, RL, MIR><<<n, T, smem, st>>>(a);
+    const uint32_t slots = ring_ctas<KK, MIR>() * (L->num_sms > 0 ? L->num_sms : 148);
+    uint32_t share = 1;
+    while (share < RING_CLUSTER && 2 * share * n <= RING_FILL * slots) share *= 2;
+    if (share == 1) {
+      near_ring_kernel<KK, RL, MIR, false><<<n, T, smem, st>>>(a);
+    } else {
+      cudaLaunchAttribute at;
+      at.id = cudaLaunchAttributeClusterDimension;
+      at.val.clusterDim.x = share;
+      at.val.clusterDim.y = at.val.clusterDim.z = 1;
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(n * share);
+      cfg.blockDim = dim3(T);
+      cfg.dynamicSmemBytes = smem;
+      cfg.stream = st;
+      cfg.attrs = &at;
+      cfg.numAttrs = 1;
+      H2B_CUDA_TRY((cudaLaunchKernelEx(&cfg, near_ring_kernel<KK, RL, MIR, true>, a)));
+    }
     h2b_note_launch();
   }
   H2B_CUDA_TRY(cudaGetLastError());
