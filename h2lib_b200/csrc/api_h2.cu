@@ -1271,7 +1271,7 @@ extern "C" int h2b_h2matrix_info(const h2b_h2matrix *h, uint64_t info[8]) {
   info[1] = (uint64_t) h->nadm * h->k * h->k;
   info[2] = h->rt.vtotal + h->ct.vtotal;
   info[3] = (uint64_t) (h->rt.n - 1 + h->ct.n - 1) * h->k * h->k;
-  info[4] = 8 * (W * (info[0] + info[1]) + info[2] + info[3]);
+  info[4] = 8 * (W * (info[0] + (uint64_t) h->nstored * h->k * h->k) + info[2] + info[3]);
   info[5] = h->nadm;
   info[6] = h->nnear;
   info[7] = h->k;
@@ -1535,11 +1535,7 @@ static int addeval_prec(double alpha_re, double alpha_im, const h2b_h2matrix *h,
       rc = H2B_ERR_CUDA;
     }
   }
-  if (rc == H2B_OK && cudaStreamSynchronize(h->st) != cudaSuccess) {
-    h2b_set_error("h2b_h2matrix_addeval: %s", cudaGetErrorString(cudaGetLastError()));
-    rc = H2B_ERR_CUDA;
-  }
-  if (rc == H2B_OK) rc = h2b_h2_check_mv_error(h);
+  if (rc == H2B_OK) rc = h2b_h2_check_mv_error(h);  // waits for the stream
   float t;
   if (rc == H2B_OK && cudaEventElapsedTime(&t, h->ev[9], h->ev[10]) == cudaSuccess)
     const_cast<h2b_h2matrix *>(h)->ms[5] = t;

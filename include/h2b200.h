@@ -275,8 +275,8 @@ int h2b_h2matrix_assemble_all(h2b_h2matrix *h2);
 int h2b_h2matrix_assemble_nearfield_pair(h2b_h2matrix *a, h2b_h2matrix *b);
 
 /* Storage and counts: info[0] nearfield entries, [1] coupling entries, [2] leaf-basis entries,
- * [3] transfer entries, [4] bytes of device storage, [5] admissible blocks, [6] nearfield blocks,
- * [7] rank k. */
+ * [3] transfer entries, [4] bytes of device storage (of two transposed coupling matrices one is
+ * stored), [5] admissible blocks, [6] nearfield blocks, [7] rank k. */
 int h2b_h2matrix_info(const h2b_h2matrix *h2, uint64_t info[8]);
 
 /* Precision of the regular (distant-pair) nearfield quadrature of later assembly calls:
@@ -374,7 +374,8 @@ int h2b_h2matrix_export_wait(h2b_h2matrix *h2);
 int h2b_h2matrix_addeval(double alpha_re, double alpha_im, const h2b_h2matrix *h2,
                          const double *x, double *y);
 
-/* Same with nrhs right-hand sides stored as columns of X (ldx) and Y (ldy). */
+/* Same with nrhs right-hand sides stored as columns of X (ldx) and Y (ldy), the columns of a product
+ * together.  Where Y overlaps X otherwise than as the same columns, one column after the other. */
 int h2b_h2matrix_addeval_multi(double alpha_re, double alpha_im, const h2b_h2matrix *h2,
                                uint32_t nrhs, const double *X, uint64_t ldx, double *Y,
                                uint64_t ldy);
