@@ -422,7 +422,7 @@ __global__ void cg_dir_kernel(double *p, const double *r, uint32_t n, const doub
 // (two buffers in turn) and gathers M p over the triangles around the vertex; sums of a CTA go to
 // the other CTAs through shared memory.  A thread keeps the first CG_KEEP triangles around its first
 // vertex in registers, so that up to 4096 vertices a step waits for one load and not for a chain of
-// four.  1026 vertices, 54 steps: separate kernels and their read-backs about 1900 us, this one 226
+// four.  678 vertices, 54 steps: separate kernels and their read-backs about 1900 us, this one 226
 // (695 without the kept triangles).
 constexpr int CG_CTAS = 8, CG_THREADS = 512, CG_KEEP = 7;
 

@@ -131,7 +131,7 @@ __device__ __forceinline__ void put_part(const GmresDev &g, const Sys &v, uint32
 // The vector kernels of a step take the columns of V in CGRP groups: thread (r, cg) has row r of the
 // CTA's TPB rows and the columns j = cg mod CGRP, so a thread's chain of loads is a quarter as long and
 // a small system (a few CTAs) keeps four times the loads in flight.  A step's vector kernels on
-// 1026 rows, k to 50: one thread per row 24.5 us, CGRP = 4 16.7; 96 systems of 570 rows on average
+// 678 rows, k to 50: one thread per row 24.5 us, CGRP = 4 16.7; 96 systems of 570 rows on average
 // 36.6 and 34.0.
 constexpr int CGRP = 4;
 constexpr int VTHREADS = TPB * CGRP;
