@@ -34,16 +34,17 @@ Z = (1.2, 1.2, 1.2)
 # algorithmic FP64 operations per quadrature point (reference source, + - * / sqrt counted as 1):
 # linear-basis single layer 64, double layer 72
 FLOPS_PER_POINT = {"slp": 64, "dlp": 72}
-# flops the tensor-factored distant-pair sum executes per triangle pair for SLP+DLP, linear basis,
-# q = 2 (FMA = 2), from the staged quadrature points: 16 point pairs x 37 (difference 3, r^2 5,
-# rsqrt 13, normal part 4, three column weights per channel 12) + 4 row points x 41 (<x_a, n> 5,
-# 3 x 3 x 2 outer FMAs 36) + 20 for the scaling.  The points themselves and their normal
-# components are formed once per staged triangle (about 1 flop per pair, not counted).
-EXECUTED_FLOPS_PER_PAIR = 16 * 37 + 4 * 41 + 20
-# the same for the constant-basis single layer (dense cc SLP leg): 16 point pairs x 23
-# (difference 3, r^2 5, rsqrt 13, weighted sum 2) + 4 row points x 2 (outer sum) + 2 (scaling);
-# the reference counts 46 per point
-CC_SLP_FLOPS_PER_PAIR = 16 * 23 + 4 * 2 + 2
+# flops the tensor-factored distant-pair sum executes per ordered triangle pair for SLP+DLP, linear
+# basis, q = 2 (FMA = 2), from the staged quadrature points.  A tile is filled together with its
+# transposed one, so an evaluation of two triangles serves both orders: 16 point pairs x 44
+# (difference 3, r^2 5, rsqrt 8, both normal parts and r^-3 10, three row weights for three channels
+# 18) + 4 column points x 54 (3 x 3 x 3 outer FMAs) + 20 (<x, n>), halved.  (Tiles on the diagonal
+# are filled alone; they are counted the same.)
+EXECUTED_FLOPS_PER_PAIR = (16 * 44 + 4 * 54 + 20) // 2
+# the same for the constant-basis single layer (dense cc SLP leg): 16 point pairs x 18 (difference 3,
+# r^2 5, rsqrt 8, weighted sum 2) + 4 row points x 2 (outer sum) + 3 (scaling), halved; the reference
+# counts 46 per point
+CC_SLP_FLOPS_PER_PAIR = (16 * 18 + 4 * 2 + 3) / 2
 CC_SLP_REF_FLOPS_PER_POINT = 46
 # reference count per point of the Helmholtz kernels, constant basis (sin, cos and exp counted
 # as 1): single layer 54, double layer 66
@@ -398,7 +399,7 @@ def run_ours(a, rank, world, local):
                                                            FLOPS_PER_POINT["dlp"])}
     uniq["executed_tflops"] = uniq["executed_flops"] / (near_dist_ms * 1e-3) / 1e12
     uniq["reference_count_tflops"] = uniq["reference_count_flops"] / (near_dist_ms * 1e-3) / 1e12
-    roofline = {"bound": "fp64", "kernel": "near_dist_kernel (fused SLP+DLP, linear basis)",
+    roofline = {"bound": "fp64", "kernel": "near_ring_kernel (fused SLP+DLP, linear basis)",
                 "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                 "traffic": NEAR_DIST_TRAFFIC if (a.split, a.clf, a.m) == (64, 64, 4) else None,
                 "flops_per_launch": executed, "flops_per_pair": EXECUTED_FLOPS_PER_PAIR,
@@ -412,7 +413,7 @@ def run_ours(a, rank, world, local):
                 "unique_pairs": uniq}
 
     # ---- matvec roofline (HBM): bytes of S, N, V, E read once per product.  The operator
-    # (0.55 GB of algorithmic bytes, 0.63 GB read) is five times L2, so products run back to back
+    # (0.38 GB of algorithmic bytes) is three times L2, so products run back to back
     # without a flush: a flush leaves L2 full of dirty lines whose write-back the next product
     # would pay for.
     x = torch.randn(V.cols, dtype=torch.float64, device="cuda")
@@ -428,8 +429,7 @@ def run_ours(a, rank, world, local):
         return statistics.mean(mv)
 
     inf = V.info()
-    mv_bytes = 8 * (inf["near_entries"] + inf["coupling_entries"] + inf["leaf_entries"]
-                    + inf["transfer_entries"])
+    mv_bytes = inf["bytes"]  # of two transposed coupling matrices one is stored and read
     mv_ms = time_mv(hb.addeval_h2matrix_avector)
     V.make_single()
     mv32_ms = time_mv(hb.addeval_h2matrix_avector_single)
@@ -447,7 +447,7 @@ def run_ours(a, rank, world, local):
                "traffic_source": "ncu on the sphere split 48, scaled by the stored entries",
                "peak_source": "MEASURED_PEAKS.json hbm_gbs" if peaks else "fallback 6650 GB/s",
                "bytes_per_launch": mv_bytes, "launch_ms": mv_ms,
-               "l2": "no flush between products (operator 4x larger than L2)",
+               "l2": "no flush between products (operator 3x larger than L2)",
                "launches_per_product": 5}
     roof_mv32 = {"bound": "hbm", "kernel": "H2 matvec from the FP32 copies (FP64 vectors/sums)",
                  "achieved": mv_bytes / 2 / (mv32_ms * 1e-3) / 1e9, "peak": hbm, "unit": "GB/s",
@@ -763,7 +763,7 @@ def run_dense(a, peak):
                       "identical": int(sing[3])},
             "near_distant_ms": d, "near_singular_ms": statistics.mean(sing_ms),
             "call_wall_ms": statistics.mean(wall),
-            "roofline": {"bound": "fp64", "kernel": "near_dist_kernel (constant basis SLP)",
+            "roofline": {"bound": "fp64", "kernel": "near_pair_kernel (constant basis SLP)",
                          "flops_per_pair": CC_SLP_FLOPS_PER_PAIR,
                          "achieved": executed / (d * 1e-3) / 1e12, "peak": peak,
                          "unit": "TFLOP/s", "frac": executed / (d * 1e-3) / 1e12 / peak,
