@@ -51,12 +51,14 @@ CC_SLP_REF_FLOPS_PER_POINT = 46
 HELM_FLOPS_PER_POINT = {"slp": 54, "dlp": 66}
 # DRAM bytes (read 5,998,336 + write 214,822,656) of one near_dist_kernel launch on the default
 # workload (sphere split 64), from an ncu capture of the full-size run (single-pass metrics
-# dram__bytes_read.sum + dram__bytes_write.sum)
+# dram__bytes_read.sum + dram__bytes_write.sum) of the kernel that filled every tile by itself; the
+# output, which is nearly all of it, is the same
 NEAR_DIST_TRAFFIC = 5998336 + 214822656
-# DRAM bytes (read + write) of one FP64 matvec product per algorithmic byte: 301.7 MB for
-# 284.3 MB on the sphere split 48 (ncu, dram__bytes_read.sum + dram__bytes_write.sum of the three
-# item-kernel launches of a product), applied to the bench's workload by its stored entries
-MATVEC_TRAFFIC_RATIO = 301.7 / 284.3
+# DRAM bytes (read + write) of one FP64 matvec product per algorithmic byte: 206.0 MB for
+# 200.8 MB on the sphere split 48 (ncu, dram__bytes_read.sum + dram__bytes_write.sum of the two
+# item-kernel launches and the coupling launch of a product), applied to the bench's workload by its
+# stored entries
+MATVEC_TRAFFIC_RATIO = 206.0 / 200.8
 
 
 def parse():
