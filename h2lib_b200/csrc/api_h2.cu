@@ -1398,7 +1398,13 @@ extern "C" int h2b_h2matrix_export_async(h2b_h2matrix *h, int part, uint32_t cou
   int rc = h2b_h2matrix_export(h, part, count, nullptr, &n);
   if (rc != H2B_OK || n == 0) return rc;
   const double *src = part == 0 ? h->rt.d_V : part == 1 ? h->rt.d_E : part == 4 ? h->d_S : h->d_N;
-  if (!h->cst) H2B_CUDA_TRY(cudaStreamCreateWithFlags(&h->cst, cudaStreamNonBlocking));
+  if (!h->cst) {
+    // ahead of the assembly that runs meanwhile: a piece of coupling matrices is put out by a small
+    // kernel before its copy, which would wait behind the nearfield's whole grid
+    int low, high;
+    H2B_CUDA_TRY(cudaDeviceGetStreamPriorityRange(&low, &high));
+    H2B_CUDA_TRY(cudaStreamCreateWithPriority(&h->cst, cudaStreamNonBlocking, high));
+  }
   if (!h->ev_copy) H2B_CUDA_TRY(cudaEventCreateWithFlags(&h->ev_copy, cudaEventDisableTiming));
   // after everything already queued on the matrix's stream, on the copy stream
   H2B_CUDA_TRY(cudaEventRecord(h->ev_copy, h->st));
