@@ -470,11 +470,11 @@ __global__ void __launch_bounds__(MAXTHREADS) mv_items_kernel(MvLaunch L) {
 // per panel: for complex rank 125 a 16 KiB panel has 8 columns, and adding its 125 rows per panel
 // took 485M FP64 additions to L2 for a product of 49152 triangles with five columns.  A panel
 // that stands for its block and the transposed one (H2B_MV_SYM) is multiplied a second time,
-// transposed, with the row cluster's x, which comes with the run's first panel.  A warp issues its own
-// copies (panel and x slices, completion on its mbarrier) as soon as it has read the panel
-// before: the other warps of the SM cover the wait, and no warp waits for another's copy to be issued
-// (one producer lane for four warps took twice as long on small matrices).  Waits are bounded; nrhs <=
-// NQ.
+// transposed, with the row cluster's x, which comes with the first of a run's panels that takes it.  A
+// warp issues its own copies (panel and x slices, completion on its mbarrier) as soon as it has read the
+// panel before: the other warps of the SM cover the wait, and no warp waits for another's copy to be
+// issued (one producer lane for four warps took twice as long on small matrices).  Waits are bounded;
+// nrhs <= NQ.
 // 49152 triangles, m = 5, complex: a product with five columns 9.6 ms as five products, 6.2 with the
 // columns together and panels added one by one, 3.2 with this kernel.  32768 triangles, m = 4, real:
 // 104 us reading every block, 88 reading one of two.
@@ -498,7 +498,7 @@ __global__ void __launch_bounds__(CP_WARPS * 32) mv_coupling_kernel(MvLaunch L) 
   __syncwarp();
   // the warp's runs: every wall-th
   const uint32_t nruns = (L.n + L.run - 1) / L.run, wall = gridDim.x * L.nw;
-  // lane 0: copies panel m and its x slices; head: the row slices too
+  // lane 0: copies panel m and its x slices; head: the row slices too, where it takes them
   auto issue = [&](const MvItem &m, bool head) {
     size_t n;
     const char *pa = panel_addr<CX, T>(L, m, n), *lo, *xl;
@@ -658,7 +658,9 @@ __global__ void __launch_bounds__(CP_WARPS * 32) mv_coupling_kernel(MvLaunch L) 
     }
     __syncwarp();
     if (ni >= L.n) break;
-    if (lane == 0) issue(nm, nm.yo != m.yo || ni != i + 1);
+    // the row slices are there already when the panel before, of the same run and row cluster, took
+    // them; a panel without H2B_MV_SYM takes none (partitions that are not symmetric mix the two)
+    if (lane == 0) issue(nm, nm.yo != m.yo || ni != i + 1 || !sym);
     m = nm;
     i = ni;
   }

@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 from h2lib_b200 import bem3d as hb
-from h2lib_b200._lib import check, lib
+from h2lib_b200._lib import check, checkp, lib
 
 pytestmark = pytest.mark.gpu
 L, K = hb.BASIS_LINEAR_BEM3D, hb.BASIS_CONSTANT_BEM3D
@@ -81,18 +81,16 @@ def test_columns_in_place():
     close(buf, ref)
 
 
-@pytest.mark.parametrize("rb,cb", [(L, L), (K, K), (K, L)])
-@pytest.mark.parametrize("pde,m", [("laplace", 2), ("laplace", 3), ("helmholtz", 5)])
-def test_product_against_parts(pde, m, rb, cb):
-    """rb != cb: the trees differ and no block stands for two."""
-    H = matrix(pde, cb, m, rb)
-    k = m ** 3
+def parts(H):
+    """The matrix put together from its exported parts: leaf bases, transfers, every admissible block's
+    coupling matrix, nearfield blocks."""
+    k = H.info()["rank"]
     rec = H.tree.block_records()
     trees = [H.tree.clusters(s) for s in (0, 1)]
     W = []
     for side, (cl, _, _) in enumerate(trees):
         V, E = H.export(2 * side), H.export(2 * side + 1)
-        vo, eo, full, stack = 0, 0, {}, []
+        vo, eo, full = 0, 0, {}
         # pre-order: leaves' V and non-root clusters' E in that order
         info = []
         for i, (off, size, sons) in enumerate(cl):
@@ -108,12 +106,12 @@ def test_product_against_parts(pde, m, rb, cb):
             if cl[i][2] == 0:
                 return i + 1
             at = i + 1
-            parts = []
+            rows = []
             for _ in range(cl[i][2]):
                 s = at
                 at = son_ids(s)
-                parts.append(full[s] @ E[s])
-            full[i] = np.concatenate(parts)
+                rows.append(full[s] @ E[s])
+            full[i] = np.concatenate(rows)
             return at
         son_ids(0)
         W.append({(int(cl[i][0]), int(cl[i][1])): full[i] for i in range(len(cl))})
@@ -130,8 +128,78 @@ def test_product_against_parts(pde, m, rb, cb):
             B = N[no:no + rs * cs].reshape(cs, rs).T
             no += rs * cs
         A[np.ix_(r, c)] = B
+    return A
+
+
+@pytest.mark.parametrize("rb,cb", [(L, L), (K, K), (K, L)])
+@pytest.mark.parametrize("pde,m", [("laplace", 2), ("laplace", 3), ("helmholtz", 5)])
+def test_product_against_parts(pde, m, rb, cb):
+    """rb != cb: the trees differ and no block stands for two."""
+    H = matrix(pde, cb, m, rb)
+    A = parts(H)
     X = vectors(H, H.cols, 3)
     Y = np.zeros((3, H.rows), dtype=H.dtype)
     multi(H, 1.0, 3, X, H.cols, Y, H.rows)
     close(Y.T, A @ X.T)
     close(singles(H, 1.0, X, np.zeros_like(Y)).T, A @ X.T)
+
+
+def one_sided(tree, by_row):
+    """The same clusters with some of the admissible blocks above the diagonal cut into their sons'
+    blocks, so that the blocks across the diagonal from them have no transposed partner.  by_row: the
+    blocks of a row cluster one after the other, else the order of the block tree."""
+    rec, box, idx = tree.clusters()
+    ids = {(int(o), int(s)): i for i, (o, s, _) in enumerate(rec)}
+    ends = {}
+
+    def walk(i):
+        end = i + 1
+        for _ in range(int(rec[i][2])):
+            end = walk(end)
+        ends[i] = end
+        return end
+    walk(0)
+    sons = {i: [i + 1, ends[i + 1]] for i in range(len(rec)) if rec[i][2]}
+    blocks = []
+    for r0, rs, c0, cs, adm in tree.block_records():
+        r, c = ids[int(r0), int(rs)], ids[int(c0), int(cs)]
+        if adm and r < c and r in sons and c in sons and (r + c) % 3:
+            blocks += [(a, b, 1) for b in sons[c] for a in sons[r]]
+        else:
+            blocks.append((r, c, int(adm)))
+    if by_row:
+        blocks.sort()
+    b = np.array(blocks, dtype=np.uint32)
+    tr = [np.ascontiguousarray(rec[:, j]) for j in range(3)] + [np.ascontiguousarray(box), len(idx), idx]
+    handle = lib.h2b_tree_new_flat(len(rec), *tr, len(rec), *tr, len(b), np.ascontiguousarray(b[:, 0]),
+                                   np.ascontiguousarray(b[:, 1]),
+                                   np.ascontiguousarray(b[:, 2].astype(np.uint8)))
+    pairs = {(r, c) for r, c, a in blocks if a}
+    alone = sum((c, r) not in pairs for r, c in pairs)
+    return hb.Tree(checkp(handle, "h2b_tree_new_flat")), alone, len(pairs)
+
+
+@pytest.mark.parametrize("shape", ["symmetric", "one-sided", "one-sided by row"])
+@pytest.mark.parametrize("pde,leaf,panels", [("laplace", 16, (4, 5, 6)), ("helmholtz", 24, (4, 6, 8))])
+def test_runs_of_panels(pde, leaf, panels, shape):
+    """Runs of several coupling panels per warp.  At rank 125 the panels of a few KiB are 21 to 63 per
+    block and 23000 to 82000 in all, which makes runs of one to seven panels where the default panels'
+    are single; some lengths divide a block's panels and some do not.  Runs keep their sums over panels,
+    change the row cluster and, with a partition that is not symmetric, go from blocks without a
+    transposed partner to blocks with one of the same row cluster and back."""
+    gr = hb.new_ellipsoid_surface3d(13, (1.0, 0.8, 1.3))
+    tree = hb.build_tree(gr, K, K, leaf, 1.4)
+    if shape != "symmetric":
+        tree, alone, total = one_sided(tree, shape.endswith("row"))
+        assert total // 8 < alone < total
+    op = (hb.new_dlp_laplace_bem3d(gr, 2, 4, K, K, 0.5) if pde == "laplace"
+          else hb.new_dlp_helmholtz_bem3d(2.0, gr, 2, 4, K, K, 0.5))
+    H = hb.H2Matrix(op, tree, 5).assemble()
+    A = parts(H)
+    for kib in panels:
+        H.set_matvec_shape(panel_kib=kib)
+        for cols in (1, 3, 5, 8):
+            X = vectors(H, H.cols, cols, cols)
+            Y = np.zeros((cols, H.rows), dtype=H.dtype)
+            multi(H, 1.0, cols, X, H.cols, Y, H.rows)
+            close(Y.T, A @ X.T)
