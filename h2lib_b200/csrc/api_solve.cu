@@ -453,6 +453,8 @@ __global__ void __cluster_dims__(CG_CTAS, 1, 1) __launch_bounds__(CG_THREADS)
                    const double *v, double *x, double *r, double *p0, double *p1, double *ap) {
   __shared__ double tot[2][CG_CTAS], red[CG_THREADS / 32];
   const uint32_t t0 = blockIdx.x * CG_THREADS + threadIdx.x, stride = CG_CTAS * CG_THREADS;
+  // the other CTAs' shared memory may be written once they all run
+  cooperative_groups::this_cluster().sync();
   int slot = 0;
   double rr = 0.0;
   for (uint32_t i = t0; i < nv; i += stride) {

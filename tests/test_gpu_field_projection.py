@@ -49,3 +49,22 @@ def test_projection(gr):
     dlp = hb.new_dlp_laplace_bem3d(gr, 2, 4, L, L, 0.5)
     z = (1.9, 2.1, -2.3)
     close(hb.project_l2_harmonic(dlp, z), orc.project_l2_harmonic(mesh(gr), z), 1e-12)
+
+
+def test_projection_beside_other_work():
+    """The CTAs of the projection's cluster write into each other's shared memory from the first sum on.
+    Beside kernels that keep the SMs full they start one after the other, as SMs become free."""
+    import torch
+    gr = hb.new_sphere_surface3d(13)
+    dlp = hb.new_dlp_laplace_bem3d(gr, 2, 4, L, L, 0.5)
+    z = (1.9, 2.1, -2.3)
+    ref = orc.project_l2_harmonic(mesh(gr), z)
+    side = torch.cuda.Stream()
+    a = torch.randn(1 << 24, device="cuda")
+    torch.cuda.synchronize()
+    for _ in range(40):
+        with torch.cuda.stream(side):
+            for _ in range(20):
+                a.mul_(1.0000001)
+        close(hb.project_l2_harmonic(dlp, z), ref, 1e-12)
+    torch.cuda.synchronize()
