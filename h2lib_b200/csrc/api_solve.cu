@@ -423,8 +423,13 @@ __global__ void cg_dir_kernel(double *p, const double *r, uint32_t n, const doub
 // the other CTAs through shared memory.  A thread keeps the first CG_KEEP triangles around its first
 // vertex in registers, so that up to 4096 vertices a step waits for one load and not for a chain of
 // four.  678 vertices, 54 steps: separate kernels and their read-backs about 1900 us, this one 226
-// (695 without the kept triangles).
+// (695 without the kept triangles).  Eight SMs are all it has, so its time grows with the vertices where
+// the separate kernels (mass_cg_launches) have the whole device and wait for the read-backs: ms per
+// call, this kernel and those, 678 vertices 0.26 and 2.37, 4098 0.44 and 2.78, 16386 1.94 and 3.04,
+// 24338 2.85 and 3.06, 32402 3.93 and 3.17, 518402 69.9 and 10.0.  It serves up to CG_MAX vertices, six
+// per thread.
 constexpr int CG_CTAS = 8, CG_THREADS = 512, CG_KEEP = 7;
+constexpr uint32_t CG_MAX = 6 * CG_CTAS * CG_THREADS;
 
 // Sum over the cluster of one value per thread; slot: the parity of the call (a CTA may still read the
 // previous sum).  Contains the cluster barrier that ends the pass.
@@ -829,6 +834,34 @@ int harm_args(const h2b_bem *bem, const double z[3], double *scratch, HarmArgs *
   return H2B_OK;
 }
 
+// The same CG by separate kernels over the whole device, the residual read back each step: sc holds
+// four doubles, v and x are set (x = 0).
+int mass_cg_launches(const h2b_surface *s, const double *v, double *x, double *r, double *p,
+                     double *ap, double *sc, cudaStream_t st) {
+  const uint32_t nv = s->nv, nt = s->nt;
+  H2B_CUDA_TRY(cudaMemcpyAsync(r, v, sizeof(double) * nv, cudaMemcpyDeviceToDevice, st));
+  H2B_CUDA_TRY(cudaMemcpyAsync(p, v, sizeof(double) * nv, cudaMemcpyDeviceToDevice, st));
+  double rr;
+  H2B_CUDA_TRY(cudaMemsetAsync(sc, 0, sizeof(double) * 4, st));
+  dot_kernel<<<64, 256, 0, st>>>(r, r, nv, sc);
+  H2B_CUDA_TRY(cudaMemcpyAsync(&rr, sc, sizeof(double), cudaMemcpyDeviceToHost, st));
+  H2B_CUDA_TRY(cudaStreamSynchronize(st));
+  const double norm = sqrt(rr);
+  for (uint32_t it = 0; sqrt(rr) > 1e-15 * norm && it + 1 < 500; it++) {
+    H2B_CUDA_TRY(cudaMemsetAsync(ap, 0, sizeof(double) * nv, st));
+    mass_multi_kernel<<<(nt + 127) / 128, 128, 0, st>>>(s->d_tri, nt, nv, p, ap);
+    H2B_CUDA_TRY(cudaMemsetAsync(sc + 1, 0, sizeof(double) * 2, st));
+    dot_kernel<<<64, 256, 0, st>>>(p, ap, nv, sc + 1);
+    cg_update_kernel<<<64, 256, 0, st>>>(x, r, p, ap, nv, sc);
+    dot_kernel<<<64, 256, 0, st>>>(r, r, nv, sc + 2);
+    cg_dir_kernel<<<64, 256, 0, st>>>(p, r, nv, sc);
+    H2B_CUDA_TRY(cudaMemcpyAsync(sc, sc + 2, sizeof(double), cudaMemcpyDeviceToDevice, st));
+    H2B_CUDA_TRY(cudaMemcpyAsync(&rr, sc, sizeof(double), cudaMemcpyDeviceToHost, st));
+    H2B_CUDA_TRY(cudaStreamSynchronize(st));
+  }
+  return H2B_OK;
+}
+
 }  // namespace
 
 extern "C" int h2b_project_l2_harmonic(const h2b_bem *bem, const double z[3], double *w) {
@@ -841,17 +874,22 @@ extern "C" int h2b_project_l2_harmonic(const h2b_bem *bem, const double z[3], do
   const uint32_t nv = s->nv, nt = s->nt;
   DevBuf buf;
   buf.st = st;
-  H2B_CUDA_TRY(cudaMallocAsync(&buf.p, sizeof(double) * (6 * (size_t) nv + 6 * 64), st));
+  H2B_CUDA_TRY(cudaMallocAsync(&buf.p, sizeof(double) * (6 * (size_t) nv + 6 * 64 + 4), st));
   double *v = (double *) buf.p, *x = v + nv, *r = x + nv, *p = r + nv, *p1 = p + nv, *ap = p1 + nv,
-         *rule = ap + nv;
+         *rule = ap + nv, *sc = rule + 6 * 64;
   HarmArgs a;
   int rc = harm_args(bem, z, rule, &a, st);
   if (rc != H2B_OK) return rc;
-  H2B_CUDA_TRY(cudaMemsetAsync(v, 0, sizeof(double) * nv, st));
+  H2B_CUDA_TRY(cudaMemsetAsync(v, 0, sizeof(double) * 2 * nv, st));
   project_rhs_kernel<<<(nt + 127) / 128, 128, 0, st>>>(a, v);
-  mass_cg_kernel<<<CG_CTAS, CG_THREADS, 0, st>>>(s->d_tri, s->d_vt_off, s->d_vt_tri, nv, v, x, r, p,
-                                                 p1, ap);
-  h2b_note_launch();
+  if (nv <= CG_MAX) {
+    mass_cg_kernel<<<CG_CTAS, CG_THREADS, 0, st>>>(s->d_tri, s->d_vt_off, s->d_vt_tri, nv, v, x, r, p,
+                                                   p1, ap);
+    h2b_note_launch();
+  } else {
+    rc = mass_cg_launches(s, v, x, r, p, ap, sc, st);
+    if (rc != H2B_OK) return rc;
+  }
   H2B_CUDA_TRY(cudaGetLastError());
   H2B_CUDA_TRY(cudaMemcpyAsync(w, x, sizeof(double) * nv, cudaMemcpyDefault, st));
   H2B_CUDA_TRY(cudaStreamSynchronize(st));

@@ -1,7 +1,8 @@
 """Field evaluation and L2 projection against the oracle where their kernels can go wrong: point
 counts around a warp and around what one pass of a CTA takes, damped wave numbers, meshes smaller
 and larger than one stretch of sources; vertices above one per thread of the projection's launch,
-vertices with more triangles than a thread keeps.
+vertices with more triangles than a thread keeps, meshes on both sides of the change (24576 vertices)
+from one launch to a kernel per pass.
 
 The field is a sum of n terms in another order: its error is at most n eps sum |terms|, and the sums
 here stay below n eps * 100 |u| = 1e-10 for n = 5e3, in the root mean square below 1e-12.  The
@@ -43,6 +44,8 @@ def test_field(basis, k, split):
 @pytest.mark.parametrize("gr", [lambda: hb.new_sphere_surface3d(1),
                                 lambda: hb.new_sphere_surface3d(32),      # 4098 vertices
                                 lambda: hb.new_cube_surface3d(38),        # 8666 vertices
+                                lambda: hb.new_sphere_surface3d(78),      # 24338, one launch
+                                lambda: hb.new_cube_surface3d(64),        # 24578, a kernel per pass
                                 lambda: bipyramid(7), lambda: bipyramid(8), lambda: bipyramid(60)])
 def test_projection(gr):
     gr = gr()
