@@ -1446,22 +1446,30 @@ extern "C" int h2b_h2matrix_addeval_multi(double alpha_re, double alpha_im,
   const uintptr_t x0 = (uintptr_t) X, x1 = (uintptr_t) (X + W * (ldx * (nrhs - 1ull) + nc));
   const uintptr_t y0 = (uintptr_t) Y, y1 = (uintptr_t) (Y + W * (ldy * (nrhs - 1ull) + nr));
   const bool apart = nrhs > 1 && (x1 <= y0 || y1 <= x0 || (X == Y && ldx == ldy));
-  if (!apart) {
+  auto one_by_one = [&]() {
     for (uint32_t r = 0; r < nrhs; r++) {
       int rc = h2b_h2matrix_addeval(alpha_re, alpha_im, h, X + W * ldx * r, Y + W * ldy * r);
       if (rc != H2B_OK) return rc;
     }
-    return H2B_OK;
-  }
+    return (int) H2B_OK;
+  };
+  if (!apart) return one_by_one();
   // The columns in one launch sequence that reads the matrix once (several when a stage's shared
   // memory holds fewer slices).  The work vectors are the call's own: a stream-ordered
-  // allocation from the device's pool.
+  // allocation from the device's pool.  Where they do not fit, the columns go one by one through the
+  // matrix's own.
   const uint32_t most = h2b_mvm_max_columns(&h->mvm, 0), seqs = (nrhs + most - 1) / most,
                  per = (nrhs + seqs - 1) / seqs;
   const bool dx = h2b_is_device_ptr(X), dy = h2b_is_device_ptr(Y);
   const size_t nwork = h2b_mvm_work_doubles(&h->mvm, per);
   double *buf = nullptr;
-  H2B_CUDA_TRY(cudaMallocAsync((void **) &buf, sizeof(double) * (nwork + W * per * (nc + nr)), h->st));
+  const cudaError_t me =
+      cudaMallocAsync((void **) &buf, sizeof(double) * (nwork + W * per * (nc + nr)), h->st);
+  if (me == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    return one_by_one();
+  }
+  H2B_CUDA_TRY(me);
   double *xd = buf + nwork, *yd = xd + W * per * nc;
   int rc = H2B_OK;
   cudaEventRecord(h->ev[9], h->st);

@@ -2,6 +2,7 @@
 against the matrix put together from its exported parts, which reads every coupling block where the
 product reads one of two transposed ones.  Sums of at most a few thousand FP64 terms in another
 order: 1e-13 on the norm."""
+import contextlib
 import ctypes as C
 
 import numpy as np
@@ -79,6 +80,50 @@ def test_columns_in_place():
         ref[r + 1] = hb.addeval_h2matrix_avector(1.0, H, ref[r].copy(), ref[r + 1].copy())
     multi(H, 1.0, 4, buf, H.cols, C.c_void_p(buf.ctypes.data + buf.strides[0]), H.cols)
     close(buf, ref)
+
+
+@contextlib.contextmanager
+def no_room():
+    """Stream-ordered allocations of 1 MiB and more fail meanwhile: they come from a pool of limited size
+    that is full."""
+    from cuda.bindings import driver as cu
+
+    def ok(r):
+        assert r[0] == cu.CUresult.CUDA_SUCCESS, r[0]
+        return r[1] if len(r) > 1 else None
+    dev = ok(cu.cuCtxGetDevice())
+    props = cu.CUmemPoolProps()
+    props.allocType = cu.CUmemAllocationType.CU_MEM_ALLOCATION_TYPE_PINNED
+    props.location.type = cu.CUmemLocationType.CU_MEM_LOCATION_TYPE_DEVICE
+    props.location.id = int(dev)
+    props.maxSize = 32 << 20
+    pool, before, held = ok(cu.cuMemPoolCreate(props)), ok(cu.cuDeviceGetMemPool(dev)), []
+    while len(held) < 256:
+        r = cu.cuMemAllocFromPoolAsync(1 << 20, pool, cu.CUstream(0))
+        if r[0] != cu.CUresult.CUDA_SUCCESS:
+            break
+        held.append(r[1])
+    assert r[0] == cu.CUresult.CUDA_ERROR_OUT_OF_MEMORY
+    ok(cu.cuDeviceSetMemPool(dev, pool))
+    try:
+        yield
+    finally:
+        ok(cu.cuDeviceSetMemPool(dev, before))
+        for p in held:
+            ok(cu.cuMemFreeAsync(p, cu.CUstream(0)))
+        ok(cu.cuCtxSynchronize())
+        ok(cu.cuMemPoolDestroy(pool))
+
+
+def test_columns_without_room():
+    """Eight columns' work vectors (5 MB) do not fit: one column after the other."""
+    H = matrix("helmholtz", K, 5)
+    X = vectors(H, H.cols, 8)
+    ref = singles(H, 1.0, X, np.zeros_like(X))
+    Y = np.zeros_like(X)
+    with no_room():
+        multi(H, 1.0, 8, X, H.cols, Y, H.rows)
+    close(Y, ref)
 
 
 def parts(H):
