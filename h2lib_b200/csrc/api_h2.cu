@@ -1280,17 +1280,23 @@ extern "C" int h2b_h2matrix_info(const h2b_h2matrix *h, uint64_t info[8]) {
 
 // The coupling matrices of the first n admissible blocks to host memory on stream st: as they are
 // stored, or, where a stored matrix stands for two blocks, put out block by block in pieces of at most
-// 64 MiB of device memory.
+// 64 MiB of device memory, less where that does not fit.
 static int copy_coupling(const h2b_h2matrix *h, uint32_t n, double *out, cudaStream_t st) {
   const uint64_t one = (uint64_t) h->k * h->k * (h->cx ? 2 : 1);
   if (h->nstored == h->nadm) {
     H2B_CUDA_TRY(cudaMemcpyAsync(out, h->d_S, sizeof(double) * one * n, cudaMemcpyDeviceToHost, st));
     return H2B_OK;
   }
-  const uint32_t per =
+  uint32_t per =
       (uint32_t) std::max<uint64_t>(1, std::min<uint64_t>(n, (64u << 20) / (sizeof(double) * one)));
   double *buf = nullptr;
-  H2B_CUDA_TRY(cudaMallocAsync((void **) &buf, sizeof(double) * one * per, st));
+  cudaError_t me;
+  while ((me = cudaMallocAsync((void **) &buf, sizeof(double) * one * per, st)) ==
+             cudaErrorMemoryAllocation && per > 1) {
+    cudaGetLastError();
+    per /= 2;
+  }
+  H2B_CUDA_TRY(me);
   int rc = H2B_OK;
   for (uint32_t b = 0; rc == H2B_OK && b < n; b += per) {
     const uint32_t m = std::min(per, n - b);

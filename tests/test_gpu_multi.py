@@ -83,9 +83,9 @@ def test_columns_in_place():
 
 
 @contextlib.contextmanager
-def no_room():
-    """Stream-ordered allocations of 1 MiB and more fail meanwhile: they come from a pool of limited size
-    that is full."""
+def no_room(left=0):
+    """Stream-ordered allocations find `left` pieces of 1 MiB meanwhile: they come from a pool of limited
+    size that is full but for these."""
     from cuda.bindings import driver as cu
 
     def ok(r):
@@ -104,6 +104,9 @@ def no_room():
             break
         held.append(r[1])
     assert r[0] == cu.CUresult.CUDA_ERROR_OUT_OF_MEMORY
+    for _ in range(left):
+        ok(cu.cuMemFreeAsync(held.pop(), cu.CUstream(0)))
+    ok(cu.cuCtxSynchronize())
     ok(cu.cuDeviceSetMemPool(dev, pool))
     try:
         yield
@@ -124,6 +127,15 @@ def test_columns_without_room():
     with no_room():
         multi(H, 1.0, 8, X, H.cols, Y, H.rows)
     close(Y, ref)
+
+
+def test_export_without_room():
+    """The coupling matrices of 1472 blocks (368 MB), put out in pieces that fit 4 MiB."""
+    H = matrix("helmholtz", K, 5)
+    ref = H.export(4)
+    with no_room(4):
+        out = H.export(4)
+    assert np.array_equal(out, ref)
 
 
 def parts(H):
