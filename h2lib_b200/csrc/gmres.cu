@@ -796,7 +796,9 @@ __global__ void precheck_kernel(GmresDev g, cudaGraphConditionalHandle hw) {
   __syncthreads();
   for (uint32_t s = threadIdx.x; s < g.nsys; s += blockDim.x) {
     GmresState *y = g.state + s;
-    y->active = keeps_going(y, g.ctl->maxiter) ? 1u : 0u;
+    // a system restarted at the end of the launch before keeps what its restart left: err is the new
+    // start's residual, and the reference steps after every restart whatever it is
+    if (!y->restart) y->active = keeps_going(y, g.ctl->maxiter) ? 1u : 0u;
     y->restart = 0;
     if (g.mask) g.mask[s] = y->active;
     if (y->active) any = 1;
