@@ -259,8 +259,9 @@ static int same_sides(const h2b_bem *bem, const h2b_tree *tree) {
          !memcmp(r.bmax, c.bmax, sizeof(double) * 3 * r.n);
 }
 
-// For every block its transposed block (row and column cluster exchanged), or UINT32_MAX: blocks
-// b with clusters (rc[b], cc[b]) of trees with n clusters.
+// For every block its transposed block (row and column cluster exchanged; a block with r = c is its own),
+// or UINT32_MAX: blocks b with clusters (rc[b], cc[b]) of trees with n clusters.  A block is the
+// transposed one of one block only, so that a list may have a block several times.
 static std::vector<uint32_t> transposed_blocks(const std::vector<uint32_t> &rc,
                                                const std::vector<uint32_t> &cc, uint32_t n) {
   // blocks by row cluster
@@ -269,12 +270,14 @@ static std::vector<uint32_t> transposed_blocks(const std::vector<uint32_t> &rc,
   for (uint32_t r = 0; r < n; r++) start[r + 1] += start[r];
   std::vector<uint32_t> fill(start.begin(), start.end() - 1);
   for (uint32_t b = 0; b < rc.size(); b++) at[fill[rc[b]]++] = b;
-  for (uint32_t b = 0; b < rc.size(); b++)
-    for (uint32_t i = start[cc[b]]; i < start[cc[b] + 1]; i++)
-      if (cc[at[i]] == rc[b]) {
+  for (uint32_t b = 0; b < rc.size(); b++) {
+    if (rc[b] == cc[b]) mate[b] = b;
+    for (uint32_t i = start[cc[b]]; mate[b] == UINT32_MAX && i < start[cc[b] + 1]; i++)
+      if (cc[at[i]] == rc[b] && mate[at[i]] == UINT32_MAX) {
         mate[b] = at[i];
-        break;
+        mate[at[i]] = b;
       }
+  }
   return mate;
 }
 

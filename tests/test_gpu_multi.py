@@ -201,12 +201,29 @@ def test_product_against_parts(pde, m, rb, cb):
     close(singles(H, 1.0, X, np.zeros_like(Y)).T, A @ X.T)
 
 
+def flat(tree, blocks):
+    """A tree with the same clusters and these blocks (row cluster, column cluster, admissible)."""
+    rec, box, idx = tree.clusters()
+    b = np.array(blocks, dtype=np.uint32)
+    tr = [np.ascontiguousarray(rec[:, j]) for j in range(3)] + [np.ascontiguousarray(box), len(idx), idx]
+    handle = lib.h2b_tree_new_flat(len(rec), *tr, len(rec), *tr, len(b), np.ascontiguousarray(b[:, 0]),
+                                   np.ascontiguousarray(b[:, 1]),
+                                   np.ascontiguousarray(b[:, 2].astype(np.uint8)))
+    return hb.Tree(checkp(handle, "h2b_tree_new_flat"))
+
+
+def block_ids(tree):
+    rec, _, _ = tree.clusters()
+    ids = {(int(o), int(s)): i for i, (o, s, _) in enumerate(rec)}
+    return [(ids[int(r0), int(rs)], ids[int(c0), int(cs)], int(adm))
+            for r0, rs, c0, cs, adm in tree.block_records()]
+
+
 def one_sided(tree, by_row):
     """The same clusters with some of the admissible blocks above the diagonal cut into their sons'
     blocks, so that the blocks across the diagonal from them have no transposed partner.  by_row: the
     blocks of a row cluster one after the other, else the order of the block tree."""
-    rec, box, idx = tree.clusters()
-    ids = {(int(o), int(s)): i for i, (o, s, _) in enumerate(rec)}
+    rec, _, _ = tree.clusters()
     ends = {}
 
     def walk(i):
@@ -218,22 +235,31 @@ def one_sided(tree, by_row):
     walk(0)
     sons = {i: [i + 1, ends[i + 1]] for i in range(len(rec)) if rec[i][2]}
     blocks = []
-    for r0, rs, c0, cs, adm in tree.block_records():
-        r, c = ids[int(r0), int(rs)], ids[int(c0), int(cs)]
+    for r, c, adm in block_ids(tree):
         if adm and r < c and r in sons and c in sons and (r + c) % 3:
             blocks += [(a, b, 1) for b in sons[c] for a in sons[r]]
         else:
-            blocks.append((r, c, int(adm)))
+            blocks.append((r, c, adm))
     if by_row:
         blocks.sort()
-    b = np.array(blocks, dtype=np.uint32)
-    tr = [np.ascontiguousarray(rec[:, j]) for j in range(3)] + [np.ascontiguousarray(box), len(idx), idx]
-    handle = lib.h2b_tree_new_flat(len(rec), *tr, len(rec), *tr, len(b), np.ascontiguousarray(b[:, 0]),
-                                   np.ascontiguousarray(b[:, 1]),
-                                   np.ascontiguousarray(b[:, 2].astype(np.uint8)))
     pairs = {(r, c) for r, c, a in blocks if a}
     alone = sum((c, r) not in pairs for r, c in pairs)
-    return hb.Tree(checkp(handle, "h2b_tree_new_flat")), alone, len(pairs)
+    return flat(tree, blocks), alone, len(pairs)
+
+
+@pytest.mark.parametrize("basis", [L, K])
+def test_blocks_listed_twice(basis):
+    """A list that has every block twice is the sum of both."""
+    gr = hb.new_ellipsoid_surface3d(9, (1.0, 0.8, 1.3))
+    tree = hb.build_tree(gr, basis, basis, 24, 1.4)
+    blocks = block_ids(tree)
+    op = hb.new_dlp_laplace_bem3d(gr, 2, 4, basis, basis, 0.5)
+    H = hb.H2Matrix(op, flat(tree, blocks), 3).assemble()
+    X = vectors(H, H.cols, 3)
+    ref = singles(H, 2.0, X, np.zeros_like(X))
+    for twice in (blocks + blocks, [b for b in blocks for _ in range(2)]):
+        H2 = hb.H2Matrix(op, flat(tree, twice), 3).assemble()
+        close(singles(H2, 1.0, X, np.zeros_like(X)), ref)
 
 
 @pytest.mark.parametrize("shape", ["symmetric", "one-sided", "one-sided by row"])
