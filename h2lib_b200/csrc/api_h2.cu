@@ -318,7 +318,6 @@ static h2b_h2matrix *h2matrix_create(const h2b_bem *bem, const h2b_tree *tree, u
   uint64_t ntot = 0;
   h2b_nearplan plan;
   h2b_nearplan_init(&plan);
-  plan.skip_sing = 1;  // singular pairs are found on the device below
   // equal sides share their triangle lists (the plan knows a list by its index pointer)
   const uint32_t *cidx = h->same ? tree->row.idx : tree->col.idx;
   for (uint32_t b = 0; rc == H2B_OK && b < tree->blocks.n; b++) {
@@ -714,7 +713,7 @@ static void build_items(const h2b_h2matrix *h, uint32_t pb, uint32_t fwd_rows, u
   }
   m.n = (uint32_t) it.size();
   for (int q = 0; q < 4; q++) m.start[q] = start[q];
-  m.max_rows = m.max_cols_t = 0;
+  m.max_rows = 0;
   m.per_block = (k + panel_cols(k) - 1) / panel_cols(k);
   for (int g = 0; g < 3; g++) m.max_bytes[g] = m.max_x[g] = m.max_x2[g] = 0;
   for (const MvItem &e : it) {
@@ -723,7 +722,6 @@ static void build_items(const h2b_h2matrix *h, uint32_t pb, uint32_t fwd_rows, u
     const int g = kind == H2B_MV_COUPLING ? 1 : kind == H2B_MV_BACKWARD ? 2 : 0;
     m.max_bytes[g] = std::max<uint32_t>(m.max_bytes[g], e.rows * e.cols * 8u * (cpx ? W : 1u));
     if (!(e.flags & H2B_MV_TRANS)) m.max_rows = std::max(m.max_rows, e.rows);
-    else m.max_cols_t = std::max(m.max_cols_t, e.cols);
     m.max_x[g] = std::max(m.max_x[g], (e.flags & H2B_MV_TRANS) ? e.rows : e.cols);
     if (e.flags & H2B_MV_SYM) m.max_x2[g] = std::max(m.max_x2[g], e.rows);
   }

@@ -59,7 +59,7 @@ template <bool CX> __device__ __forceinline__ void st(double *p, size_t i, cd v)
 // The arrays of one system.
 struct Sys {
   uint32_t n, nblk, s;
-  double *qr, *tau, *T, *rhat, *w, *u, *q, *abuf, *part;
+  double *qr, *tau, *T, *rhat, *u, *q, *abuf, *part;
   GmresState *state;
 };
 
@@ -75,7 +75,6 @@ __device__ __forceinline__ Sys sys_view(const GmresDev &g, uint32_t s) {
   v.tau = g.tau + 2 * (size_t) s * g.kmax;
   v.T = g.T + 2 * (size_t) s * g.kmax * g.kmax;
   v.rhat = g.rhat + 2 * (size_t) s * (g.kmax + 1);
-  v.w = g.w + 2 * (size_t) s * (g.kmax + 1);
   v.u = g.u + 2 * (size_t) s * (g.kmax + 1);
   v.q = g.q + W * y.row0;
   v.abuf = g.abuf + W * y.row0;
@@ -303,7 +302,7 @@ constexpr int SMALL_THREADS = SGRP * GMRES_KMAX;
 // all its loads in flight at once; the warps' sums are combined in shared memory.  The caller
 // synchronises before reading z.
 __device__ void sum_parts_all(const GmresDev &g, const Sys &v, uint32_t k, double *zr,
-                              double *zi, uint32_t j0 = 0) {
+                              double *zi) {
   constexpr int NW = SMALL_THREADS / 32;  // warps of the bookkeeping CTA
   __shared__ double wsr[NW][GMRES_KMAX], wsi[NW][GMRES_KMAX];
   const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -311,8 +310,8 @@ __device__ void sum_parts_all(const GmresDev &g, const Sys &v, uint32_t k, doubl
     double sr = 0.0, si = 0.0;
 #pragma unroll 8
     for (uint32_t b = w; b < v.nblk; b += NW) {
-      sr += v.part[(size_t) b * g.ldpart * 2 + 2 * (j0 + j)];
-      si += v.part[(size_t) b * g.ldpart * 2 + 2 * (j0 + j) + 1];
+      sr += v.part[(size_t) b * g.ldpart * 2 + 2 * j];
+      si += v.part[(size_t) b * g.ldpart * 2 + 2 * j + 1];
     }
     wsr[w][j] = sr;
     wsi[w][j] = si;
@@ -453,10 +452,6 @@ __global__ void __launch_bounds__(SMALL_THREADS) small_kernel(GmresDev g, int ph
     // after vth: w = V^H a; u = T^H w
     sum_parts_all(g, v, k, zr, zi);
     __syncthreads();
-    if (t <= k) {
-      v.w[2 * t] = zr[t];
-      v.w[2 * t + 1] = zi[t];
-    }
     cd u = {0.0, 0.0};
     if (r <= k) {
 #pragma unroll 8
@@ -879,7 +874,7 @@ size_t h2b_gmres_workspace(int cx, uint32_t nsys, const uint32_t *sizes, uint32_
   return W * n * kmax                       // qr
          + 2 * (size_t) nsys * kmax          // tau
          + 2 * (size_t) nsys * kmax * kmax   // T
-         + 3 * 2 * (size_t) nsys * ld        // rhat, w, u
+         + 2 * 2 * (size_t) nsys * ld        // rhat, u
          + 2 * W * n                         // q, abuf
          + 2 * nb * ld                       // part
          + (sizeof(GmresState) * nsys + sizeof(GmresCtl) + sizeof(GmresSys) * nsys +
@@ -914,7 +909,6 @@ void h2b_gmres_layout(GmresDev *g, double *p, int cx, uint32_t nsys, const uint3
   g->tau = p; p += 2 * (size_t) nsys * kmax;
   g->T = p; p += 2 * (size_t) nsys * kmax * kmax;
   g->rhat = p; p += 2 * (size_t) nsys * ld;
-  g->w = p; p += 2 * (size_t) nsys * ld;
   g->u = p; p += 2 * (size_t) nsys * ld;
   g->q = p; p += W * n;
   g->abuf = p; p += W * n;

@@ -49,7 +49,7 @@ struct GmresDev {
   double *tau;               // nsys x kmax (complex pairs)
   double *T;                 // nsys x kmax x kmax (complex pairs)
   double *rhat;              // nsys x (kmax + 1) (complex pairs)
-  double *w, *u;             // nsys x (kmax + 1) (complex pairs)
+  double *u;                 // nsys x (kmax + 1) (complex pairs)
   double *q;                 // n
   double *abuf;              // n
   double *part;              // nblocks x ldpart (complex pairs)

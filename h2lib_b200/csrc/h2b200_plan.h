@@ -45,10 +45,6 @@ typedef struct {
   h2b_triref *refs;
   uint32_t nrefs;
   size_t crefs;
-  h2b_sing *sing;
-  uint32_t nsing;
-  size_t csing;
-  uint32_t case_start[5];   /* after finalize: singular pairs of case c in [case_start[c], [c+1]) */
   /* triangle lists already in `refs`, keyed by (index pointer, length, basis): the tiles of one
    * cluster share a single list (open addressing, capacity a power of two) */
   const uint32_t **lkey;
@@ -56,8 +52,6 @@ typedef struct {
   size_t lcap, lcount;
   uint64_t *order;          /* scratch of the list ordering */
   size_t corder;
-  /* 1: leave the singular pairs to the device classification (h2b_near_classify) */
-  int skip_sing;
 } h2b_nearplan;
 
 /* Vertex -> triangle adjacency plus scratch stamps for the plan builder. */
@@ -65,7 +59,7 @@ typedef struct {
   uint32_t nv, nt;
   uint32_t *off, *tri;
   const uint32_t *t;
-  uint32_t *vstamp, *tstamp, *tpos;
+  uint32_t *vstamp, *tstamp;
   int32_t *vloc;
   uint32_t gen;
 } h2b_adjacency;
@@ -80,7 +74,6 @@ int h2b_nearplan_add_block(h2b_nearplan *p, h2b_adjacency *adj, int row_basis, i
                            const uint32_t *ridx, uint32_t rows, const uint32_t *cidx,
                            uint32_t cols, uint64_t out_off, uint32_t ld, int ntrans,
                            uint32_t tile);
-int h2b_nearplan_finalize(h2b_nearplan *p);
 /* Triangle list of an index set (linear: triangles touching the vertices, with local rows;
  * constant: the triangles themselves), appended to p->refs. */
 int h2b_nearplan_add_reflist(h2b_nearplan *p, h2b_adjacency *adj, int linear,
@@ -89,9 +82,8 @@ int h2b_nearplan_add_reflist(h2b_nearplan *p, h2b_adjacency *adj, int linear,
  * tiles on the same index pointer. */
 int h2b_nearplan_tile_list(h2b_nearplan *p, h2b_adjacency *adj, int linear, const uint32_t *idx,
                            uint32_t n, uint32_t *off, uint32_t *len);
-uint32_t h2b_pair_code(const uint32_t *tv, const uint32_t *sv);
-/* Marks the tiles of one block (row and column index lists equal: first tile t0, nt tiles per side)
- * or of two blocks with exchanged row and column lists (t0: nr x nc tiles, t1: nc x nr tiles) as each
+/* Marks the tiles of one block (row and column index lists equal: t0 = t1, nr = nc tiles per side) or
+ * of two blocks with exchanged row and column lists (t0: nr x nc tiles, t1: nc x nr tiles) as each
  * other's mates.  Tiles are in add_block's order. */
 void h2b_nearplan_mate(h2b_nearplan *p, uint32_t t0, uint32_t t1, uint32_t nr, uint32_t nc);
 /* The tiles to run when mates are filled together: of two mates only the first, largest products of

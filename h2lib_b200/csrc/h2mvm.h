@@ -38,7 +38,6 @@ struct MvItems {
   uint32_t max_x[3];         // longest x slice (elements: cols, or rows when transposed)
   uint32_t max_x2[3];        // longest second x slice (rows of an H2B_MV_SYM item), 0: none
   uint32_t max_rows;         // largest rows of an untransposed item
-  uint32_t max_cols_t;       // largest columns of a transposed item
   uint32_t per_block;        // panels of a coupling block
 };
 

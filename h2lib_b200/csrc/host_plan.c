@@ -1,14 +1,12 @@
 /* Host-side nearfield plans: cut the requested blocks into output tiles of at most 64 x 64
- * entries, list the triangles each tile touches, and find the singular (vertex-sharing) triangle
- * pairs, bucketed by Sauter-Schwab case.  The device kernels consume the flat arrays.
+ * entries and list the triangles each tile touches.  The device kernels consume the flat arrays; the
+ * singular (vertex-sharing) triangle pairs are found on the device (h2b_near_classify).
  *
  * Semantics follow the reference's nearfield callbacks:
  *   constant basis  assemble_cc_near_bem3d   Library/bem3d.c:1151 — one triangle pair per entry;
  *   linear basis    assemble_ll_near_bem3d   Library/bem3d.c:3038 — entry (i, j) sums every pair
  *                   (t, s) with vertex i in t and vertex j in s, using the weight of the local
  *                   basis functions of i in t and j in s; cl / lc mix the two.
- * Classification and vertex permutation restate select_quadrature_singquad2d
- * (Library/singquad2d.c:549): the shared vertices come first, in the row triangle's order.
  */
 #include <stdint.h>
 #include <stdlib.h>
@@ -39,8 +37,7 @@ h2b_adjacency_build(uint32_t vertices, uint32_t triangles, const uint32_t *t, h2
   adj->vstamp = (uint32_t *) calloc(vertices ? vertices : 1, sizeof(uint32_t));
   adj->vloc = (int32_t *) calloc(vertices ? vertices : 1, sizeof(int32_t));
   adj->tstamp = (uint32_t *) calloc(triangles ? triangles : 1, sizeof(uint32_t));
-  adj->tpos = (uint32_t *) calloc(triangles ? triangles : 1, sizeof(uint32_t));
-  if (!adj->off || !adj->tri || !adj->vstamp || !adj->vloc || !adj->tstamp || !adj->tpos) {
+  if (!adj->off || !adj->tri || !adj->vstamp || !adj->vloc || !adj->tstamp) {
     h2b_adjacency_free(adj);
     return H2B_ERR_NOMEM;
   }
@@ -72,7 +69,6 @@ void
 h2b_adjacency_free(h2b_adjacency *adj)
 {
   free(adj->off); free(adj->tri); free(adj->vstamp); free(adj->vloc); free(adj->tstamp);
-  free(adj->tpos);
   memset(adj, 0, sizeof(*adj));
 }
 
@@ -85,7 +81,7 @@ h2b_nearplan_init(h2b_nearplan *p)
 void
 h2b_nearplan_free(h2b_nearplan *p)
 {
-  free(p->tiles); free(p->refs); free(p->sing);
+  free(p->tiles); free(p->refs);
   free((void *) p->lkey); free(p->lkn); free(p->loff); free(p->llen);
   free(p->order);
   memset(p, 0, sizeof(*p));
@@ -270,46 +266,6 @@ h2b_nearplan_add_reflist(h2b_nearplan *p, h2b_adjacency *adj, int linear, const 
   return add_reflist(p, adj, linear, idx, n, off, len);
 }
 
-/* Vertex permutation of a pair: returns the number of shared vertices and the packed code
- * case | tp0<<2 | tp1<<4 | tp2<<6 | sp0<<8 | sp1<<10 | sp2<<12. */
-uint32_t
-h2b_pair_code(const uint32_t *tv, const uint32_t *sv)
-{
-  uint32_t p = 0, i, j, q, tp[3] = {0, 1, 2}, sp[3] = {0, 1, 2};
-  for (i = 0; i < 3; i++)
-    for (j = 0; j < 3; j++)
-      p += (tv[i] == sv[j]);
-  if (p == 1 || p == 2) {
-    uint32_t c = 0;
-    for (i = 0; i < 3; i++)
-      for (j = 0; j < 3; j++)
-        if (tv[i] == sv[j]) {
-          tp[c] = i;
-          sp[c] = j;
-          c++;
-          break;
-        }
-    q = c;
-    for (i = 0; i < 3; i++) {
-      for (j = 0; j < q && tv[i] != tv[tp[j]]; j++)
-        ;
-      if (j == q)
-        tp[q++] = i;
-    }
-    q = c;
-    for (i = 0; i < 3; i++) {
-      for (j = 0; j < q && sv[i] != sv[sp[j]]; j++)
-        ;
-      if (j == q)
-        sp[q++] = i;
-    }
-  }
-  if (p > 3)
-    p = 3;
-  return p | (tp[0] << 2) | (tp[1] << 4) | (tp[2] << 6) | (sp[0] << 8) | (sp[1] << 10)
-         | (sp[2] << 12);
-}
-
 /* add_reflist, reusing the list of an index range seen before. */
 static int
 cached_reflist(h2b_nearplan *p, h2b_adjacency *adj, int linear, const uint32_t *idx, uint32_t n,
@@ -348,17 +304,13 @@ h2b_nearplan_tile_list(h2b_nearplan *p, h2b_adjacency *adj, int linear, const ui
 static int
 add_tile(h2b_nearplan *p, h2b_adjacency *adj, int row_linear, int col_linear,
          const uint32_t *ridx, uint32_t rows, const uint32_t *cidx, uint32_t cols,
-         uint64_t out_off, uint32_t ld, int ntrans, uint32_t reuse_tr_off, uint32_t reuse_tr_len)
+         uint64_t out_off, uint32_t ld, int ntrans)
 {
   h2b_tile *tl;
-  uint32_t tr_off, tr_len, sc_off, sc_len, js, i, gt;
+  uint32_t tr_off, tr_len, sc_off, sc_len;
   int rc;
 
-  if (reuse_tr_len != UINT32_MAX) {
-    tr_off = reuse_tr_off;
-    tr_len = reuse_tr_len;
-  }
-  else if ((rc = cached_reflist(p, adj, row_linear, ridx, rows, &tr_off, &tr_len)) != H2B_OK)
+  if ((rc = cached_reflist(p, adj, row_linear, ridx, rows, &tr_off, &tr_len)) != H2B_OK)
     return rc;
   if ((rc = cached_reflist(p, adj, col_linear, cidx, cols, &sc_off, &sc_len)) != H2B_OK)
     return rc;
@@ -375,43 +327,6 @@ add_tile(h2b_nearplan *p, h2b_adjacency *adj, int row_linear, int col_linear,
   tl->cols = (uint16_t) cols;
   tl->flags = ntrans ? 1u : 0u;
   tl->mate = 0;
-
-  if (p->skip_sing) {
-    p->ntiles++;
-    return H2B_OK;
-  }
-  /* singular pairs: row triangles sharing a vertex with a column triangle */
-  gt = next_gen(adj);
-  for (i = 0; i < tr_len; i++) {
-    uint32_t tt = p->refs[tr_off + i].t;
-    adj->tstamp[tt] = gt;
-    adj->tpos[tt] = tr_off + i;
-  }
-  for (js = 0; js < sc_len; js++) {
-    uint32_t ss = p->refs[sc_off + js].t, found[24], nf = 0, k, a, f;
-    const uint32_t *sv = adj->t + 3 * (size_t) ss;
-    for (k = 0; k < 3; k++)
-      for (a = adj->off[sv[k]]; a < adj->off[sv[k] + 1]; a++) {
-        uint32_t tt = adj->tri[a];
-        if (adj->tstamp[tt] != gt)
-          continue;
-        for (f = 0; f < nf && found[f] != tt; f++)
-          ;
-        if (f < nf || nf == 24)
-          continue;
-        found[nf++] = tt;
-      }
-    for (f = 0; f < nf; f++) {
-      h2b_sing *sg;
-      uint32_t code = h2b_pair_code(adj->t + 3 * (size_t) found[f], sv);
-      GROW(p->sing, p->nsing, p->csing, 1, h2b_sing);
-      sg = &p->sing[p->nsing++];
-      sg->tile = p->ntiles;
-      sg->tr = adj->tpos[found[f]];
-      sg->sc = sc_off + js;
-      sg->code = code;
-    }
-  }
   p->ntiles++;
   return H2B_OK;
 }
@@ -430,8 +345,7 @@ h2b_nearplan_add_block(h2b_nearplan *p, h2b_adjacency *adj, int row_basis, int c
     for (r0 = 0; r0 < rows; r0 += tile) {
       uint32_t nr = rows - r0 < tile ? rows - r0 : tile;
       uint64_t off = ntrans ? out_off + c0 + (uint64_t) r0 * ld : out_off + r0 + (uint64_t) c0 * ld;
-      int rc = add_tile(p, adj, rl, cl, ridx + r0, nr, cidx + c0, nc, off, ld, ntrans, 0,
-                        UINT32_MAX);
+      int rc = add_tile(p, adj, rl, cl, ridx + r0, nr, cidx + c0, nc, off, ld, ntrans);
       if (rc != H2B_OK)
         return rc;
     }
@@ -476,32 +390,4 @@ h2b_nearplan_halves(const h2b_nearplan *p, uint32_t *list)
 #undef SKIP
 #undef WORK
   return n;
-}
-
-/* Stable counting sort of the singular pairs by case (1 vertex, 2 edge, 3 identical), so that
- * warps meet runs of equal trip counts. */
-int
-h2b_nearplan_finalize(h2b_nearplan *p)
-{
-  uint32_t cnt[4] = {0, 0, 0, 0}, start[4], i;
-  h2b_sing *tmp;
-  if (p->nsing == 0)
-    return H2B_OK;
-  tmp = (h2b_sing *) malloc(sizeof(h2b_sing) * p->nsing);
-  if (!tmp)
-    return H2B_ERR_NOMEM;
-  for (i = 0; i < p->nsing; i++)
-    cnt[p->sing[i].code & 3]++;
-  start[0] = 0;
-  for (i = 1; i < 4; i++)
-    start[i] = start[i - 1] + cnt[i - 1];
-  for (i = 0; i < 4; i++)
-    p->case_start[i] = start[i];
-  p->case_start[4] = p->nsing;
-  for (i = 0; i < p->nsing; i++)
-    tmp[start[p->sing[i].code & 3]++] = p->sing[i];
-  free(p->sing);
-  p->sing = tmp;
-  p->csing = p->nsing;
-  return H2B_OK;
 }

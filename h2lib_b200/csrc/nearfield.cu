@@ -1781,9 +1781,9 @@ int launch_kk(const h2b_near_launch *L, cudaStream_t st) {
   return launch_kk_basis<KK, false, false>(L, st);
 }
 
-// Vertex permutation of a pair, the device twin of h2b_pair_code (host_plan.c): number of shared
-// vertices in bits 0-1, the row triangle's order (shared vertices first) in bits 2-7, the column
-// triangle's in bits 8-13 (select_quadrature_singquad2d, Library/singquad2d.c:549).
+// Vertex permutation of a pair: number of shared vertices in bits 0-1, the row triangle's order (shared
+// vertices first) in bits 2-7, the column triangle's in bits 8-13 (select_quadrature_singquad2d,
+// Library/singquad2d.c:549).
 __device__ uint32_t pair_code_dev(const uint32_t tv[3], const uint32_t sv[3]) {
   uint32_t p = 0, tp[3] = {0, 1, 2}, sp[3] = {0, 1, 2};
   for (int i = 0; i < 3; i++)

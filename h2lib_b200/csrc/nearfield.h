@@ -53,7 +53,7 @@ int h2b_near_upload_dist_rules(void);
 /* The QuadRec of every triangle (after h2b_near_upload_dist_rules). */
 int h2b_near_quad_records(const void *tri, uint32_t nt, void *qrec, cudaStream_t st);
 /* The triangles around each triangle (those that share a vertex with it, itself included), with the
- * vertex permutation code of h2b_pair_code: triangle t's are (id, code) at nb[off[t]] ..
+ * vertex permutation code (pair_code_dev): triangle t's are (id, code) at nb[off[t]] ..
  * nb[off[t] + len[t]).  vt_off / vt_tri: the surface's vertex -> triangle lists (CSR); cursor: a
  * device counter set to 0; nb: room for the sum over the vertices of their squared triangle counts. */
 int h2b_near_neighbours(const void *tri, uint32_t nt, const uint32_t *vt_off, const uint32_t *vt_tri,
