@@ -637,19 +637,19 @@ __global__ void point_source_kernel(HarmArgs a, double k, double cre, double cim
 // eval_brakhage_werner_c / _l (Tests/test_helmholtzbem3d.c:68 / :134).
 //
 // The work is a sine, a cosine and about 35 FP64 instructions per (point, quadrature point), so the
-// density's values are formed once per quadrature point (bw_source_kernel: position, normal, kconst g
-// w) and the sums (bw_eval_kernel) keep an evaluation point per lane: a warp walks over its sources,
-// each one broadcast load, its lanes on pl points (a power of two, the other lanes share the
-// sources).  CTAs take 32 points and one of `chunks` ranges of the sources, as many as fill the
-// SMs whatever the number of points; the chunks' sums are added in order by a third kernel, so a sum is
-// the same on every run.  49152 triangles, 400 points: one CTA per point over triangle records
-// 1535 us, this form 513 us.
+// density's values are formed once per quadrature point (bw_source_kernel: position, normal, g w) and
+// the sums (bw_eval_kernel) keep an evaluation point per lane: a warp walks over its sources, each one
+// broadcast load, its lanes on pl points (a power of two, the other lanes share the sources).  CTAs take
+// 32 points and one of `chunks` ranges of the sources, as many as fill the SMs whatever the number of
+// points; the chunks' sums are added in a fixed order by a third kernel, so a sum is the same on every
+// run.  49152 triangles, 400 points: one CTA per point over triangle records 1535 us, this form 513 us.
+// Against 80-bit arithmetic both are off by 8e-16 of the norm there (1.3e-15, for 1 % less time, with r
+// from the reciprocal root alone, one sum per lane, an addition per product and the chunks in one sum).
 struct __align__(16) BwSource {
   double y[3], n[3], re, im;
 };
 
-__global__ void bw_source_kernel(HarmArgs a, const double *w, int linear, double kconst,
-                                 BwSource *out) {
+__global__ void bw_source_kernel(HarmArgs a, const double *w, int linear, BwSource *out) {
   const uint64_t i = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x;
   const uint32_t t = (uint32_t) (i / (uint32_t) a.ns), q = (uint32_t) (i - (uint64_t) t * a.ns);
   if (i >= (uint64_t) a.nt * a.ns) return;
@@ -667,10 +667,9 @@ __global__ void bw_source_kernel(HarmArgs a, const double *w, int linear, double
     vr = a.ws[q] * w[2 * (size_t) t];
     vi = a.ws[q] * w[2 * (size_t) t + 1];
   }
-  const double f = kconst * T.g;
   for (int d = 0; d < 3; d++) s.n[d] = T.n[d];
-  s.re = f * vr;
-  s.im = f * vi;
+  s.re = T.g * vr;
+  s.im = T.g * vi;
   out[i] = s;
 }
 
@@ -689,13 +688,13 @@ __global__ void __launch_bounds__(BW_THREADS)
   const uint64_t s0 = ns / parts * me + ns % parts * me / parts;
   const uint32_t len = (uint32_t) (ns / parts * (me + 1) + ns % parts * (me + 1) / parts - s0);
   src += s0;
-  double ur = 0.0, ui = 0.0;
-#pragma unroll 2
-  for (uint32_t i = sub; i < len; i += subs) {
-    const BwSource s = src[i];
+  // two sums in turn: half as many terms behind one another, half the rounding of a long sum
+  double ur = 0.0, ui = 0.0, vr = 0.0, vi = 0.0;
+  auto add = [&](const BwSource &s, double &ur, double &ui) {
     const double d0 = x0 - s.y[0], d1 = x1 - s.y[1], d2 = x2 - s.y[2];
     const double r2 = fma(d0, d0, fma(d1, d1, d2 * d2));
-    const double ri = rsqrt_nr(r2), r = r2 * ri;
+    // r as near as a square root (one step of Newton's method): the phase takes its error times k r
+    const double ri = rsqrt_nr(r2), rt = r2 * ri, r = fma(fma(-rt, rt, r2), 0.5 * ri, rt);
     const double dn = fma(d0, s.n[0], fma(d1, s.n[1], d2 * s.n[2]));
     const double krr = kr * r;
     double sn, cs;
@@ -706,9 +705,17 @@ __global__ void __launch_bounds__(BW_THREADS)
     const double pr = e * fma(ei, r2, DAMPED ? fma(ki * r, dn, dn) : dn);
     const double pi = -e * fma(krr, dn, er * r2);
     const double qr = cs * pr - sn * pi, qi = fma(cs, pi, sn * pr);
-    ur = fma(qr, s.re, fma(-qi, s.im, ur));
-    ui = fma(qr, s.im, fma(qi, s.re, ui));
+    ur += fma(qr, s.re, -qi * s.im);
+    ui += fma(qr, s.im, qi * s.re);
+  };
+  uint32_t i = sub;
+  for (; i + subs < len; i += 2 * subs) {
+    add(src[i], ur, ui);
+    add(src[i + subs], vr, vi);
   }
+  if (i < len) add(src[i], ur, ui);
+  ur += vr;
+  ui += vi;
   for (uint32_t o = pl; o < 32u; o <<= 1) {
     ur += __shfl_xor_sync(0xffffffffu, ur, o);
     ui += __shfl_xor_sync(0xffffffffu, ui, o);
@@ -725,14 +732,20 @@ __global__ void __launch_bounds__(BW_THREADS)
   }
 }
 
-// out[p] = the chunks' sums of point p, in order
-__global__ void bw_sum_kernel(const double *part, uint32_t np, uint32_t chunks, double *out) {
+// out[p] = kconst times the chunks' sums of point p, added in a fixed order: eight sums in turn, then
+// those in pairs, so that no long chain of additions rounds at the size of the result
+__global__ void bw_sum_kernel(const double *part, uint32_t np, uint32_t chunks, double kconst,
+                              double *out) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= 2 * np) return;
-  double s = 0.0;
-#pragma unroll 4
-  for (uint32_t c = 0; c < chunks; c++) s += part[(size_t) c * 2 * np + i];
-  out[i] = s;
+  double s[8];
+#pragma unroll
+  for (int q = 0; q < 8; q++) s[q] = 0.0;
+  for (uint32_t c = 0; c < chunks; c += 8)
+#pragma unroll
+    for (int q = 0; q < 8; q++)
+      if (c + q < chunks) s[q] += part[(size_t) (c + q) * 2 * np + i];
+  out[i] = kconst * (((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7])));
 }
 
 // Several surfaces (triangle ranges tri_off[s] .. tri_off[s+1]) and right-hand sides: the source
@@ -1144,7 +1157,7 @@ extern "C" int h2b_eval_brakhage_werner(const h2b_bem *bem, uint32_t npoints, co
   if (rc != H2B_OK) return rc;
   H2B_CUDA_TRY(cudaMemcpyAsync(dw, w, sizeof(double) * 2 * n, cudaMemcpyDefault, st));
   H2B_CUDA_TRY(cudaMemcpyAsync(dp, points, sizeof(double) * 3 * npoints, cudaMemcpyDefault, st));
-  bw_source_kernel<<<(uint32_t) ((ns + 255) / 256), 256, 0, st>>>(a, dw, linear, bem->kconst, src);
+  bw_source_kernel<<<(uint32_t) ((ns + 255) / 256), 256, 0, st>>>(a, dw, linear, src);
   h2b_note_launch();
   const dim3 grid(groups, chunks);
   if (bem->k_im != 0.0)
@@ -1154,7 +1167,7 @@ extern "C" int h2b_eval_brakhage_werner(const h2b_bem *bem, uint32_t npoints, co
     bw_eval_kernel<false><<<grid, BW_THREADS, 0, st>>>(src, ns, dp, npoints, pl, bem->k_re, 0.0,
                                                        eta_re, eta_im, part);
   h2b_note_launch();
-  bw_sum_kernel<<<(2 * npoints + 127) / 128, 128, 0, st>>>(part, npoints, chunks, du);
+  bw_sum_kernel<<<(2 * npoints + 127) / 128, 128, 0, st>>>(part, npoints, chunks, bem->kconst, du);
   h2b_note_launch();
   H2B_CUDA_TRY(cudaGetLastError());
   H2B_CUDA_TRY(cudaMemcpyAsync(u, du, sizeof(double) * 2 * npoints, cudaMemcpyDefault, st));

@@ -39,8 +39,7 @@
 namespace {
 
 constexpr int MAXTHREADS = 288;              // up to 8 consumer warps and the producer warp
-constexpr int MAXROWS = 128;                 // rows of an untransposed item, columns of a transposed
-                                             // one (four 32-lane slots)
+constexpr int MAXROWS = 128;                 // rows of an untransposed item (four 32-lane slots)
 constexpr uint32_t WAIT_LIMIT = 1u << 24;    // try_wait polls before a stage counts as lost
 
 // Vectors of a product with nrhs right-hand sides.  With a mask (batched solves on a forest:
