@@ -49,11 +49,10 @@ CC_SLP_REF_FLOPS_PER_POINT = 46
 # reference count per point of the Helmholtz kernels, constant basis (sin, cos and exp counted
 # as 1): single layer 54, double layer 66
 HELM_FLOPS_PER_POINT = {"slp": 54, "dlp": 66}
-# DRAM bytes (read 5,998,336 + write 214,822,656) of one near_dist_kernel launch on the default
-# workload (sphere split 64), from an ncu capture of the full-size run (single-pass metrics
-# dram__bytes_read.sum + dram__bytes_write.sum) of the kernel that filled every tile by itself; the
-# output, which is nearly all of it, is the same
-NEAR_DIST_TRAFFIC = 5998336 + 214822656
+# DRAM bytes (read + write) of one near_ring_kernel launch on the default workload (sphere split 64, V
+# and K together), from an ncu capture of the full-size run (single-pass metrics dram__bytes_read.sum +
+# dram__bytes_write.sum)
+NEAR_DIST_TRAFFIC = 9467648 + 215022080
 # DRAM bytes (read + write) of one FP64 matvec product per algorithmic byte: 206.0 MB for
 # 200.8 MB on the sphere split 48 (ncu, dram__bytes_read.sum + dram__bytes_write.sum of the two
 # item-kernel launches and the coupling launch of a product), applied to the bench's workload by its
@@ -393,7 +392,7 @@ def run_ours(a, rank, world, local):
     achieved = executed / (near_dist_ms * 1e-3) / 1e12
     ref_tflops = dist_flops / (near_dist_ms * 1e-3) / 1e12
     # distinct triangle pairs: a pair that several nearfield blocks touch (linear basis) is
-    # evaluated once per block, as in the reference; counted once here
+    # evaluated once per block (and its transposed block); counted once here
     up = V.unique_pairs()
     uniq = {"pairs": up, "evaluations_per_distant_pair": pc["distant"] / up["distant"],
             "executed_flops": up["distant"] * EXECUTED_FLOPS_PER_PAIR,

@@ -542,8 +542,9 @@ int h2b_check_err_flag(const h2b_bem *b, cudaStream_t st) {
 // s vertices touches about 2 s + 4.3 sqrt(s) triangles (the inner ones and those along the border,
 // counted on refined spheres), rows in groups of 32 lanes, so smaller tiles evaluate border pairs more
 // often but spread a small block over the SMs; with constant bases tiles share no pairs.  Linear
-// columns with q = 2 spread a tile over a cluster of up to eight CTAs as well (near_ring_kernel; the
-// same rule as its launch).  FIXED is the fixed cost of a tile in pairs (clearing, staging and writing
+// columns with q = 2 spread a tile over a cluster of up to eight CTAs as well (near_ring_kernel).  The
+// estimate fills two CTAs per SM three times over, as the launch does (RING_FILL) for kernels of up to
+// three planes; the launch of the complex double layer with mates counts one CTA per SM.  FIXED is the fixed cost of a tile in pairs (clearing, staging and writing
 // it).  60 x 57 linear block: four tiles of 32 take 46 us, 8 x 8 tiles 16 us, with clusters 10.
 // 578 x 578 complex double layer, us: a CTA per tile of 16 613, of 32 533 to 642; a
 // cluster per tile of 64 421.

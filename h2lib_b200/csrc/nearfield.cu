@@ -1632,7 +1632,7 @@ int launch_dist(const h2b_near_launch *L, cudaStream_t st) {
 }
 
 // MIR: the tiles of L->half fill their mates too; otherwise every tile by itself.  (block_tile in
-// api_core.cu counts on the cluster rule.)
+// api_core.cu estimates with this cluster rule at two CTAs per SM.)
 template <int KK, bool RL, bool MIR>
 int launch_ring(const h2b_near_launch *L, cudaStream_t st) {
   constexpr int T = ring_threads<KK, MIR>();

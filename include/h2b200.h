@@ -375,7 +375,8 @@ int h2b_h2matrix_addeval(double alpha_re, double alpha_im, const h2b_h2matrix *h
                          const double *x, double *y);
 
 /* Same with nrhs right-hand sides stored as columns of X (ldx) and Y (ldy), the columns of a product
- * together.  Where Y overlaps X otherwise than as the same columns, one column after the other. */
+ * together: up to eight columns' work vectors are allocated on the matrix's stream for the call.  Where
+ * they do not fit, or Y overlaps X otherwise than as the same columns, one column after the other. */
 int h2b_h2matrix_addeval_multi(double alpha_re, double alpha_im, const h2b_h2matrix *h2,
                                uint32_t nrhs, const double *X, uint64_t ldx, double *Y,
                                uint64_t ldy);
