@@ -774,7 +774,7 @@ void h2b_h2_fill_mvm_plan(h2b_h2matrix *h) {
   p.ctas_per_sm = h->mv_ctas;
   p.warps = h->mv_warps;
   p.stages = h->mv_stages;
-  h2b_mvm_prepare();
+  h2b_mvm_prepare(&p);
 }
 
 // ------------------------------------------------------------------------------------------

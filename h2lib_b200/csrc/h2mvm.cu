@@ -961,6 +961,8 @@ int launch_pair(const MvmPlan *p, const MvmPlan *q, const double *x, double *y, 
 
 }  // namespace
 
+// The kernels that products of a plan launch with entries of type T: one kernel's rank class of the
+// coupling's three, every number of columns.
 template <bool CX, typename T, int SL>
 static int prepare_coupling(void) {
   H2B_CUDA_TRY((h2b_allow_smem<mv_coupling_kernel<CX, T, SL, 1>>()));
@@ -969,27 +971,18 @@ static int prepare_coupling(void) {
   return H2B_OK;
 }
 template <bool CX, typename T>
-static int prepare_ranks(void) {
-  int rc = prepare_coupling<CX, T, 1>();
-  if (rc == H2B_OK) rc = prepare_coupling<CX, T, 2>();
-  return rc == H2B_OK ? prepare_coupling<CX, T, 4>() : rc;
+static int prepare_type(int k) {
+  H2B_CUDA_TRY((h2b_allow_smem<mv_items_kernel<CX, T, 1>>()));
+  H2B_CUDA_TRY((h2b_allow_smem<mv_items_kernel<CX, T, MULTI>>()));
+  return k <= 32 ? prepare_coupling<CX, T, 1>()
+                 : k <= 64 ? prepare_coupling<CX, T, 2>() : prepare_coupling<CX, T, 4>();
 }
 
-extern "C" int h2b_mvm_prepare(void) {
-  int rc = prepare_ranks<false, double>();
-  if (rc == H2B_OK) rc = prepare_ranks<true, double>();
-  if (rc == H2B_OK) rc = prepare_ranks<false, float>();
-  if (rc == H2B_OK) rc = prepare_ranks<true, float>();
-  if (rc != H2B_OK) return rc;
-  H2B_CUDA_TRY((h2b_allow_smem<mv_items_kernel<false, double, 1>>()));
-  H2B_CUDA_TRY((h2b_allow_smem<mv_items_kernel<false, double, MULTI>>()));
-  H2B_CUDA_TRY((h2b_allow_smem<mv_items_kernel<true, double, 1>>()));
-  H2B_CUDA_TRY((h2b_allow_smem<mv_items_kernel<true, double, MULTI>>()));
-  H2B_CUDA_TRY((h2b_allow_smem<mv_items_kernel<false, float, 1>>()));
-  H2B_CUDA_TRY((h2b_allow_smem<mv_items_kernel<false, float, MULTI>>()));
-  H2B_CUDA_TRY((h2b_allow_smem<mv_items_kernel<true, float, 1>>()));
-  H2B_CUDA_TRY((h2b_allow_smem<mv_items_kernel<true, float, MULTI>>()));
-  return H2B_OK;
+extern "C" int h2b_mvm_prepare(const MvmPlan *p) {
+  int rc = p->cx ? prepare_type<true, double>(p->k) : prepare_type<false, double>(p->k);
+  if (rc == H2B_OK && p->fS)
+    rc = p->cx ? prepare_type<true, float>(p->k) : prepare_type<false, float>(p->k);
+  return rc;
 }
 
 static size_t smem_any(const MvmPlan *p, int single, uint32_t nrhs) {
