@@ -89,7 +89,7 @@ extern "C" int h2b_mvm_launch_batch(const MvmPlan *p, int single, uint32_t nrhs,
 // Sets the shared-memory limits of the kernels that a plan's products launch (once per process and
 // kernel); called when a matrix is made and when it gets its FP32 copies, so that no later launch,
 // possibly inside a CUDA graph capture, has to.  Only those kernels, since setting the limit loads a
-// kernel: a process's first matrix (1024 triangles) takes 6.3 ms, with all 44 loaded 8.3 to 10.
+// kernel: a process's first matrix (2048 triangles) takes 6.3 ms, with all 44 loaded 8.3 to 10.
 extern "C" int h2b_mvm_prepare(const MvmPlan *p);
 // Shared-memory bytes per CTA of the item kernel at the plan's launch shape.
 extern "C" size_t h2b_mvm_smem_bytes(const MvmPlan *p, int single);
