@@ -642,9 +642,10 @@ __global__ void point_source_kernel(HarmArgs a, double k, double cre, double cim
 // broadcast load, its lanes on pl points (a power of two, the other lanes share the sources).  CTAs take
 // 32 points and one of `chunks` ranges of the sources, as many as fill the SMs whatever the number of
 // points; the chunks' sums are added in a fixed order by a third kernel, so a sum is the same on every
-// run.  49152 triangles, 400 points: one CTA per point over triangle records 1535 us, this form 513 us.
-// Against 80-bit arithmetic both are off by 8e-16 of the norm there (1.3e-15, for 1 % less time, with r
-// from the reciprocal root alone, one sum per lane, an addition per product and the chunks in one sum).
+// run.  49152 triangles, 400 points: a call with one CTA per point over triangle records 1640 us, this
+// form 497.  Against 80-bit arithmetic both are off by 8e-16 of the norm there (1.3e-15, for 2 % less time,
+// with r from the reciprocal root alone, one sum per lane, an addition per product and the chunks in one
+// sum).
 struct __align__(16) BwSource {
   double y[3], n[3], re, im;
 };
@@ -732,20 +733,25 @@ __global__ void __launch_bounds__(BW_THREADS)
   }
 }
 
-// out[p] = kconst times the chunks' sums of point p, added in a fixed order: eight sums in turn, then
-// those in pairs, so that no long chain of additions rounds at the size of the result
-__global__ void bw_sum_kernel(const double *part, uint32_t np, uint32_t chunks, double kconst,
-                              double *out) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= 2 * np) return;
-  double s[8];
-#pragma unroll
-  for (int q = 0; q < 8; q++) s[q] = 0.0;
-  for (uint32_t c = 0; c < chunks; c += 8)
-#pragma unroll
-    for (int q = 0; q < 8; q++)
-      if (c + q < chunks) s[q] += part[(size_t) (c + q) * 2 * np + i];
-  out[i] = kconst * (((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7])));
+// out[p] = kconst times the chunks' sums of point p: a CTA takes 32 words of the output, a warp every
+// BS_WARPS-th chunk, and the warps' sums are added in pairs, so that no long chain of additions rounds at
+// the size of the result and few points do not wait for a chain of loads.
+constexpr int BS_WARPS = 16;
+__global__ void __launch_bounds__(32 * BS_WARPS)
+    bw_sum_kernel(const double *part, uint32_t np, uint32_t chunks, double kconst, double *out) {
+  __shared__ double red[BS_WARPS][32];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, i = blockIdx.x * 32u + lane;
+  double s = 0.0;
+  if (i < 2 * np) {
+#pragma unroll 4
+    for (uint32_t c = warp; c < chunks; c += BS_WARPS) s += part[(size_t) c * 2 * np + i];
+  }
+  red[warp][lane] = s;
+  for (uint32_t h = BS_WARPS / 2; h > 0; h /= 2) {
+    __syncthreads();
+    if (warp < h) red[warp][lane] += red[warp + h][lane];
+  }
+  if (warp == 0 && i < 2 * np) out[i] = kconst * red[0][lane];
 }
 
 // Several surfaces (triangle ranges tri_off[s] .. tri_off[s+1]) and right-hand sides: the source
@@ -1134,10 +1140,13 @@ extern "C" int h2b_eval_brakhage_werner(const h2b_bem *bem, uint32_t npoints, co
   const int linear = bem->col_basis == H2B_BASIS_LINEAR;
   const size_t n = linear ? s->nv : s->nt;
   cudaStream_t st = s->stream;
-  // chunks of the sources: about four CTAs per SM, at least 32 sources per warp
+  // chunks of the sources: at most twelve CTAs per SM, three rounds of the four that fit, so that a last
+  // round is short, and at least 32 sources per warp.  400 points of 49152 triangles, us a call: at least
+  // four per SM (the 6 CTAs above 592 took a round of their own) 625, at most four 541, eight 509, twelve
+  // 497; 3000 points 3510, 3370, 3110, 3030
   const uint64_t ns = (uint64_t) s->nt * bem->quad.ns;
   const uint32_t groups = (npoints + 31) / 32;
-  const uint32_t want = (4u * (uint32_t) s->num_sms + groups - 1) / groups;
+  const uint32_t want = 12u * (uint32_t) s->num_sms / groups;
   const uint32_t chunks = (uint32_t) std::max<uint64_t>(1, std::min<uint64_t>(want, ns / BW_THREADS));
   uint32_t pl = 1;
   while (pl < 32 && pl < npoints) pl *= 2;
@@ -1167,7 +1176,8 @@ extern "C" int h2b_eval_brakhage_werner(const h2b_bem *bem, uint32_t npoints, co
     bw_eval_kernel<false><<<grid, BW_THREADS, 0, st>>>(src, ns, dp, npoints, pl, bem->k_re, 0.0,
                                                        eta_re, eta_im, part);
   h2b_note_launch();
-  bw_sum_kernel<<<(2 * npoints + 127) / 128, 128, 0, st>>>(part, npoints, chunks, bem->kconst, du);
+  bw_sum_kernel<<<(2 * npoints + 31) / 32, 32 * BS_WARPS, 0, st>>>(part, npoints, chunks, bem->kconst,
+                                                                   du);
   h2b_note_launch();
   H2B_CUDA_TRY(cudaGetLastError());
   H2B_CUDA_TRY(cudaMemcpyAsync(u, du, sizeof(double) * 2 * npoints, cudaMemcpyDefault, st));
